@@ -53,6 +53,8 @@ Context::~Context() {
     cudaFree(splitk_ws);
     cudaFree(merged_ws);
     for (double* q : merged_retired) cudaFree(q);
+    cudaFree(tile_ws);
+    for (double* q : tile_retired) cudaFree(q);
     for (auto& p : pending) {
         cudaEventDestroy(p.second.first);
         cudaEventDestroy(p.second.second);
@@ -563,7 +565,7 @@ RunSchedule& Context::schedule(Plan& p) {
         const std::string& lab = label_of(p.steps[s]);
         size_t e = s;
         while (e < p.steps.size() && p.steps[e].kind == kind && label_of(p.steps[e]) == lab) e++;
-        if (e - s >= 2) {
+        if (kind == Step::GEMM || e - s >= 2) {
             if (kind == Step::GEMM) build_run(p, rs, (int)s, (int)e);
             else build_elementwise_run(p, rs, (int)s, (int)e);
         }
@@ -586,23 +588,18 @@ void Context::build_run(Plan& p, RunSchedule& rs, int first, int end) {
         auto ub = std::upper_bound(v.begin(), v.end(), off);
         return {h, ub == v.begin() ? 0 : *(ub - 1)};
     };
-    // small products (less than a wave of tiles; either little work or no split-K on
-    // their own) gain from sharing a launch; larger ones keep their own kernel choice
+    // products for the tiled kernel share launches of equal pieces of work (plan_tile_work)
     auto groupable = [&](const GemmStep& g) {
         if (routes_split(g) || g.M <= 0 || g.N <= 0 || g.K <= 0) return false;
-        if (kern::fp64_tiles(g.M, g.N) >= 148) return false;
+        if (fp64_tiled_only || kern::skinny_groups(g.M, g.N) == 0) return true;
         // a skinny product (one extent <= 32) with a long operand of 4M elements or more is
         // bandwidth work for the skinny kernel: on a 128 x 64 tile it would use 1/64 to 1/2
         // of every tile (F(ae) += <am||ef> t(fm) at o=16 v=128: 2.3 ms grouped)
-        if (!fp64_tiled_only && std::min(g.M, g.N) <= 32 && (int64_t)std::max(g.M, g.N) * g.K >= (int64_t)1 << 22)
-            return false;
+        if ((int64_t)std::max(g.M, g.N) * g.K >= (int64_t)1 << 22) return false;
         // and so is a skinny product with a long side of a tile or more: the grouped skinny
         // launch streams it (the tiles would stay 1/8 to 1/2 empty and walk it at a fraction
         // of the rate: W~(am,ei) += <am||ef> t(fi) at o=48 v=336 D2h took 16 ms on tiles)
-        if (!fp64_tiled_only && std::min(g.M, g.N) <= 32 && std::max(g.M, g.N) >= 128) return false;
-        // a grouped tile walks the whole K range: long-K products keep their split-K launch
-        if (g.flops() < 4e8 && g.K <= 4096) return true;
-        return kern::fp64_ksplit(g.M, g.N, g.K, !fp64_tiled_only) == 1 && kern::fp64_ksplit(g.M, g.N, g.K, false) == 1;
+        return std::max(g.M, g.N) < 128;
     };
     // short products (both extents <= 64, long K) compute partials on the short kernel and
     // join the fold below, whatever their levels
@@ -615,6 +612,10 @@ void Context::build_run(Plan& p, RunSchedule& rs, int first, int end) {
     auto skinny_groupable = [&](const GemmStep& g) {
         return !fp64_tiled_only && !routes_split(g) && !groupable(g) && kern::skinny_groups(g.M, g.N) > 0 &&
                kern::fp64_ksplit(g.M, g.N, g.K, true) == 1;
+    };
+    // tiled products by operand contiguity (bits 0, 1) and tile size (bit 2: 32 x 32)
+    auto tile_class = [](const GemmStep& g) {
+        return (g.a_kcontig ? 2 : 0) + (g.b_kcontig ? 1 : 0) + (kern::fp64_tile_rows(g.M, g.N) == 32 ? 4 : 0);
     };
     int nskinny = 0;
     std::map<std::pair<int, int64_t>, int> last;
@@ -664,7 +665,7 @@ void Context::build_run(Plan& p, RunSchedule& rs, int first, int end) {
         for (int i = first; i < end; i++)
             if (!merged[i - first] && groupable(p.gemms[p.steps[i].idx])) ngroupable++;
     }
-    if (!any_group && ngroupable < 2 && nshort == 0 && nskinny < 2) return;
+    if (!any_group && ngroupable == 0 && nshort == 0 && nskinny < 2) return;
 
     // Shared-output groups.  Small one-destination products that several levels would
     // serialise (block contractions of a symmetry-blocked statement summing into the same
@@ -730,10 +731,9 @@ void Context::build_run(Plan& p, RunSchedule& rs, int first, int end) {
                 owner = false;
             };
             int64_t off = 0;
-            std::vector<kern::GemmArgs> probs[4];
-            std::vector<int> tstart[4];
-            int tiles[4] = {0, 0, 0, 0};
-            double fl[4] = {0, 0, 0, 0};
+            // by operand contiguity and tile size
+            std::vector<kern::GemmArgs> probs[8];
+            double fl[8] = {0, 0, 0, 0, 0, 0, 0, 0};
             std::map<std::pair<int, int>, std::vector<kern::ShortDesc>> sprobs;
             std::map<std::pair<int, int>, std::vector<int>> sstart;
             std::map<std::pair<int, int>, int> sctas_total;
@@ -765,10 +765,8 @@ void Context::build_run(Plan& p, RunSchedule& rs, int first, int end) {
                     a.ws_elems = (int64_t)g.M * g.N;
                     a.partial_out = true;
                     off += (int64_t)g.M * g.N;
-                    const int c = (g.a_kcontig ? 2 : 0) + (g.b_kcontig ? 1 : 0);
+                    const int c = tile_class(g);
                     probs[c].push_back(a);
-                    tstart[c].push_back(tiles[c]);
-                    tiles[c] += kern::fp64_tiles(g.M, g.N);
                     fl[c] += g.flops();
                 } else if (in_fold[i - first] == 3) {
                     bool lk;
@@ -822,20 +820,11 @@ void Context::build_run(Plan& p, RunSchedule& rs, int first, int end) {
                     sfl[shape] += g.flops();
                 }
             }
-            for (int c = 0; c < 4; c++) {
+            for (int c = 0; c < 8; c++) {
                 if (probs[c].empty()) continue;
-                GemmLaunch l;
-                l.kind = GemmLaunch::GEMM_GROUPED;
-                l.ak = (c & 2) != 0;
-                l.bk = (c & 1) != 0;
-                l.nprob = (int)probs[c].size();
-                l.tiles = tiles[c];
+                GemmLaunch l = group_tiles(probs[c], c & 4 ? 32 : 64, (c & 2) != 0, (c & 1) != 0);
                 l.flops = fl[c];
                 own(l);
-                l.d_probs = (kern::GemmArgs*)dmalloc(probs[c].size() * sizeof(kern::GemmArgs));
-                l.d_tile_start = (int*)dmalloc(tstart[c].size() * sizeof(int));
-                stage_h2d(l.d_probs, probs[c].data(), probs[c].size() * sizeof(kern::GemmArgs));
-                stage_h2d(l.d_tile_start, tstart[c].data(), tstart[c].size() * sizeof(int));
                 run.launches.push_back(l);
             }
             for (auto& kv : sprobs) {
@@ -927,14 +916,14 @@ void Context::build_run(Plan& p, RunSchedule& rs, int first, int end) {
     }
 
     for (int L = 0; L <= maxlvl; L++) {
-        std::vector<int> grp[4];
+        std::vector<int> grp[8];
         std::map<std::pair<int, bool>, std::vector<int>> sk;
         for (int i = first; i < end; i++) {
             if (level[i - first] != L || in_fold[i - first] || merged[i - first]) continue;
             const int gi = p.steps[i].idx;
             const GemmStep& g = p.gemms[gi];
             if (groupable(g)) {
-                grp[(g.a_kcontig ? 2 : 0) + (g.b_kcontig ? 1 : 0)].push_back(gi);
+                grp[tile_class(g)].push_back(gi);
             } else if (skinny_groupable(g)) {
                 const bool lk = g.M >= g.N ? g.a_kcontig : g.b_kcontig;
                 sk[{kern::skinny_groups(g.M, g.N), lk}].push_back(gi);
@@ -945,38 +934,18 @@ void Context::build_run(Plan& p, RunSchedule& rs, int first, int end) {
                 run.launches.push_back(l);
             }
         }
-        for (int c = 0; c < 4; c++) {
+        for (int c = 0; c < 8; c++) {
             if (grp[c].empty()) continue;
-            if (grp[c].size() == 1) {
-                GemmLaunch l;
-                l.gemm = grp[c][0];
-                l.flops = p.gemms[grp[c][0]].flops();
-                run.launches.push_back(l);
-                continue;
-            }
-            GemmLaunch l;
-            l.kind = GemmLaunch::GEMM_GROUPED;
-            l.ak = (c & 2) != 0;
-            l.bk = (c & 1) != 0;
             std::vector<kern::GemmArgs> probs;
-            std::vector<int> tstart;
-            int tiles = 0;
+            double fl = 0;
             for (int gi : grp[c]) {
-                const GemmStep& g = p.gemms[gi];
-                kern::GemmArgs a = gemm_args(p, g);
-                a.ws = nullptr;
-                a.ws_elems = 0;
-                probs.push_back(a);
-                tstart.push_back(tiles);
-                tiles += kern::fp64_tiles(g.M, g.N);
-                l.flops += g.flops();
+                probs.push_back(gemm_args(p, p.gemms[gi]));
+                probs.back().ws = nullptr;
+                probs.back().ws_elems = 0;
+                fl += p.gemms[gi].flops();
             }
-            l.nprob = (int)probs.size();
-            l.tiles = tiles;
-            l.d_probs = (kern::GemmArgs*)dmalloc(probs.size() * sizeof(kern::GemmArgs));
-            l.d_tile_start = (int*)dmalloc(tstart.size() * sizeof(int));
-            stage_h2d(l.d_probs, probs.data(), probs.size() * sizeof(kern::GemmArgs));
-            stage_h2d(l.d_tile_start, tstart.data(), tstart.size() * sizeof(int));
+            GemmLaunch l = group_tiles(probs, c & 4 ? 32 : 64, (c & 2) != 0, (c & 1) != 0);
+            l.flops = fl;
             run.launches.push_back(l);
             any_group = true;
         }
@@ -1019,6 +988,41 @@ void Context::build_run(Plan& p, RunSchedule& rs, int first, int end) {
     if (!any_group) return;
     rs.run_at[first] = (int)rs.runs.size();
     rs.runs.push_back(std::move(run));
+}
+
+void Context::ensure_tile_ws(int64_t elems) {
+    if (elems <= tile_ws_elems) return;
+    // a captured graph may hold the old buffer: it lives as long as the context
+    if (tile_ws) tile_retired.push_back(tile_ws);
+    tile_ws = (double*)dmalloc(elems * sizeof(double));
+    tile_ws_elems = elems;
+}
+
+// one launch of the tiled kernel over these problems, its work laid out and uploaded
+GemmLaunch Context::group_tiles(const std::vector<kern::GemmArgs>& probs, int rows, bool ak, bool bk) {
+    GemmLaunch l;
+    l.kind = GemmLaunch::GEMM_GROUPED;
+    l.ak = ak;
+    l.bk = bk;
+    l.rows = rows;
+    l.nprob = (int)probs.size();
+    std::vector<kern::TileProblem> shapes;
+    for (auto& g : probs) shapes.push_back({g.M, g.N, g.K});
+    const kern::TileWork w = kern::plan_tile_work(shapes, rows, true);
+    l.nctas = (int)w.seg_start.size() - 1;
+    l.nfolds = (int)w.folds.size();
+    l.slots = w.slots;
+    if (w.slots > 0) ensure_tile_ws(kern::tile_ws_elems(w.slots, rows));
+    l.d_probs = (kern::GemmArgs*)dmalloc(probs.size() * sizeof(kern::GemmArgs));
+    stage_h2d(l.d_probs, probs.data(), probs.size() * sizeof(kern::GemmArgs));
+    l.at_start = w.segs.size() * sizeof(kern::TileSeg);
+    l.at_folds = l.at_start + w.seg_start.size() * sizeof(int);
+    l.desc_bytes = l.at_folds + w.folds.size() * sizeof(kern::TileFold);
+    l.d_desc = dmalloc(l.desc_bytes);
+    stage_h2d(l.d_desc, w.segs.data(), l.at_start);
+    stage_h2d((char*)l.d_desc + l.at_start, w.seg_start.data(), l.at_folds - l.at_start);
+    stage_h2d((char*)l.d_desc + l.at_folds, w.folds.data(), l.desc_bytes - l.at_folds);
+    return l;
 }
 
 // A run of permuted sums or of scalings of one statement.  Sums read their A blocks (an
@@ -1175,7 +1179,9 @@ void Context::launch(Plan& p, const GemmLaunch& l, const std::string& label, dou
         case GemmLaunch::MERGED_SPLIT: run_merged(p, *l.merged, label); break;
         case GemmLaunch::GEMM: run_gemm(p, p.gemms[l.gemm]); break;
         case GemmLaunch::GEMM_GROUPED:
-            kern::gemm_fp64_grouped(l.d_probs, l.d_tile_start, l.nprob, l.tiles, l.ak, l.bk, stream);
+            kern::gemm_fp64_grouped(l.d_probs, (const kern::TileSeg*)l.d_desc, (const int*)((char*)l.d_desc + l.at_start),
+                                    l.nctas, (const kern::TileFold*)((char*)l.d_desc + l.at_folds), l.nfolds, tile_ws,
+                                    l.rows, l.ak, l.bk, stream);
             break;
         case GemmLaunch::DOT_BATCHED:
             kern::dot_batched((const kern::DotDesc*)l.d_desc, l.d_chunks, l.nprob, l.chunks, l.d_part, dot_acc, stream);

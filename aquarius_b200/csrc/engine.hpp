@@ -192,7 +192,10 @@ struct GemmLaunch {
                                        // grouped skinny: nt n-groups, ak = L contiguous along k
                                        // (d_desc: SkinnyArgs[nprob])
     int nprob = 0, tiles = 0;
-    kern::GemmArgs* d_probs = nullptr;
+    kern::GemmArgs* d_probs = nullptr; // grouped GEMM: problems and, in d_desc, their TileSeg[], the
+    int rows = 64, nctas = 0;          // CTAs' first segments and the TileFold[] of shared tiles
+    int nfolds = 0, slots = 0;
+    size_t at_start = 0, at_folds = 0; // byte offsets of the two in d_desc
     int* d_tile_start = nullptr;
     double* d_part = nullptr;          // shared-output group: partial products (part_elems doubles)
     int64_t part_elems = 0;
@@ -319,6 +322,11 @@ public:
     double* merged_ws = nullptr;                           // dense products of merged launches
     int64_t merged_ws_elems = 0;
     std::vector<double*> merged_retired;                   // outgrown, kept until the context goes
+    double* tile_ws = nullptr;                             // partial tiles of grouped FP64 launches
+    int64_t tile_ws_elems = 0;
+    std::vector<double*> tile_retired;                     // outgrown, kept until the context goes
+    void ensure_tile_ws(int64_t elems);
+    GemmLaunch group_tiles(const std::vector<kern::GemmArgs>& probs, int rows, bool ak, bool bk);
     void build_merged(Plan& p, GemmRun& run, int first, int end, std::vector<char>& merged,
                       const std::function<std::pair<int, int64_t>(int, int64_t)>& block_of);
     void run_merged(Plan& p, MergedProduct& m, const std::string& label);

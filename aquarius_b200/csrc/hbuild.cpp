@@ -114,8 +114,7 @@ struct Builder {
             Tables tb{ctx, {}};
             const int64_t* d = tb.up(all);
             std::vector<kern::GemmArgs> probs;
-            std::vector<int> tstart;
-            int tiles = 0;
+            std::vector<kern::TileProblem> shapes;
             size_t q = 0;
             for (auto& pc : lv) {
                 kern::GemmArgs a;
@@ -133,16 +132,19 @@ struct Builder {
                 a.Cm[0] = d + at[q++];
                 a.Cn[0] = d + at[q++];
                 probs.push_back(a);
-                tstart.push_back(tiles);
-                tiles += kern::fp64_tiles(pc.M, pc.N);
+                shapes.push_back({pc.M, pc.N, pc.K});
             }
-            kern::GemmArgs* dp = (kern::GemmArgs*)ctx.dmalloc(probs.size() * sizeof(kern::GemmArgs));
-            int* dt = (int*)ctx.dmalloc(tstart.size() * sizeof(int));
-            ctx.stage_h2d(dp, probs.data(), probs.size() * sizeof(kern::GemmArgs));
-            ctx.stage_h2d(dt, tstart.data(), tstart.size() * sizeof(int));
-            kern::gemm_fp64_grouped(dp, dt, (int)probs.size(), tiles, false, false, ctx.stream);
-            ctx.dfree(dp, probs.size() * sizeof(kern::GemmArgs));
-            ctx.dfree(dt, tstart.size() * sizeof(int));
+            // one launch per tile size; k runs over the auxiliary functions, so no tile is split
+            const kern::GemmArgs* dp = tb.up(probs);
+            for (int rows : {32, 64}) {
+                std::vector<kern::TileProblem> part = shapes;
+                for (auto& x : part)
+                    if (kern::fp64_tile_rows(x.M, x.N) != rows) x = kern::TileProblem();
+                const kern::TileWork w = kern::plan_tile_work(part, rows, false);
+                if (w.segs.empty()) continue;
+                kern::gemm_fp64_grouped(dp, tb.up(w.segs), tb.up(w.seg_start), (int)w.seg_start.size() - 1, nullptr, 0,
+                                        nullptr, rows, false, false, ctx.stream);
+            }
             lv.clear();
         }
     }

@@ -2,6 +2,7 @@
 #pragma once
 #include <cstdint>
 #include <utility>
+#include <vector>
 #include <cuda_runtime.h>
 
 namespace ccsd {
@@ -111,13 +112,34 @@ int fp64_ksplit(int M, int N, int K, bool skinny_ok = true);
 
 // native FP64 tensor-core (DMMA) GETT kernel
 void gemm_fp64(const GemmArgs& g, cudaStream_t s);
-// output tiles of the tiled FP64 kernel for an M x N product
-int fp64_tiles(int M, int N);
-// One launch of the tiled FP64 kernel over nprob problems (device array of GemmArgs, all
-// with the given operand contiguity, no split-K, pairwise disjoint outputs); tile_start
-// (device, nprob entries) holds each problem's first tile.
-void gemm_fp64_grouped(const GemmArgs* probs, const int* tile_start, int nprob, int total_tiles, bool a_kcontig,
-                       bool b_kcontig, cudaStream_t s);
+// One launch of the tiled FP64 kernel over many problems (device array of GemmArgs, all with
+// the given operand contiguity, pairwise disjoint outputs).  The work is laid out on the
+// host: a CTA's segments are segs[seg_start[cta] .. seg_start[cta + 1]), each a tile of a
+// problem and a range of its k chunks; a tile that several CTAs share leaves one partial
+// tile per part in ws (slots slot0, slot0 + 1, ... in order of k), added by a second launch.
+struct TileProblem {
+    int M = 0, N = 0, K = 0;
+};
+struct TileSeg {
+    int prob = 0, m0 = 0, n0 = 0, kt0 = 0, nkt = 0, slot = -1;
+};
+struct TileFold {
+    int prob = 0, m0 = 0, n0 = 0, slot0 = 0, parts = 0;
+};
+struct TileWork {
+    int rows = 64, slots = 0;
+    std::vector<TileSeg> segs;
+    std::vector<int> seg_start;        // CTAs + 1 entries
+    std::vector<TileFold> folds;
+};
+// tile edge (32 or 64) for an M x N product
+int fp64_tile_rows(int M, int N);
+// split: tiles may be shared by CTAs (needs tile_ws_elems(slots, rows) doubles of ws)
+TileWork plan_tile_work(const std::vector<TileProblem>& probs, int rows, bool split);
+int64_t tile_ws_elems(int slots, int rows);
+void gemm_fp64_grouped(const GemmArgs* probs, const TileSeg* segs, const int* seg_start, int nctas,
+                       const TileFold* folds, int nfolds, double* ws, int rows, bool a_kcontig, bool b_kcontig,
+                       cudaStream_t s);
 
 // ---- split (Ozaki-style) path ----------------------------------------------------
 // Slice kinds: BF16 slices of 8 significant bits (3 or 4 per operand, FP32 tensor

@@ -42,22 +42,41 @@ void set_smem_once(const void* kernel, int bytes) {
 // ---------------------------------------------------------------------------
 namespace {
 
-constexpr int BM = 128, BN = 64, BK = 16, STAGES = 3, THREADS = 256;
-constexpr int LDMK = BM + 8;   // A stored [k][m]
-constexpr int LDNK = BN + 8;   // B stored [k][n]
-constexpr int LDK = BK + 4;    // operands stored [m][k] / [n][k]
+constexpr int BK = 16;                  // k per chunk
+constexpr int TILE_THREADS = 128;       // 2 x 2 warps, each a quarter of the tile
 
-template <bool AK, bool BK_>
-struct Smem {
-    static constexpr int a_elems = AK ? BM * LDK : BK * LDMK;
-    static constexpr int b_elems = BK_ ? BN * LDK : BK * LDNK;
-    static constexpr size_t bytes = (size_t)STAGES * (a_elems + b_elems) * sizeof(double) + (BM + BN) * sizeof(int64_t);
+// Tile shapes.  The FP64 tensor pipe (36.8 TFLOP/s measured for m8n8k4) bounds large
+// products.  64 x 64 (32 x 32 per warp, 64 accumulator registers) leaves room for four CTAs
+// of four warps per SM, whose barriers and copy latencies hide behind one another's
+// products: 28.6 TFLOP/s at M=25600 N=400 K=4096 and 29.9 at 2048^3 (pipe 83% busy),
+// against 25.4 for 128 x 64 tiles with two CTAs per SM and 18.5-22.7 for 128 x 128 with one;
+// the 128 x 64 kernel with one CTA per SM before it ran the ladder of o=20 v=160 at 13.5.
+// With extents that leave every other pair misaligned (8-byte copies) it keeps 22.3.
+// 32 x 32 (16 x 16 per warp) takes the products that would leave a 64 x 64 tile mostly empty.
+template <int ROWS>
+struct Tile {
+    static constexpr int BM = ROWS, BN = ROWS, WM = ROWS / 2, WN = ROWS / 2, STAGES = 3;
+    static constexpr int MT = WM / 8, NT = WN / 8;
+    static constexpr int PER_SM = ROWS == 64 ? 4 : 8;
+    static constexpr int LD = ROWS + 2;                 // [k][row] layout: 2 mod 8 doubles
+    static constexpr int ELEMS = BM * BN;
+};
+
+template <class T, bool AK, bool BKc>
+struct TileSmem {
+    static constexpr int a_elems = AK ? T::BM * BK : BK * T::LD;
+    static constexpr int b_elems = BKc ? T::BN * BK : BK * T::LD;
+    static constexpr size_t bytes = (size_t)T::STAGES * (a_elems + b_elems) * sizeof(double) + 2 * 2 * BK * sizeof(int64_t);
 };
 
 __device__ __forceinline__ void cp_async8(void* smem, const void* gmem, bool valid) {
     unsigned s = (unsigned)__cvta_generic_to_shared(smem);
     int sz = valid ? 8 : 0;
     asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;\n" ::"r"(s), "l"(gmem), "r"(sz));
+}
+__device__ __forceinline__ void cp_async16(void* smem, const void* gmem) {
+    unsigned s = (unsigned)__cvta_generic_to_shared(smem);
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(s), "l"(gmem));
 }
 __device__ __forceinline__ void cp_commit() { asm volatile("cp.async.commit_group;\n" ::); }
 template <int N>
@@ -69,203 +88,319 @@ __device__ __forceinline__ void dmma(double& d0, double& d1, double a, double b)
                  : "d"(a), "d"(b));
 }
 
-// One BM x BN output tile of one problem, K-range kz of nz (split-K writes raw partials
-// to g.ws[kz]).  smem_raw: the dynamic shared memory of Smem<AK, BKc>.
-template <bool AK, bool BKc>
-__device__ __forceinline__ void fp64_tile(const GemmArgs& g, const int m0, const int n0, const int kz, const int nz,
-                                          unsigned char* smem_raw) {
-    using S = Smem<AK, BKc>;
+// [row][k] tiles: 16 k = eight 16-byte units per row, unit XOR 4 on odd rows, so that the
+// 16-byte fragment reads of a quarter warp (2 rows x 4 units) fall on different banks
+__device__ __forceinline__ int tile_rk(int r, int k) { return r * BK + (k ^ ((r & 1) << 3)); }
+
+// Copies one operand's rows x BK tiles into shared memory, two neighbours at a time (along
+// k where the operand is contiguous there, else along the rows): one 16-byte copy where the
+// two are adjacent and aligned, two 8-byte copies otherwise.  A thread's rows are the same
+// for every chunk and stay in registers; the chunk's k offsets come from shared memory.
+template <int ROWS, int LD, bool KC>
+struct TileLoader {
+    static constexpr int N = ROWS * BK / 2 / TILE_THREADS;   // pairs per thread
+    static constexpr int NR = KC ? N : 2;
+    int64_t row[NR];                                         // -1 past the last row
+    bool adj = true;                                         // the two rows of a pair are adjacent
+    __device__ __forceinline__ void init(const int64_t* __restrict__ R, int r0, int nrows, int64_t parity) {
+        const int tid = threadIdx.x;
+        if (KC) {
+#pragma unroll
+            for (int i = 0; i < N; i++) {
+                const int r = r0 + tid / (BK / 2) + (TILE_THREADS / (BK / 2)) * i;
+                row[i] = r < nrows ? __ldg(R + r) + parity : -1;
+            }
+        } else {
+            const int r = r0 + 2 * (tid % (ROWS / 2));
+            row[0] = r < nrows ? __ldg(R + r) + parity : -1;
+            row[1] = r + 1 < nrows ? __ldg(R + r + 1) + parity : -1;
+            adj = row[0] >= 0 && row[1] == row[0] + 1;
+        }
+    }
+    // X is the operand moved down to a 16-byte boundary (the parity sits in the row
+    // offsets); tab holds the chunk's BK offsets, -1 past K
+    __device__ __forceinline__ void copy(double* dst, const double* __restrict__ X, const int64_t* tab) const {
+        const int tid = threadIdx.x;
+#pragma unroll
+        for (int i = 0; i < N; i++) {
+            int64_t o0, o1;
+            bool v0, v1;
+            double* d;
+            if (KC) {
+                const int k = 2 * (tid % (BK / 2)), r = tid / (BK / 2) + (TILE_THREADS / (BK / 2)) * i;
+                const int64_t k0 = tab[k], k1 = tab[k + 1];
+                o0 = row[i] + k0;
+                o1 = row[i] + k1;
+                v0 = (row[i] | k0) >= 0;
+                v1 = (row[i] | k1) >= 0;
+                d = dst + tile_rk(r, k);
+            } else {
+                const int k = tid / (ROWS / 2) + (TILE_THREADS / (ROWS / 2)) * i;
+                const int64_t kk = tab[k];
+                o0 = row[0] + kk;
+                o1 = row[1] + kk;
+                v0 = (row[0] | kk) >= 0;
+                v1 = (row[1] | kk) >= 0;
+                d = dst + k * LD + 2 * (tid % (ROWS / 2));
+            }
+            if (v0 && v1 && (KC ? o1 == o0 + 1 : adj) && !(o0 & 1)) {
+                cp_async16(d, X + o0);
+            } else {
+                cp_async8(d, v0 ? X + o0 : X, v0);
+                cp_async8(d + 1, v1 ? X + o1 : X, v1);
+            }
+        }
+    }
+};
+
+template <class T>
+struct TileAcc {
+    double v[T::MT][T::NT][2];
+};
+
+// Row / column of the tile that accumulator (i, j, c) of this lane holds.  Operands stored
+// [k][row] are read two neighbouring rows at a time, which interleaves the rows of two
+// 8-row fragments.
+template <class T, bool AK>
+__device__ __forceinline__ int tile_row(int i) {
+    const int warp = threadIdx.x >> 5, fr = (threadIdx.x & 31) >> 2;
+    return (warp & 1) * T::WM + (AK ? 8 * i + fr : 16 * (i >> 1) + 2 * fr + (i & 1));
+}
+template <class T, bool BKc>
+__device__ __forceinline__ int tile_col(int j, int c) {
+    const int warp = threadIdx.x >> 5, fk = threadIdx.x & 3;
+    return (warp >> 1) * T::WN + (BKc ? 8 * j + 2 * fk + c : 16 * (j >> 1) + 4 * fk + 2 * c + (j & 1));
+}
+
+// Chunks [kt0, kt0 + nkt) of the tile at (m0, n0) into acc.  Three stages of cp.async; the
+// k offsets of a chunk are fetched to a register two chunks ahead of the chunk's copies and
+// staged in shared memory one chunk ahead, so no copy waits on a table load.  Within an
+// 8-k block a lane takes k = 2 (lane % 4) and the next one: 16-byte fragment reads, the
+// same permutation of k for both operands.
+template <class T, bool AK, bool BKc>
+__device__ __forceinline__ void tile_product(const GemmArgs& g, int m0, int n0, int kt0, int nkt, TileAcc<T>& acc,
+                                             unsigned char* smem_raw) {
+    using S = TileSmem<T, AK, BKc>;
+    constexpr int MT = T::MT, NT = T::NT, STAGES = T::STAGES;
     double* As = reinterpret_cast<double*>(smem_raw);
     double* Bs = As + STAGES * S::a_elems;
-    int64_t* sAm = reinterpret_cast<int64_t*>(Bs + STAGES * S::b_elems);
-    int64_t* sBn = sAm + BM;
-
+    int64_t* tab = reinterpret_cast<int64_t*>(Bs + STAGES * S::b_elems);   // [2][A | B][BK]
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const int wm = (warp & 3) * 32, wn = (warp >> 2) * 32;
-
-    for (int i = tid; i < BM; i += THREADS) sAm[i] = (m0 + i < g.M) ? g.Am[m0 + i] : 0;
-    for (int i = tid; i < BN; i += THREADS) sBn[i] = (n0 + i < g.N) ? g.Bn[n0 + i] : 0;
-    __syncthreads();
-
-    // this CTA's K-range (split-K: range kz of nz)
-    const int ktiles_all = (g.K + BK - 1) / BK;
-    const int per_split = (ktiles_all + nz - 1) / nz;
-    const int kt0 = kz * per_split;
-    const int ktiles = max(0, min(ktiles_all, kt0 + per_split) - kt0);
-
-    auto load_stage = [&](int stage, int kt) {
-        const int k0 = kt * BK;
-        double* as = As + stage * S::a_elems;
-        double* bs = Bs + stage * S::b_elems;
-        // A tile: BM x BK
-#pragma unroll
-        for (int i = 0; i < (BM * BK) / THREADS; i++) {
-            int e = tid + i * THREADS;
-            int m, k;
-            if (AK) { k = e % BK; m = e / BK; }
-            else    { m = e % BM; k = e / BM; }
-            bool ok = (m0 + m < g.M) && (k0 + k < g.K);
-            const double* src =
-                ok ? g.A + sAm[m] + (g.ak_affine ? g.ak0 + g.ak_step * (k0 + k) : __ldg(g.Ak + k0 + k)) : g.A;
-            double* dst = AK ? as + m * LDK + k : as + k * LDMK + m;
-            cp_async8(dst, src, ok);
-        }
-        // B tile: BK x BN
-#pragma unroll
-        for (int i = 0; i < (BN * BK) / THREADS; i++) {
-            int e = tid + i * THREADS;
-            int n, k;
-            if (BKc) { k = e % BK; n = e / BK; }
-            else     { n = e % BN; k = e / BN; }
-            bool ok = (n0 + n < g.N) && (k0 + k < g.K);
-            const double* src =
-                ok ? g.B + sBn[n] + (g.bk_affine ? g.bk0 + g.bk_step * (k0 + k) : __ldg(g.Bk + k0 + k)) : g.B;
-            double* dst = BKc ? bs + n * LDK + k : bs + k * LDNK + n;
-            cp_async8(dst, src, ok);
-        }
+    const int wm = (warp & 1) * T::WM, wn = (warp >> 1) * T::WN;
+    const int64_t pa = (reinterpret_cast<uintptr_t>(g.A) >> 3) & 1, pb = (reinterpret_cast<uintptr_t>(g.B) >> 3) & 1;
+    const double* A = g.A - pa;
+    const double* B = g.B - pb;
+    TileLoader<T::BM, T::LD, AK> la;
+    TileLoader<T::BN, T::LD, BKc> lb;
+    la.init(g.Am, m0, g.M, pa);
+    lb.init(g.Bn, n0, g.N, pb);
+    const int64_t* kt_src = tid < BK ? g.Ak : g.Bk;
+    const int K = g.K;
+    auto fetch = [&](int c) -> int64_t {
+        const int k = (kt0 + c) * BK + (tid & (BK - 1));
+        return (tid < 2 * BK && k < K) ? __ldg(kt_src + k) : -1;
     };
+    auto put = [&](int c, int64_t v) {
+        if (tid < 2 * BK) tab[(c & 1) * 2 * BK + tid] = v;
+    };
+    auto load = [&](int c) {
+        const int64_t* t = tab + (c & 1) * 2 * BK;
+        la.copy(As + (c % STAGES) * S::a_elems, A, t);
+        lb.copy(Bs + (c % STAGES) * S::b_elems, B, t + BK);
+    };
+#pragma unroll
+    for (int i = 0; i < MT; i++)
+#pragma unroll
+        for (int j = 0; j < NT; j++) acc.v[i][j][0] = acc.v[i][j][1] = 0.0;
 
-    double acc[4][4][2];
+    int64_t next = fetch(0);
 #pragma unroll
-    for (int i = 0; i < 4; i++)
-#pragma unroll
-        for (int j = 0; j < 4; j++) acc[i][j][0] = acc[i][j][1] = 0.0;
-
-#pragma unroll
-    for (int s = 0; s < STAGES - 1; s++) {
-        if (s < ktiles) load_stage(s, kt0 + s);
+    for (int c = 0; c < STAGES - 1; c++) {
+        put(c, next);
+        next = fetch(c + 1);
+        __syncthreads();
+        if (c < nkt) load(c);
         cp_commit();
     }
-
-    for (int kt = 0; kt < ktiles; kt++) {
+    put(STAGES - 1, next);
+    next = fetch(STAGES);
+    const int fr = lane >> 2, fk = lane & 3;
+    for (int kt = 0; kt < nkt; kt++) {
         cp_wait<STAGES - 2>();
         __syncthreads();
-        {
-            int nk = kt + STAGES - 1;
-            if (nk < ktiles) load_stage(nk % STAGES, kt0 + nk);
-            cp_commit();
-        }
+        if (kt + STAGES - 1 < nkt) load(kt + STAGES - 1);
+        cp_commit();
+        put(kt + STAGES, next);
+        next = fetch(kt + STAGES + 1);
         const double* as = As + (kt % STAGES) * S::a_elems;
         const double* bs = Bs + (kt % STAGES) * S::b_elems;
 #pragma unroll
-        for (int kk = 0; kk < BK; kk += 4) {
-            double af[4], bf[4];
-            const int kr = kk + (lane & 3);
+        for (int kb = 0; kb < BK; kb += 8) {
+            double af[2][MT], bf[2][NT];     // [k of the lane's pair][fragment]
+            if (AK) {
 #pragma unroll
-            for (int i = 0; i < 4; i++) {
-                int m = wm + i * 8 + (lane >> 2);
-                af[i] = AK ? as[m * LDK + kr] : as[kr * LDMK + m];
+                for (int i = 0; i < MT; i++) {
+                    const double2 v = *reinterpret_cast<const double2*>(as + tile_rk(wm + 8 * i + fr, kb + 2 * fk));
+                    af[0][i] = v.x;
+                    af[1][i] = v.y;
+                }
+            } else {
+#pragma unroll
+                for (int s = 0; s < 2; s++)
+#pragma unroll
+                    for (int i = 0; i < MT; i += 2) {
+                        const double2 v = *reinterpret_cast<const double2*>(as + (kb + 2 * fk + s) * T::LD + wm + 8 * i + 2 * fr);
+                        af[s][i] = v.x;
+                        af[s][i + 1] = v.y;
+                    }
+            }
+            if (BKc) {
+#pragma unroll
+                for (int j = 0; j < NT; j++) {
+                    const double2 v = *reinterpret_cast<const double2*>(bs + tile_rk(wn + 8 * j + fr, kb + 2 * fk));
+                    bf[0][j] = v.x;
+                    bf[1][j] = v.y;
+                }
+            } else {
+#pragma unroll
+                for (int s = 0; s < 2; s++)
+#pragma unroll
+                    for (int j = 0; j < NT; j += 2) {
+                        const double2 v = *reinterpret_cast<const double2*>(bs + (kb + 2 * fk + s) * T::LD + wn + 8 * j + 2 * fr);
+                        bf[s][j] = v.x;
+                        bf[s][j + 1] = v.y;
+                    }
             }
 #pragma unroll
-            for (int j = 0; j < 4; j++) {
-                int n = wn + j * 8 + (lane >> 2);
-                bf[j] = BKc ? bs[n * LDK + kr] : bs[kr * LDNK + n];
-            }
+            for (int s = 0; s < 2; s++)
 #pragma unroll
-            for (int i = 0; i < 4; i++)
+                for (int i = 0; i < MT; i++)
 #pragma unroll
-                for (int j = 0; j < 4; j++) dmma(acc[i][j][0], acc[i][j][1], af[i], bf[j]);
+                    for (int j = 0; j < NT; j++) dmma(acc.v[i][j][0], acc.v[i][j][1], af[s][i], bf[s][j]);
         }
     }
     cp_wait<0>();
+}
 
-    if (nz > 1 || g.partial_out) {
-        // split-K (or a shared-output group): raw partial sums, folded by splitk_fold_kernel
-        // (fold_groups_kernel)
-        double* wz = g.ws + (int64_t)kz * g.M * g.N;
+// one row of fragments of a finished tile: raw to a dense product, or scattered into C
+template <class T, bool AK, bool BKc>
+__device__ __forceinline__ void tile_write_row(const GemmArgs& g, int m0, int n0, int i, const double (&v)[T::NT][2],
+                                               double* dense) {
+    constexpr int NT = T::NT;
+    const int m = m0 + tile_row<T, AK>(i);
+    if (m >= g.M) return;
+    if (dense) {
+        double* w = dense + (int64_t)m * g.N;
 #pragma unroll
-        for (int i = 0; i < 4; i++) {
-            int m = m0 + wm + i * 8 + (lane >> 2);
-            if (m >= g.M) continue;
+        for (int j = 0; j < NT; j++)
 #pragma unroll
-            for (int j = 0; j < 4; j++)
-#pragma unroll
-                for (int h = 0; h < 2; h++) {
-                    int n = n0 + wn + j * 8 + 2 * (lane & 3) + h;
-                    if (n < g.N) wz[(int64_t)m * g.N + n] = acc[i][j][h];
-                }
-        }
+            for (int c = 0; c < 2; c++) {
+                const int n = n0 + tile_col<T, BKc>(j, c);
+                if (n < g.N) w[n] = v[j][c];
+            }
         return;
     }
-
     if (g.nvm == 1 && g.nvn == 1) {
-        // one destination per element: the 8 read-modify-writes of a row group are
-        // issued as 8 reads, then 8 writes (overlapped instead of one by one)
+        // one destination per element: the reads of the row first, then its writes, so that
+        // the read-modify-writes of a thread overlap instead of running one by one
+        const int64_t cm = __ldg(g.Cm[0] + m);
+        const double sc = g.alpha * g.vsign[0];
+        int64_t off[2 * NT];
+        double old[2 * NT];
 #pragma unroll
-        for (int i = 0; i < 4; i++) {
-            const int m = m0 + wm + i * 8 + (lane >> 2);
-            if (m >= g.M) continue;
-            const int64_t cm = g.Cm[0][m];
-            const double sc = g.alpha * g.vsign[0];
-            int64_t off[8];
-            double old[8];
-#pragma unroll
-            for (int t = 0; t < 8; t++) {
-                const int n = n0 + wn + (t >> 1) * 8 + 2 * (lane & 3) + (t & 1);
-                off[t] = n < g.N ? cm + g.Cn[0][n] : -1;
-            }
-#pragma unroll
-            for (int t = 0; t < 8; t++) old[t] = off[t] >= 0 ? g.C[off[t]] : 0.0;
-#pragma unroll
-            for (int t = 0; t < 8; t++)
-                if (off[t] >= 0) g.C[off[t]] = old[t] + sc * acc[i][t >> 1][t & 1];
+        for (int t = 0; t < 2 * NT; t++) {
+            const int n = n0 + tile_col<T, BKc>(t >> 1, t & 1);
+            off[t] = n < g.N ? cm + __ldg(g.Cn[0] + n) : -1;
         }
+#pragma unroll
+        for (int t = 0; t < 2 * NT; t++) old[t] = off[t] >= 0 ? g.C[off[t]] : 0.0;
+#pragma unroll
+        for (int t = 0; t < 2 * NT; t++)
+            if (off[t] >= 0) g.C[off[t]] = old[t] + sc * v[t >> 1][t & 1];
         return;
     }
-    // epilogue: scatter to every destination variant
+    // every destination variant in turn
 #pragma unroll
-    for (int i = 0; i < 4; i++) {
-        int m = m0 + wm + i * 8 + (lane >> 2);
-        if (m >= g.M) continue;
-        int64_t cm[2];
-        cm[0] = g.Cm[0][m];
-        cm[1] = g.nvm > 1 ? g.Cm[1][m] : 0;
+    for (int j = 0; j < NT; j++)
 #pragma unroll
-        for (int j = 0; j < 4; j++) {
-#pragma unroll
-            for (int h = 0; h < 2; h++) {
-                int n = n0 + wn + j * 8 + 2 * (lane & 3) + h;
-                if (n >= g.N) continue;
-                double v = g.alpha * acc[i][j][h];
-                for (int a = 0; a < g.nvm; a++)
-                    for (int b = 0; b < g.nvn; b++) {
-                        double* dst = g.C + cm[a] + g.Cn[b][n];
-                        *dst += g.vsign[a * g.nvn + b] * v;
-                    }
-            }
+        for (int c = 0; c < 2; c++) {
+            const int n = n0 + tile_col<T, BKc>(j, c);
+            if (n >= g.N) continue;
+            const double x = g.alpha * v[j][c];
+            for (int a = 0; a < g.nvm; a++)
+                for (int b = 0; b < g.nvn; b++) g.C[g.Cm[a][m] + g.Cn[b][n]] += g.vsign[a * g.nvn + b] * x;
         }
-    }
 }
 
-template <bool AK, bool BKc>
-__global__ void __launch_bounds__(THREADS, 1) gemm_fp64_kernel(GemmArgs g) {
+// One problem, one CTA per output tile and K range (blockIdx.y of gridDim.y; more than one
+// range, or partial_out, writes raw products to g.ws[z][m][n]).  The shorter side of the
+// tile grid runs fastest, so that the CTAs in flight share the panels of the longer operand.
+template <class T, bool AK, bool BKc>
+__global__ void __launch_bounds__(TILE_THREADS, T::PER_SM) gemm_fp64_kernel(GemmArgs g) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    fp64_tile<AK, BKc>(g, blockIdx.y * BM, blockIdx.x * BN, blockIdx.z, gridDim.z, smem_raw);
-}
-
-// Grouped launch: one CTA per output tile of any of nprob problems whose outputs are
-// pairwise disjoint; tile_start[p] is the first tile of problem p.
-template <bool AK, bool BKc>
-__global__ void __launch_bounds__(THREADS, 1)
-    gemm_fp64_grouped_kernel(const GemmArgs* __restrict__ probs, const int* __restrict__ tile_start, int nprob) {
-    extern __shared__ __align__(16) unsigned char smem_raw[];
-    __shared__ GemmArgs sg;
-    __shared__ int sp;
+    const int tm = (g.M + T::BM - 1) / T::BM, tn = (g.N + T::BN - 1) / T::BN;
     const int t = blockIdx.x;
-    if (threadIdx.x == 0) {
-        int lo = 0, hi = nprob - 1;
-        while (lo < hi) {
-            const int mid = (lo + hi + 1) >> 1;
-            if (tile_start[mid] <= t) lo = mid;
-            else hi = mid - 1;
+    const int m0 = (tm <= tn ? t % tm : t / tn) * T::BM, n0 = (tm <= tn ? t / tm : t % tn) * T::BN;
+    const int chunks = (g.K + BK - 1) / BK, per = (chunks + gridDim.y - 1) / gridDim.y;
+    const int kt0 = blockIdx.y * per;
+    TileAcc<T> acc;
+    tile_product<T, AK, BKc>(g, m0, n0, kt0, max(0, min(chunks, kt0 + per) - kt0), acc, smem_raw);
+    double* dense = gridDim.y > 1 || g.partial_out ? g.ws + (int64_t)blockIdx.y * g.M * g.N : nullptr;
+#pragma unroll
+    for (int i = 0; i < T::MT; i++) tile_write_row<T, AK, BKc>(g, m0, n0, i, acc.v[i], dense);
+}
+
+// Many problems with pairwise disjoint outputs: each CTA walks its segments (a tile and a
+// range of its chunks, laid out by plan_tile_work).  A segment that covers its tile writes
+// the output; one that shares its tile with other CTAs leaves its accumulators in slot
+// seg.slot of ws, in register order.
+template <class T, bool AK, bool BKc>
+__global__ void __launch_bounds__(TILE_THREADS, T::PER_SM)
+    gemm_fp64_grouped_kernel(const GemmArgs* __restrict__ probs, const TileSeg* __restrict__ segs,
+                             const int* __restrict__ seg_start, double* __restrict__ ws) {
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    const int s1 = seg_start[blockIdx.x + 1];
+    for (int s = seg_start[blockIdx.x]; s < s1; s++) {
+        const TileSeg seg = segs[s];
+        const GemmArgs& g = probs[seg.prob];
+        TileAcc<T> acc;
+        tile_product<T, AK, BKc>(g, seg.m0, seg.n0, seg.kt0, seg.nkt, acc, smem_raw);
+        if (seg.slot >= 0) {
+            double* w = ws + (int64_t)seg.slot * T::ELEMS + threadIdx.x;
+#pragma unroll
+            for (int i = 0; i < T::MT; i++)
+#pragma unroll
+                for (int j = 0; j < T::NT; j++)
+#pragma unroll
+                    for (int c = 0; c < 2; c++) w[((i * T::NT + j) * 2 + c) * TILE_THREADS] = acc.v[i][j][c];
+        } else {
+            double* dense = g.partial_out ? g.ws : nullptr;
+#pragma unroll
+            for (int i = 0; i < T::MT; i++) tile_write_row<T, AK, BKc>(g, seg.m0, seg.n0, i, acc.v[i], dense);
         }
-        sp = lo;
-        sg = probs[lo];
+        __syncthreads();   // the stages and the offset table are free for the next segment
     }
-    __syncthreads();
-    const int local = t - tile_start[sp];
-    const int tn = (sg.N + BN - 1) / BN;
-    fp64_tile<AK, BKc>(sg, (local / tn) * BM, (local % tn) * BN, 0, 1, smem_raw);
+}
+
+// The tiles that several CTAs share: blockIdx.y's row of fragments of tile blockIdx.x, its
+// parts added in order of k
+template <class T, bool AK, bool BKc>
+__global__ void __launch_bounds__(TILE_THREADS)
+    tile_fold_kernel(const GemmArgs* __restrict__ probs, const TileFold* __restrict__ folds, const double* __restrict__ ws) {
+    const TileFold f = folds[blockIdx.x];
+    const GemmArgs& g = probs[f.prob];
+    const int i = blockIdx.y;
+    const double* w = ws + (int64_t)f.slot0 * T::ELEMS + (int64_t)i * T::NT * 2 * TILE_THREADS + threadIdx.x;
+    double v[T::NT][2];
+#pragma unroll
+    for (int j = 0; j < T::NT; j++) v[j][0] = v[j][1] = 0.0;
+#pragma unroll 4
+    for (int p = 0; p < f.parts; p++, w += T::ELEMS)
+#pragma unroll
+        for (int j = 0; j < T::NT; j++)
+#pragma unroll
+            for (int c = 0; c < 2; c++) v[j][c] += w[(j * 2 + c) * TILE_THREADS];
+    tile_write_row<T, AK, BKc>(g, f.m0, f.n0, i, v, g.partial_out ? g.ws : nullptr);
 }
 
 // shared-output groups: each CTA folds the partial products of one group of output blocks,
@@ -329,11 +464,6 @@ struct SkinnyShape {
 // [r][k] tiles (k contiguous, 8 per row): k XOR 4 on every other pair of rows, so that the
 // eight rows x four k of an A fragment fall on 16 different double banks
 __device__ __forceinline__ int lk_index(int r, int k) { return r * SK_KC + (k ^ (((r >> 1) & 1) << 2)); }
-
-__device__ __forceinline__ void cp_async16(void* smem, const void* gmem) {
-    unsigned s = (unsigned)__cvta_generic_to_shared(smem);
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(s), "l"(gmem));
-}
 
 // one CTA: rows [rtile * SK_TM, +SK_TM) of the long operand over K range z of nz
 template <int NT, bool LK>
@@ -783,13 +913,14 @@ namespace {
 
 template <bool AK, bool BKc>
 void launch_fp64(const GemmArgs& g, cudaStream_t s) {
-    using S = Smem<AK, BKc>;
-    set_smem_once((const void*)gemm_fp64_kernel<AK, BKc>, (int)S::bytes);
+    using T = Tile<64>;
+    constexpr size_t bytes = TileSmem<T, AK, BKc>::bytes;
+    set_smem_once((const void*)gemm_fp64_kernel<T, AK, BKc>, (int)bytes);
     int ks = fp64_ksplit(g.M, g.N, g.K, false);
     if (!g.ws || (int64_t)ks * g.M * g.N > g.ws_elems) ks = 1;
-    if ((g.M + BM - 1) / BM > 65535) throw std::runtime_error("FP64 GEMM: M too large for the grid");
-    dim3 grid((g.N + BN - 1) / BN, (g.M + BM - 1) / BM, ks);
-    gemm_fp64_kernel<AK, BKc><<<grid, THREADS, S::bytes, s>>>(g);
+    const int64_t tiles = (int64_t)((g.M + T::BM - 1) / T::BM) * ((g.N + T::BN - 1) / T::BN);
+    if (tiles > INT32_MAX) throw std::runtime_error("FP64 GEMM: too many output tiles for the grid");
+    gemm_fp64_kernel<T, AK, BKc><<<dim3((unsigned)tiles, ks), TILE_THREADS, bytes, s>>>(g);
     COUNT_LAUNCH();
     if (ks > 1) {
         const int64_t mn = (int64_t)g.M * g.N;
@@ -801,15 +932,16 @@ void launch_fp64(const GemmArgs& g, cudaStream_t s) {
 
 }  // namespace
 
-// Few output tiles and a long K: split K so that about two waves of CTAs stream the
-// operands; every split keeps at least 512 k.
+// One product in a launch of its own, few output tiles and a long K: split K so that about
+// two waves of CTAs stream the operands; every split keeps at least 512 k.
 int fp64_ksplit(int M, int N, int K, bool skinny_ok) {
     if (const int nt = skinny_ok ? skinny_groups(M, N) : 0) return skinny_ksplit(std::max(M, N), K, nt);
-    const int64_t tiles = (int64_t)((M + BM - 1) / BM) * ((N + BN - 1) / BN);
-    const int ktiles = (K + BK - 1) / BK;
-    if (tiles >= 148) return 1;
-    int64_t ks = (2 * 148 + tiles - 1) / tiles;
-    ks = std::min<int64_t>(ks, ktiles / 32);
+    const int64_t tiles = (int64_t)((M + 63) / 64) * ((N + 63) / 64);
+    const int chunks = (K + BK - 1) / BK;
+    const int64_t slots = 148 * Tile<64>::PER_SM;
+    if (tiles >= slots) return 1;
+    int64_t ks = (2 * slots + tiles - 1) / tiles;
+    ks = std::min<int64_t>(ks, chunks / 32);
     ks = std::min<int64_t>(ks, 256);
     return (int)std::max<int64_t>(ks, 1);
 }
@@ -829,8 +961,6 @@ void gemm_fp64(const GemmArgs& g, cudaStream_t s) {
     }
 }
 
-int fp64_tiles(int M, int N) { return ((M + BM - 1) / BM) * ((N + BN - 1) / BN); }
-
 void splitk_fold(const GemmArgs& g, int ks, cudaStream_t s) {
     const int64_t mn = (int64_t)g.M * g.N;
     if (mn <= 0 || ks <= 1) return;
@@ -839,26 +969,148 @@ void splitk_fold(const GemmArgs& g, int ks, cudaStream_t s) {
     COUNT_LAUNCH();
 }
 
+int fp64_tile_rows(int M, int N) {
+    // 64 unless 32 x 32 tiles cover the product with at most three fifths of the area
+    auto area = [&](int64_t r) { return ((M + r - 1) / r) * ((N + r - 1) / r) * r * r; };
+    return 5 * area(32) <= 3 * area(64) ? 32 : 64;
+}
+
+// Tiles of longer K first.  The tiles of the last full waves run one per CTA; the tiles
+// before them (up to two waves, and every tile whose K is more than half of a CTA's share)
+// form one range of chunks that is cut into equal pieces, one per CTA of a wave, so that
+// neither a last wave that is nearly empty nor a tile of long K keeps the rest waiting.  A
+// cut closer to a tile's end than TILE_MIN_CHUNKS / 2 moves there: a short piece would cost
+// more in its prologue and its partial tile than it balances.  (597 tiles of K=12720 on 592
+// CTA slots ran at 22.5 TFLOP/s one per CTA; with the cuts the three ladder products of o=20
+// v=160, 597 + 2800 + 597 tiles, take 21.8 ms at 29.7 TFLOP/s, 47.8 ms before.)
+TileWork plan_tile_work(const std::vector<TileProblem>& probs, int rows, bool split) {
+    constexpr int TILE_MIN_CHUNKS = 16;
+    TileWork w;
+    w.rows = rows;
+    const int64_t slots = 148 * (rows == 64 ? Tile<64>::PER_SM : Tile<32>::PER_SM);
+    auto tiles_of = [&](const TileProblem& p) { return (int64_t)((p.M + rows - 1) / rows) * ((p.N + rows - 1) / rows); };
+    auto chunks_of = [&](const TileProblem& p) { return (int64_t)(p.K + BK - 1) / BK; };
+    std::vector<int> order(probs.size());
+    int64_t T = 0, U = 0;
+    for (size_t i = 0; i < probs.size(); i++) {
+        order[i] = (int)i;
+        T += tiles_of(probs[i]);
+        U += tiles_of(probs[i]) * chunks_of(probs[i]);
+    }
+    if (T == 0) return w;
+    if (U > INT32_MAX || T > INT32_MAX / 2) split = false;
+    std::stable_sort(order.begin(), order.end(), [&](int a, int b) { return probs[a].K > probs[b].K; });
+    // the range of chunks that is cut: its tiles, chunks and pieces
+    int64_t R = 0, UR = 0, P = 0;
+    if (split) {
+        const int64_t whole = T >= 2 * slots ? (T / slots - 1) * slots : 0;
+        const double share = (double)U / slots;
+        int64_t seen = 0, longest = 0;
+        for (int i : order) {
+            const int64_t nt = tiles_of(probs[i]), c = chunks_of(probs[i]);
+            longest = std::max(longest, c);
+            int64_t take = std::max<int64_t>(0, std::min(nt, T - whole - seen));
+            if (c > std::max(0.5 * share, (double)TILE_MIN_CHUNKS)) take = nt;
+            if (take == 0) break;
+            R += take;
+            UR += take * c;
+            seen += nt;
+            if (take < nt) break;
+        }
+        P = std::min(slots, UR / TILE_MIN_CHUNKS);
+        // not worth cutting: no tile is long enough for two pieces, or the pieces would be no
+        // shorter than the longest tile by a third
+        if (P <= 0 || longest < TILE_MIN_CHUNKS || (R <= slots && 3 * UR > 2 * P * longest)) R = UR = P = 0;
+    }
+    constexpr int64_t h = TILE_MIN_CHUNKS / 2;
+    int64_t ts = 0, b = 1, left = R;       // first chunk of the tile in the range, next cut, tiles left in it
+    w.seg_start.push_back(0);
+    auto next_cta = [&] {
+        if ((int)w.segs.size() > w.seg_start.back()) w.seg_start.push_back((int)w.segs.size());
+    };
+    for (int i : order) {
+        const TileProblem& p = probs[i];
+        const int tm = (p.M + rows - 1) / rows, tn = (p.N + rows - 1) / rows;
+        const int64_t c = chunks_of(p), nt = tiles_of(p);
+        for (int64_t t = 0; t < nt; t++) {
+            TileSeg s;
+            s.prob = i;
+            s.m0 = (int)(tm <= tn ? t % tm : t / tn) * rows;
+            s.n0 = (int)(tm <= tn ? t / tm : t % tn) * rows;
+            auto add = [&](int64_t from, int64_t to, int slot) {
+                s.kt0 = (int)from;
+                s.nkt = (int)(to - from);
+                s.slot = slot;
+                w.segs.push_back(s);
+            };
+            if (left == 0) {
+                next_cta();
+                add(0, c, -1);
+                continue;
+            }
+            left--;
+            int64_t at = 0;
+            int parts = 0;
+            bool after = false;
+            for (; b < P && b * UR / P < ts + c; b++) {
+                const int64_t x = b * UR / P - ts;
+                if (x < h) {
+                    next_cta();
+                } else if (c - x < h) {
+                    after = true;
+                } else {
+                    add(at, x, w.slots + parts++);
+                    at = x;
+                    next_cta();
+                }
+            }
+            add(at, c, parts ? w.slots + parts++ : -1);
+            if (after) next_cta();
+            if (parts) {
+                w.folds.push_back({i, s.m0, s.n0, w.slots, parts});
+                w.slots += parts;
+            }
+            ts += c;
+        }
+    }
+    next_cta();
+    return w;
+}
+
 namespace {
-template <bool AK, bool BKc>
-void launch_grouped_t(const GemmArgs* probs, const int* tile_start, int nprob, int total_tiles, cudaStream_t s) {
-    using S = Smem<AK, BKc>;
-    set_smem_once((const void*)gemm_fp64_grouped_kernel<AK, BKc>, (int)S::bytes);
-    gemm_fp64_grouped_kernel<AK, BKc><<<total_tiles, THREADS, S::bytes, s>>>(probs, tile_start, nprob);
+template <class T, bool AK, bool BKc>
+void launch_tiles_t(const GemmArgs* probs, const TileSeg* segs, const int* seg_start, int nctas, const TileFold* folds,
+                    int nfolds, double* ws, cudaStream_t s) {
+    constexpr size_t bytes = TileSmem<T, AK, BKc>::bytes;
+    set_smem_once((const void*)gemm_fp64_grouped_kernel<T, AK, BKc>, (int)bytes);
+    gemm_fp64_grouped_kernel<T, AK, BKc><<<nctas, TILE_THREADS, bytes, s>>>(probs, segs, seg_start, ws);
+    COUNT_LAUNCH();
+    if (nfolds > 0) {
+        tile_fold_kernel<T, AK, BKc><<<dim3(nfolds, T::MT), TILE_THREADS, 0, s>>>(probs, folds, ws);
+        COUNT_LAUNCH();
+    }
+}
+template <class T>
+void launch_tiles(bool ak, bool bk, const GemmArgs* probs, const TileSeg* segs, const int* seg_start, int nctas,
+                  const TileFold* folds, int nfolds, double* ws, cudaStream_t s) {
+    if (ak) {
+        if (bk) launch_tiles_t<T, true, true>(probs, segs, seg_start, nctas, folds, nfolds, ws, s);
+        else launch_tiles_t<T, true, false>(probs, segs, seg_start, nctas, folds, nfolds, ws, s);
+    } else {
+        if (bk) launch_tiles_t<T, false, true>(probs, segs, seg_start, nctas, folds, nfolds, ws, s);
+        else launch_tiles_t<T, false, false>(probs, segs, seg_start, nctas, folds, nfolds, ws, s);
+    }
 }
 }  // namespace
 
-void gemm_fp64_grouped(const GemmArgs* probs, const int* tile_start, int nprob, int total_tiles, bool a_kcontig,
-                       bool b_kcontig, cudaStream_t s) {
-    if (nprob <= 0 || total_tiles <= 0) return;
-    if (a_kcontig) {
-        if (b_kcontig) launch_grouped_t<true, true>(probs, tile_start, nprob, total_tiles, s);
-        else launch_grouped_t<true, false>(probs, tile_start, nprob, total_tiles, s);
-    } else {
-        if (b_kcontig) launch_grouped_t<false, true>(probs, tile_start, nprob, total_tiles, s);
-        else launch_grouped_t<false, false>(probs, tile_start, nprob, total_tiles, s);
-    }
-    COUNT_LAUNCH();
+int64_t tile_ws_elems(int slots, int rows) { return (int64_t)slots * rows * rows; }
+
+void gemm_fp64_grouped(const GemmArgs* probs, const TileSeg* segs, const int* seg_start, int nctas,
+                       const TileFold* folds, int nfolds, double* ws, int rows, bool a_kcontig, bool b_kcontig,
+                       cudaStream_t s) {
+    if (nctas <= 0) return;
+    if (rows == 64) launch_tiles<Tile<64>>(a_kcontig, b_kcontig, probs, segs, seg_start, nctas, folds, nfolds, ws, s);
+    else launch_tiles<Tile<32>>(a_kcontig, b_kcontig, probs, segs, seg_start, nctas, folds, nfolds, ws, s);
 }
 
 std::pair<int, int> short_shape(int M, int N) {
