@@ -41,6 +41,8 @@ struct Tables {
 struct Builder {
     Context& ctx;
     int n, naux, o;
+    // B[P, p, q] stored [P][q][p]: a piece's rows run over p fastest, and so do the copies of
+    // its tiles (whole sectors; read along p from [P][p][q], every element was a sector)
     double* dB = nullptr;
     std::vector<int> aux_irrep;   // per P
     bool aux_known = false;
@@ -51,6 +53,15 @@ struct Builder {
         const Spaces& S = ctx.spaces;
         int base = space == OCC ? 0 : o;
         return base + S.off[space][ALPHA][irrep] + x;
+    }
+
+    void upload_factor(const double* B) {
+        const int64_t bytes = (int64_t)naux * n * n * sizeof(double);
+        double* raw = (double*)ctx.dmalloc(bytes);
+        dB = (double*)ctx.dmalloc(bytes);
+        CCSD_CUDA(cudaMemcpyAsync(raw, B, bytes, cudaMemcpyHostToDevice, ctx.stream));
+        kern::transpose_factor(raw, dB, naux, n, ctx.stream);
+        ctx.dfree(raw, bytes);
     }
 
     std::vector<int64_t> aux_list(int irrep) const {
@@ -166,13 +177,13 @@ struct Builder {
         for (int y = 0; y < len[pb]; y++)
             for (int x = 0; x < len[pa]; x++) {
                 int64_t m = x + (int64_t)len[pa] * y;
-                Am[m] = (int64_t)gidx(space[pa], irrep[pa], x) * n + gidx(space[pb], irrep[pb], y);
+                Am[m] = (int64_t)gidx(space[pb], irrep[pb], y) * n + gidx(space[pa], irrep[pa], x);
                 Cm[m] = off + stride[pa] * x + stride[pb] * y;
             }
         for (int y = 0; y < len[pd]; y++)
             for (int x = 0; x < len[pc]; x++) {
                 int64_t m = x + (int64_t)len[pc] * y;
-                Bn[m] = (int64_t)gidx(space[pc], irrep[pc], x) * n + gidx(space[pd], irrep[pd], y);
+                Bn[m] = (int64_t)gidx(space[pd], irrep[pd], y) * n + gidx(space[pc], irrep[pc], x);
                 Cn[m] = stride[pc] * x + stride[pd] * y;
             }
         if (batch) {
@@ -326,13 +337,13 @@ struct Builder {
         for (int y = 0; y < len[1]; y++)
             for (int x = 0; x < len[0]; x++) {
                 int64_t m = x + (int64_t)len[0] * y;
-                Am[m] = (int64_t)gidx(space[0], irrep[0], a0 + x) * n + gidx(space[1], irrep[1], y);
+                Am[m] = (int64_t)gidx(space[1], irrep[1], y) * n + gidx(space[0], irrep[0], a0 + x);
                 Cm[m] = stride[0] * x + stride[1] * y;
             }
         for (int y = 0; y < len[3]; y++)
             for (int x = 0; x < len[2]; x++) {
                 int64_t m = x + (int64_t)len[2] * y;
-                Bn[m] = (int64_t)gidx(space[2], irrep[2], x) * n + gidx(space[3], irrep[3], y);
+                Bn[m] = (int64_t)gidx(space[3], irrep[3], y) * n + gidx(space[2], irrep[2], x);
                 Cn[m] = stride[2] * x + stride[3] * y;
             }
         Tables tb{ctx, {}};
@@ -435,8 +446,7 @@ void build_rhf_hamiltonian(Context& ctx, int naux, const double* B, const double
         if ((int)bld.aux_irrep.size() != naux) throw Error(CCSD_ERR_ARG, "aux_per_irrep does not sum to naux");
     }
     const int64_t nB = (int64_t)naux * bld.n * bld.n;
-    bld.dB = (double*)ctx.dmalloc(nB * sizeof(double));
-    CCSD_CUDA(cudaMemcpyAsync(bld.dB, B, nB * sizeof(double), cudaMemcpyHostToDevice, ctx.stream));
+    bld.upload_factor(B);
     create_rhf_hamiltonian_tensors(ctx, H);
     bld.batch = S.nirrep > 1;
     bld.one_electron(H->fAB, eps);
@@ -501,8 +511,7 @@ void build_hamiltonian(Context& ctx, int naux, const double* B, const double* ep
         if ((int)bld.aux_irrep.size() != naux) throw Error(CCSD_ERR_ARG, "aux_per_irrep does not sum to naux");
     }
     const int64_t nB = (int64_t)naux * bld.n * bld.n;
-    bld.dB = (double*)ctx.dmalloc(nB * sizeof(double));
-    CCSD_CUDA(cudaMemcpyAsync(bld.dB, B, nB * sizeof(double), cudaMemcpyHostToDevice, ctx.stream));
+    bld.upload_factor(B);
 
     create_hamiltonian_tensors(ctx, pack_vvvv, H);
     bld.batch = S.nirrep > 1;

@@ -118,6 +118,9 @@ void gemm_fp64(const GemmArgs& g, cudaStream_t s);
 // problem and a range of its k chunks; a tile that several CTAs share leaves one partial
 // tile per part in ws (slots slot0, slot0 + 1, ... in order of k), added by a second launch.
 struct TileProblem {
+// out[P][q][p] = in[P][p][q] for naux n x n matrices
+void transpose_factor(const double* in, double* out, int naux, int n, cudaStream_t s);
+
     int M = 0, N = 0, K = 0;
 };
 struct TileSeg {

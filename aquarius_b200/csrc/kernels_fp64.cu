@@ -2013,6 +2013,19 @@ __global__ void eri_gather_kernel(EriGatherArgs a, const double* __restrict__ er
 #pragma unroll
         for (int p = 0; p < 4; p++) {
             const int x = (int)(r % a.len[p]);
+// 32 x 32 tiles of one matrix per blockIdx.z, 32 x 8 threads
+__global__ void transpose_factor_kernel(const double* __restrict__ in, double* __restrict__ out, int n) {
+    __shared__ double tile[32][33];
+    const int64_t base = (int64_t)blockIdx.z * n * n;
+    int x = blockIdx.x * 32 + threadIdx.x, y = blockIdx.y * 32 + threadIdx.y;
+    for (int j = 0; j < 32; j += 8)
+        if (x < n && y + j < n) tile[threadIdx.y + j][threadIdx.x] = in[base + (int64_t)(y + j) * n + x];
+    __syncthreads();
+    x = blockIdx.y * 32 + threadIdx.x;
+    y = blockIdx.x * 32 + threadIdx.y;
+    for (int j = 0; j < 32; j += 8)
+        if (x < n && y + j < n) out[base + (int64_t)(y + j) * n + x] = tile[threadIdx.x][threadIdx.y + j];
+}
             r /= a.len[p];
             dst += a.st[p] * x;
             g[p] = a.g[p][x];
@@ -2032,6 +2045,15 @@ void eri_gather(const EriGatherArgs& a, const double* eri, cudaStream_t s) {
 }
 
 namespace {
+void transpose_factor(const double* in, double* out, int naux, int n, cudaStream_t s) {
+    const int t = (n + 31) / 32;
+    for (int p = 0; p < naux; p += 65535) {
+        const int64_t off = (int64_t)p * n * n;
+        transpose_factor_kernel<<<dim3(t, t, std::min(naux - p, 65535)), dim3(32, 8), 0, s>>>(in + off, out + off, n);
+        COUNT_LAUNCH();
+    }
+}
+
 __global__ void closed_shell_jk_kernel(const double* __restrict__ eri, int n, int nocc, double* __restrict__ F) {
     const int64_t pq = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
     if (pq >= (int64_t)n * n) return;
