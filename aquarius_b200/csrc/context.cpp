@@ -463,7 +463,7 @@ void Context::release(Plan& p) {
                 if (l.d_probs) dfree(l.d_probs, l.nprob * sizeof(kern::GemmArgs));
                 if (l.d_part) dfree(l.d_part, l.part_elems * sizeof(double));
                 if (l.d_tile_start)
-                    dfree(l.d_tile_start, (l.kind == GemmLaunch::FOLD_GROUPS ? l.ngroups + 1 : l.nprob) * sizeof(int));
+                    dfree(l.d_tile_start, l.nprob * sizeof(int));
                 if (l.d_desc) dfree(l.d_desc, l.desc_bytes);
                 if (l.d_chunks) dfree(l.d_chunks, l.nprob * sizeof(int64_t));
                 if (l.arena) dfree(l.arena, l.arena_bytes);
@@ -742,24 +742,37 @@ void Context::build_run(Plan& p, RunSchedule& rs, int first, int end) {
             std::map<std::pair<int, bool>, std::vector<int>> kstart;
             std::map<std::pair<int, bool>, int> ktiles;
             std::map<std::pair<int, bool>, double> kfl;
-            std::vector<kern::FoldDesc> fdesc(end - first);
+            // each product's own fold: its output map (a node) and its partials (the term), with
+            // the host tables of the map
+            struct Fold {
+                kern::FoldNode node;
+                kern::FoldTerm term;
+                const std::vector<int64_t>* hm[2];
+                const std::vector<int64_t>* hn[2];
+            };
+            std::vector<Fold> fdesc(end - first);
             for (int i = first; i < end; i++) {
                 if (!in_fold[i - first]) continue;
                 const GemmStep& g = p.gemms[p.steps[i].idx];
                 kern::GemmArgs a = gemm_args(p, g);
-                kern::FoldDesc& f = fdesc[i - first];
-                f.part = d_part + off;
+                kern::FoldNode& f = fdesc[i - first].node;
+                kern::FoldTerm& ft = fdesc[i - first].term;
+                auto& hm = fdesc[i - first].hm;
+                auto& hn = fdesc[i - first].hn;
+                ft.part = d_part + off;
                 f.C = a.C;
                 for (int v = 0; v < 2; v++) {
                     f.Cm[v] = a.Cm[v];
                     f.Cn[v] = a.Cn[v];
+                    hm[v] = &g.hCm[v];
+                    hn[v] = &g.hCn[v];
                 }
                 f.nvm = a.nvm;
                 f.nvn = a.nvn;
                 for (int v = 0; v < 4; v++) f.vsign[v] = a.vsign[v];
                 f.M = g.M;
                 f.N = g.N;
-                f.scale = a.alpha;
+                ft.scale = a.alpha;
                 if (in_fold[i - first] == 1) {
                     a.ws = d_part + off;
                     a.ws_elems = (int64_t)g.M * g.N;
@@ -780,12 +793,13 @@ void Context::build_run(Plan& p, RunSchedule& rs, int first, int end) {
                     for (int v = 0; v < 2; v++) {
                         f.Cm[v] = k.Cr[v];
                         f.Cn[v] = k.Cs[v];
+                        if (g.M < g.N) std::swap(hm[v], hn[v]);
                     }
                     f.nvm = k.nvr;
                     f.nvn = k.nvs;
                     for (int v = 0; v < 4; v++) f.vsign[v] = k.vsign[v];
-                    f.scale = k.alpha;
-                    f.ks = k.nz;
+                    ft.scale = k.alpha;
+                    ft.ks = k.nz;
                     off += (int64_t)k.nz * k.R * k.NS;
                     const std::pair<int, bool> cls{kern::skinny_groups(g.M, g.N), lk};
                     kstart[cls].push_back(ktiles[cls]);
@@ -812,10 +826,10 @@ void Context::build_run(Plan& p, RunSchedule& rs, int first, int end) {
                     d.K = g.K;
                     d.kper = skper[i - first];
                     d.part = d_part + off;
-                    f.ks = sctas[i - first];
-                    off += (int64_t)f.ks * g.M * g.N;
+                    ft.ks = sctas[i - first];
+                    off += (int64_t)ft.ks * g.M * g.N;
                     sstart[shape].push_back(sctas_total[shape]);
-                    sctas_total[shape] += f.ks;
+                    sctas_total[shape] += ft.ks;
                     sprobs[shape].push_back(d);
                     sfl[shape] += g.flops();
                 }
@@ -894,22 +908,55 @@ void Context::build_run(Plan& p, RunSchedule& rs, int first, int end) {
                 if (!members.count(r)) group_order.push_back(r);
                 members[r].push_back(i - first);
             }
-            std::vector<kern::FoldDesc> descs;
-            std::vector<int> gstart;
+            // products of one group with the same output map are the terms of one node; a group
+            // that is a single node is cut into items of kFoldChunk elements, the nodes of the
+            // others follow one another in one item
+            auto same_map = [](const Fold& x, const Fold& y) {
+                const kern::FoldNode &a = x.node, &b = y.node;
+                if (a.C != b.C || a.M != b.M || a.N != b.N || a.nvm != b.nvm || a.nvn != b.nvn) return false;
+                for (int v = 0; v < a.nvm * a.nvn; v++)
+                    if (a.vsign[v] != b.vsign[v]) return false;
+                for (int v = 0; v < a.nvm; v++)
+                    if (*x.hm[v] != *y.hm[v]) return false;
+                for (int v = 0; v < a.nvn; v++)
+                    if (*x.hn[v] != *y.hn[v]) return false;
+                return true;
+            };
+            std::vector<kern::FoldItem> items;
+            std::vector<kern::FoldNode> nodes;
+            std::vector<kern::FoldTerm> terms;
             for (int r : group_order) {
-                gstart.push_back((int)descs.size());
-                for (int j : members[r]) descs.push_back(fdesc[j]);
+                std::vector<std::vector<int>> maps;
+                for (int j : members[r]) {
+                    auto it = std::find_if(maps.begin(), maps.end(),
+                                           [&](const std::vector<int>& m) { return same_map(fdesc[m[0]], fdesc[j]); });
+                    if (it == maps.end()) maps.push_back({j});
+                    else it->push_back(j);
+                }
+                const int n0 = (int)nodes.size();
+                int most = 0;
+                for (auto& m : maps) {
+                    kern::FoldNode f = fdesc[m[0]].node;
+                    f.term0 = (int)terms.size();
+                    f.nterms = (int)m.size();
+                    for (int j : m) terms.push_back(fdesc[j].term);
+                    most = std::max(most, f.M * f.N);
+                    nodes.push_back(f);
+                }
+                const int step = maps.size() == 1 ? kern::kFoldChunk : most;
+                for (int l = 0; l < most; l += step) items.push_back({n0, (int)nodes.size(), l, l + step});
             }
-            gstart.push_back((int)descs.size());
             GemmLaunch fl_l;
             fl_l.kind = GemmLaunch::FOLD_GROUPS;
-            fl_l.nprob = (int)descs.size();
-            fl_l.ngroups = (int)group_order.size();
-            fl_l.desc_bytes = descs.size() * sizeof(kern::FoldDesc);
+            fl_l.nprob = (int)items.size();
+            auto align = [](size_t b) { return (b + 15) & ~(size_t)15; };
+            fl_l.at_start = align(items.size() * sizeof(kern::FoldItem));
+            fl_l.at_folds = align(fl_l.at_start + nodes.size() * sizeof(kern::FoldNode));
+            fl_l.desc_bytes = fl_l.at_folds + terms.size() * sizeof(kern::FoldTerm);
             fl_l.d_desc = dmalloc(fl_l.desc_bytes);
-            fl_l.d_tile_start = (int*)dmalloc(gstart.size() * sizeof(int));
-            stage_h2d(fl_l.d_desc, descs.data(), fl_l.desc_bytes);
-            stage_h2d(fl_l.d_tile_start, gstart.data(), gstart.size() * sizeof(int));
+            stage_h2d(fl_l.d_desc, items.data(), items.size() * sizeof(kern::FoldItem));
+            stage_h2d((char*)fl_l.d_desc + fl_l.at_start, nodes.data(), nodes.size() * sizeof(kern::FoldNode));
+            stage_h2d((char*)fl_l.d_desc + fl_l.at_folds, terms.data(), terms.size() * sizeof(kern::FoldTerm));
             run.launches.push_back(fl_l);
             any_group = true;
         }
@@ -1198,7 +1245,8 @@ void Context::launch(Plan& p, const GemmLaunch& l, const std::string& label, dou
             kern::short_grouped((const kern::ShortDesc*)l.d_desc, l.d_tile_start, l.nprob, l.tiles, l.mt, l.nt, stream);
             break;
         case GemmLaunch::FOLD_GROUPS:
-            kern::fold_groups((const kern::FoldDesc*)l.d_desc, l.d_tile_start, l.ngroups, stream);
+            kern::fold_groups((const kern::FoldItem*)l.d_desc, l.nprob, (const kern::FoldNode*)((char*)l.d_desc + l.at_start),
+                              (const kern::FoldTerm*)((char*)l.d_desc + l.at_folds), stream);
             break;
         case GemmLaunch::SUM_BATCHED:
             kern::sum_batched((const kern::SumDesc*)l.d_desc, l.d_chunks, l.nprob, l.chunks, stream);

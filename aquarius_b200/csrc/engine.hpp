@@ -199,7 +199,8 @@ struct GemmLaunch {
     int* d_tile_start = nullptr;
     double* d_part = nullptr;          // shared-output group: partial products (part_elems doubles)
     int64_t part_elems = 0;
-    int ngroups = 0;                   // fold: output blocks (d_desc: FoldDesc[nprob], d_tile_start: group starts)
+                                       // fold: d_desc holds FoldItem[nprob], FoldNode[] from at_start
+                                       // and FoldTerm[] from at_folds
     void* d_desc = nullptr;            // batched sums / scalings: descriptors
     int64_t* d_chunks = nullptr;       // ... and their first chunks
     size_t desc_bytes = 0;

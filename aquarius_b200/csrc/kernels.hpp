@@ -40,20 +40,28 @@ struct GemmArgs {
     bool dense_out = false;
 };
 
-// Fold of dense partial products into C: with p = sum over z < ks of part[z*M*N + m*N + n]
-// (the partials in order), C[Cm[a][m] + Cn[b][n]] += scale * vsign[a*nvn + b] * p for every
-// variant (a, b); the problems of one group of output blocks in order.
-struct FoldDesc {
+// Fold of dense partial products into C.  A node is one output map: for every element (m, n),
+//   v = sum over its terms of scale * (part[m*N + n] + part[M*N + m*N + n] + ...)   (ks partials)
+//   C[Cm[a][m] + Cn[b][n]] += vsign[a*nvn + b] * v   for every variant (a, b).
+// An item is one CTA's work: elements [l0, l1) of nodes [n0, n1), one node after the other.
+struct FoldTerm {
     const double* part = nullptr;
+    double scale = 0;
+    int ks = 1;
+};
+struct FoldNode {
     double* C = nullptr;
     const int64_t* Cm[2] = {nullptr, nullptr};
     const int64_t* Cn[2] = {nullptr, nullptr};
-    int M = 0, N = 0, ks = 1, nvm = 1, nvn = 1;
+    int M = 0, N = 0, nvm = 1, nvn = 1;
     double vsign[4] = {1, 1, 1, 1};
-    double scale = 0;
+    int term0 = 0, nterms = 0;
 };
-// one CTA per group: problems [group_start[g], group_start[g + 1]) of d, in order
-void fold_groups(const FoldDesc* d, const int* group_start, int ngroups, cudaStream_t s);
+struct FoldItem {
+    int n0 = 0, n1 = 0, l0 = 0, l1 = 0;
+};
+constexpr int kFoldChunk = 256;        // elements per item of a node that has its blocks to itself
+void fold_groups(const FoldItem* items, int nitems, const FoldNode* nodes, const FoldTerm* terms, cudaStream_t s);
 
 // Skinny FP64 product: one small extent (<= 32) against a long operand L:
 //   C[Cr_v[r] + Cs_w[s]] += sign_vw * alpha * sum_k L[Lr[r] + Lk[k]] * S[Sk[k] + Sn[s]]
@@ -71,7 +79,7 @@ struct SkinnyArgs {
     double alpha = 0;
     double* ws = nullptr;
     // grouped launches: nz K ranges per row tile; partial: every K range writes its raw
-    // product to ws[z][r][s] for a fold (FoldDesc with ks = nz), even with nz = 1
+    // product to ws[z][r][s] for a fold (a FoldTerm with ks = nz), even with nz = 1
     int nz = 1;
     bool partial = false;
 };
@@ -89,7 +97,7 @@ void skinny_grouped(const SkinnyArgs* d, const int* tile_start, int nprob, int t
 // Short products: both extents <= 64 with (M/8) * (N/8) <= 16 fragments and a long K
 // (F(mi) += <mn||ef> t(ef,in) per irrep block).  The CTAs of a problem split its K range
 // (kper k each) and write their M x N partial products to part[cta][m][n]; a fold adds
-// them (FoldDesc, ks = the problem's CTAs).  One launch covers every problem of one
+// them (a FoldTerm, ks = the problem's CTAs).  One launch covers every problem of one
 // fragment shape, cta_start[p] being the first CTA of problem p.
 struct ShortDesc {
     const double* A = nullptr;
@@ -110,6 +118,9 @@ void short_grouped(const ShortDesc* d, const int* cta_start, int nprob, int tota
 // K-ranges the FP64 GEMM splits a contraction into (1 = none); ws needs ksplit*M*N doubles
 int fp64_ksplit(int M, int N, int K, bool skinny_ok = true);
 
+// out[P][q][p] = in[P][p][q] for naux n x n matrices
+void transpose_factor(const double* in, double* out, int naux, int n, cudaStream_t s);
+
 // native FP64 tensor-core (DMMA) GETT kernel
 void gemm_fp64(const GemmArgs& g, cudaStream_t s);
 // One launch of the tiled FP64 kernel over many problems (device array of GemmArgs, all with
@@ -118,9 +129,6 @@ void gemm_fp64(const GemmArgs& g, cudaStream_t s);
 // problem and a range of its k chunks; a tile that several CTAs share leaves one partial
 // tile per part in ws (slots slot0, slot0 + 1, ... in order of k), added by a second launch.
 struct TileProblem {
-// out[P][q][p] = in[P][p][q] for naux n x n matrices
-void transpose_factor(const double* in, double* out, int naux, int n, cudaStream_t s);
-
     int M = 0, N = 0, K = 0;
 };
 struct TileSeg {

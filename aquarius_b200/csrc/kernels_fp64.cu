@@ -403,22 +403,30 @@ __global__ void __launch_bounds__(TILE_THREADS)
     tile_write_row<T, AK, BKc>(g, f.m0, f.n0, i, v, g.partial_out ? g.ws : nullptr);
 }
 
-// shared-output groups: each CTA folds the partial products of one group of output blocks,
-// its problems one after another and each problem's partials in order (fixed order)
-__global__ void fold_groups_kernel(const FoldDesc* __restrict__ d, const int* __restrict__ gstart) {
-    const int g = blockIdx.x;
-    for (int p = gstart[g]; p < gstart[g + 1]; p++) {
-        const FoldDesc f = d[p];
-        const int64_t mn = (int64_t)f.M * f.N;
-        for (int64_t l = threadIdx.x; l < mn; l += blockDim.x) {
-            double s = 0.0;
-            for (int z = 0; z < f.ks; z++) s += f.part[z * mn + l];
-            const int m = (int)(l / f.N), n = (int)(l % f.N);
-            const double v = f.scale * s;
+// Shared-output groups.  Latency bounds this kernel (a few KB to a few MB of partials): a
+// thread adds all terms of its element, their loads in flight together, and writes once.
+// The terms of a node are added in plan order, the nodes of an item one after the other.
+__global__ void __launch_bounds__(256) fold_groups_kernel(const FoldItem* __restrict__ items, const FoldNode* __restrict__ nodes,
+                                                          const FoldTerm* __restrict__ terms) {
+    const FoldItem it = items[blockIdx.x];
+    for (int q = it.n0; q < it.n1; q++) {
+        const FoldNode& f = nodes[q];
+        const int mn = f.M * f.N, hi = min(it.l1, mn), t1 = f.term0 + f.nterms;
+        for (int l = it.l0 + threadIdx.x; l < hi; l += blockDim.x) {
+            double v = 0.0;
+            for (int t = f.term0; t < t1; t++) {
+                const double* p = terms[t].part + l;
+                const int ks = terms[t].ks;
+                double s = 0.0;
+#pragma unroll 8
+                for (int z = 0; z < ks; z++) s += p[(int64_t)z * mn];
+                v += terms[t].scale * s;
+            }
+            const int m = l / f.N, n = l % f.N;
             for (int a = 0; a < f.nvm; a++)
                 for (int b = 0; b < f.nvn; b++) f.C[f.Cm[a][m] + f.Cn[b][n]] += f.vsign[a * f.nvn + b] * v;
         }
-        __syncthreads();
+        if (q + 1 < it.n1) __syncthreads();   // the next node may write the same elements
     }
 }
 
@@ -1153,9 +1161,9 @@ void short_grouped(const ShortDesc* d, const int* cta_start, int nprob, int tota
     COUNT_LAUNCH();
 }
 
-void fold_groups(const FoldDesc* d, const int* group_start, int ngroups, cudaStream_t s) {
-    if (ngroups <= 0) return;
-    fold_groups_kernel<<<ngroups, 256, 0, s>>>(d, group_start);
+void fold_groups(const FoldItem* items, int nitems, const FoldNode* nodes, const FoldTerm* terms, cudaStream_t s) {
+    if (nitems <= 0) return;
+    fold_groups_kernel<<<nitems, 256, 0, s>>>(items, nodes, terms);
     COUNT_LAUNCH();
 }
 
@@ -2005,14 +2013,6 @@ __global__ void tau_kernel(TauArgs a) {
         a.tau[l] = v;
     }
 }
-__global__ void eri_gather_kernel(EriGatherArgs a, const double* __restrict__ eri) {
-    const int64_t total = (int64_t)a.len[0] * a.len[1] * a.len[2] * a.len[3];
-    for (int64_t l = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; l < total; l += (int64_t)gridDim.x * blockDim.x) {
-        int64_t r = l, dst = a.off;
-        int64_t g[4];
-#pragma unroll
-        for (int p = 0; p < 4; p++) {
-            const int x = (int)(r % a.len[p]);
 // 32 x 32 tiles of one matrix per blockIdx.z, 32 x 8 threads
 __global__ void transpose_factor_kernel(const double* __restrict__ in, double* __restrict__ out, int n) {
     __shared__ double tile[32][33];
@@ -2026,6 +2026,14 @@ __global__ void transpose_factor_kernel(const double* __restrict__ in, double* _
     for (int j = 0; j < 32; j += 8)
         if (x < n && y + j < n) out[base + (int64_t)(y + j) * n + x] = tile[threadIdx.x][threadIdx.y + j];
 }
+__global__ void eri_gather_kernel(EriGatherArgs a, const double* __restrict__ eri) {
+    const int64_t total = (int64_t)a.len[0] * a.len[1] * a.len[2] * a.len[3];
+    for (int64_t l = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; l < total; l += (int64_t)gridDim.x * blockDim.x) {
+        int64_t r = l, dst = a.off;
+        int64_t g[4];
+#pragma unroll
+        for (int p = 0; p < 4; p++) {
+            const int x = (int)(r % a.len[p]);
             r /= a.len[p];
             dst += a.st[p] * x;
             g[p] = a.g[p][x];
@@ -2037,14 +2045,6 @@ __global__ void transpose_factor_kernel(const double* __restrict__ in, double* _
 
 }  // namespace
 
-void eri_gather(const EriGatherArgs& a, const double* eri, cudaStream_t s) {
-    const int64_t n = (int64_t)a.len[0] * a.len[1] * a.len[2] * a.len[3];
-    if (n <= 0) return;
-    eri_gather_kernel<<<ew_blocks(n), EW_THREADS, 0, s>>>(a, eri);
-    COUNT_LAUNCH();
-}
-
-namespace {
 void transpose_factor(const double* in, double* out, int naux, int n, cudaStream_t s) {
     const int t = (n + 31) / 32;
     for (int p = 0; p < naux; p += 65535) {
@@ -2054,6 +2054,14 @@ void transpose_factor(const double* in, double* out, int naux, int n, cudaStream
     }
 }
 
+void eri_gather(const EriGatherArgs& a, const double* eri, cudaStream_t s) {
+    const int64_t n = (int64_t)a.len[0] * a.len[1] * a.len[2] * a.len[3];
+    if (n <= 0) return;
+    eri_gather_kernel<<<ew_blocks(n), EW_THREADS, 0, s>>>(a, eri);
+    COUNT_LAUNCH();
+}
+
+namespace {
 __global__ void closed_shell_jk_kernel(const double* __restrict__ eri, int n, int nocc, double* __restrict__ F) {
     const int64_t pq = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
     if (pq >= (int64_t)n * n) return;
