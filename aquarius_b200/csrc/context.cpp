@@ -738,10 +738,8 @@ void Context::build_run(Plan& p, RunSchedule& rs, int first, int end) {
             std::map<std::pair<int, int>, std::vector<int>> sstart;
             std::map<std::pair<int, int>, int> sctas_total;
             std::map<std::pair<int, int>, double> sfl;
-            std::map<std::pair<int, bool>, std::vector<kern::SkinnyArgs>> kprobs;
-            std::map<std::pair<int, bool>, std::vector<int>> kstart;
-            std::map<std::pair<int, bool>, int> ktiles;
-            std::map<std::pair<int, bool>, double> kfl;
+            std::map<int, std::vector<kern::SkinnyArgs>> kprobs;   // by n-groups
+            std::map<int, double> kfl;
             // each product's own fold: its output map (a node) and its partials (the term), with
             // the host tables of the map
             struct Fold {
@@ -782,8 +780,7 @@ void Context::build_run(Plan& p, RunSchedule& rs, int first, int end) {
                     probs[c].push_back(a);
                     fl[c] += g.flops();
                 } else if (in_fold[i - first] == 3) {
-                    bool lk;
-                    kern::SkinnyArgs k = kern::skinny_args(a, &lk);
+                    kern::SkinnyArgs k = kern::skinny_args(a);
                     k.nz = sctas[i - first];
                     k.partial = true;
                     k.ws = d_part + off;
@@ -801,11 +798,9 @@ void Context::build_run(Plan& p, RunSchedule& rs, int first, int end) {
                     ft.scale = k.alpha;
                     ft.ks = k.nz;
                     off += (int64_t)k.nz * k.R * k.NS;
-                    const std::pair<int, bool> cls{kern::skinny_groups(g.M, g.N), lk};
-                    kstart[cls].push_back(ktiles[cls]);
-                    ktiles[cls] += kern::skinny_tiles(k.R) * k.nz;
-                    kprobs[cls].push_back(k);
-                    kfl[cls] += g.flops();
+                    const int nt = kern::skinny_groups(g.M, g.N);
+                    kprobs[nt].push_back(k);
+                    kfl[nt] += g.flops();
                 } else {
                     const auto shape = kern::short_shape(g.M, g.N);
                     kern::ShortDesc d;
@@ -858,19 +853,9 @@ void Context::build_run(Plan& p, RunSchedule& rs, int first, int end) {
                 run.launches.push_back(l);
             }
             for (auto& kv : kprobs) {
-                GemmLaunch l;
-                l.kind = GemmLaunch::SKINNY_GROUPED;
-                l.nt = kv.first.first;
-                l.ak = kv.first.second;
-                l.nprob = (int)kv.second.size();
-                l.tiles = ktiles[kv.first];
+                GemmLaunch l = group_skinny(kv.second, kv.first);
                 l.flops = kfl[kv.first];
                 own(l);
-                l.desc_bytes = kv.second.size() * sizeof(kern::SkinnyArgs);
-                l.d_desc = dmalloc(l.desc_bytes);
-                l.d_tile_start = (int*)dmalloc(kv.second.size() * sizeof(int));
-                stage_h2d(l.d_desc, kv.second.data(), l.desc_bytes);
-                stage_h2d(l.d_tile_start, kstart[kv.first].data(), kv.second.size() * sizeof(int));
                 run.launches.push_back(l);
             }
             // groups: products connected through a shared output block, in plan order
@@ -964,7 +949,7 @@ void Context::build_run(Plan& p, RunSchedule& rs, int first, int end) {
 
     for (int L = 0; L <= maxlvl; L++) {
         std::vector<int> grp[8];
-        std::map<std::pair<int, bool>, std::vector<int>> sk;
+        std::map<int, std::vector<int>> sk;   // by n-groups
         for (int i = first; i < end; i++) {
             if (level[i - first] != L || in_fold[i - first] || merged[i - first]) continue;
             const int gi = p.steps[i].idx;
@@ -972,8 +957,7 @@ void Context::build_run(Plan& p, RunSchedule& rs, int first, int end) {
             if (groupable(g)) {
                 grp[tile_class(g)].push_back(gi);
             } else if (skinny_groupable(g)) {
-                const bool lk = g.M >= g.N ? g.a_kcontig : g.b_kcontig;
-                sk[{kern::skinny_groups(g.M, g.N), lk}].push_back(gi);
+                sk[kern::skinny_groups(g.M, g.N)].push_back(gi);
             } else {
                 GemmLaunch l;
                 l.gemm = gi;
@@ -1004,30 +988,15 @@ void Context::build_run(Plan& p, RunSchedule& rs, int first, int end) {
                 run.launches.push_back(l);
                 continue;
             }
-            GemmLaunch l;
-            l.kind = GemmLaunch::SKINNY_GROUPED;
-            l.nt = kv.first.first;
-            l.ak = kv.first.second;
             std::vector<kern::SkinnyArgs> probs;
-            std::vector<int> tstart;
-            int tiles = 0;
+            double fl = 0;
             for (int gi : kv.second) {
-                const GemmStep& g = p.gemms[gi];
-                bool lk;
-                kern::SkinnyArgs a = kern::skinny_args(gemm_args(p, g), &lk);
-                a.ws = nullptr;
-                probs.push_back(a);
-                tstart.push_back(tiles);
-                tiles += kern::skinny_tiles(a.R);
-                l.flops += g.flops();
+                probs.push_back(kern::skinny_args(gemm_args(p, p.gemms[gi])));
+                probs.back().ws = nullptr;
+                fl += p.gemms[gi].flops();
             }
-            l.nprob = (int)probs.size();
-            l.tiles = tiles;
-            l.desc_bytes = probs.size() * sizeof(kern::SkinnyArgs);
-            l.d_desc = dmalloc(l.desc_bytes);
-            l.d_tile_start = (int*)dmalloc(tstart.size() * sizeof(int));
-            stage_h2d(l.d_desc, probs.data(), l.desc_bytes);
-            stage_h2d(l.d_tile_start, tstart.data(), tstart.size() * sizeof(int));
+            GemmLaunch l = group_skinny(probs, kv.first);
+            l.flops = fl;
             run.launches.push_back(l);
             any_group = true;
         }
@@ -1069,6 +1038,26 @@ GemmLaunch Context::group_tiles(const std::vector<kern::GemmArgs>& probs, int ro
     stage_h2d(l.d_desc, w.segs.data(), l.at_start);
     stage_h2d((char*)l.d_desc + l.at_start, w.seg_start.data(), l.at_folds - l.at_start);
     stage_h2d((char*)l.d_desc + l.at_folds, w.folds.data(), l.desc_bytes - l.at_folds);
+    return l;
+}
+
+// one launch of the skinny kernel over these problems (their nz K ranges each)
+GemmLaunch Context::group_skinny(const std::vector<kern::SkinnyArgs>& probs, int nt) {
+    GemmLaunch l;
+    l.kind = GemmLaunch::SKINNY_GROUPED;
+    l.nt = nt;
+    l.nprob = (int)probs.size();
+    std::vector<int2> ctas;
+    for (size_t i = 0; i < probs.size(); i++) {
+        const int n = kern::skinny_tiles(probs[i]) * probs[i].nz;
+        for (int t = 0; t < n; t++) ctas.push_back({(int)i, t});
+    }
+    l.tiles = (int)ctas.size();
+    l.at_start = (probs.size() * sizeof(kern::SkinnyArgs) + 15) & ~(size_t)15;
+    l.desc_bytes = l.at_start + ctas.size() * sizeof(int2);
+    l.d_desc = dmalloc(l.desc_bytes);
+    stage_h2d(l.d_desc, probs.data(), probs.size() * sizeof(kern::SkinnyArgs));
+    stage_h2d((char*)l.d_desc + l.at_start, ctas.data(), ctas.size() * sizeof(int2));
     return l;
 }
 
@@ -1239,7 +1228,8 @@ void Context::launch(Plan& p, const GemmLaunch& l, const std::string& label, dou
                                      stream);
             break;
         case GemmLaunch::SKINNY_GROUPED:
-            kern::skinny_grouped((const kern::SkinnyArgs*)l.d_desc, l.d_tile_start, l.nprob, l.tiles, l.nt, l.ak, stream);
+            kern::skinny_grouped((const kern::SkinnyArgs*)l.d_desc, (const int2*)((char*)l.d_desc + l.at_start), l.tiles, l.nt,
+                                 stream);
             break;
         case GemmLaunch::SHORT_GROUPED:
             kern::short_grouped((const kern::ShortDesc*)l.d_desc, l.d_tile_start, l.nprob, l.tiles, l.mt, l.nt, stream);

@@ -189,8 +189,8 @@ struct GemmLaunch {
     int step = -1;                     // single SUM / SCALE: index into Plan::sums / scales
     bool ak = false, bk = false;       // grouped GEMM: operand contiguity
     int mt = 0, nt = 0;                // short products: fragment shape (d_desc: ShortDesc[nprob]);
-                                       // grouped skinny: nt n-groups, ak = L contiguous along k
-                                       // (d_desc: SkinnyArgs[nprob])
+                                       // grouped skinny: nt n-groups, d_desc: SkinnyArgs[nprob]
+                                       // and, from at_start, the int2 of the `tiles` CTAs
     int nprob = 0, tiles = 0;
     kern::GemmArgs* d_probs = nullptr; // grouped GEMM: problems and, in d_desc, their TileSeg[], the
     int rows = 64, nctas = 0;          // CTAs' first segments and the TileFold[] of shared tiles
@@ -328,6 +328,7 @@ public:
     std::vector<double*> tile_retired;                     // outgrown, kept until the context goes
     void ensure_tile_ws(int64_t elems);
     GemmLaunch group_tiles(const std::vector<kern::GemmArgs>& probs, int rows, bool ak, bool bk);
+    GemmLaunch group_skinny(const std::vector<kern::SkinnyArgs>& probs, int nt);
     void build_merged(Plan& p, GemmRun& run, int first, int end, std::vector<char>& merged,
                       const std::function<std::pair<int, int64_t>(int, int64_t)>& block_of);
     void run_merged(Plan& p, MergedProduct& m, const std::string& label);

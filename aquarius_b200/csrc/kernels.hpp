@@ -78,21 +78,26 @@ struct SkinnyArgs {
     double vsign[4] = {1, 1, 1, 1};   // [vr * nvs + vs]
     double alpha = 0;
     double* ws = nullptr;
+    // warps of a CTA that share a row slot (1, 2 or 4), each a part of the CTA's k
+    int wk = 1;
     // grouped launches: nz K ranges per row tile; partial: every K range writes its raw
     // product to ws[z][r][s] for a fold (a FoldTerm with ks = nz), even with nz = 1
     int nz = 1;
     bool partial = false;
 };
-// a contraction as a skinny product (the longer of M, N as the rows of L); *lk: L is
-// contiguous along k
-SkinnyArgs skinny_args(const GemmArgs& g, bool* lk);
-// n-groups of 8 for a small extent (0: not a skinny product), and the row tiles of R rows
+// a contraction as a skinny product (the longer of M, N as the rows of L)
+SkinnyArgs skinny_args(const GemmArgs& g);
+// n-groups of 8 for a small extent (0: not a skinny product), the split of a product's k over
+// warps and CTAs, and its row tiles (128 / wk rows each)
 int skinny_groups(int M, int N);
-int skinny_tiles(int R);
-// many skinny products in one launch: tile_start[p] is the first of problem p's
-// skinny_tiles(R) * nz CTAs; products writing C directly must have disjoint outputs
-void skinny_grouped(const SkinnyArgs* d, const int* tile_start, int nprob, int tiles, int nt, bool lk,
-                    cudaStream_t s);
+struct SkinnySplit {
+    int wk = 1, nz = 1;
+};
+SkinnySplit skinny_split(int R, int K, int nt);
+__host__ __device__ inline int skinny_tiles(const SkinnyArgs& a) { return (a.R + 128 / a.wk - 1) / (128 / a.wk); }
+// many skinny products in one launch: ctas[t] = (problem, row tile + tiles * K range), tiles *
+// nz CTAs per problem; products writing C directly must have disjoint outputs
+void skinny_grouped(const SkinnyArgs* d, const int2* ctas, int nctas, int nt, cudaStream_t s);
 
 // Short products: both extents <= 64 with (M/8) * (N/8) <= 16 fragments and a long K
 // (F(mi) += <mn||ef> t(ef,in) per irrep block).  The CTAs of a problem split its K range

@@ -446,202 +446,150 @@ __global__ void splitk_fold_kernel(GemmArgs g, int ks) {
 // ---------------------------------------------------------------------------
 // Skinny FP64 product: one small extent (<= 32) against a long operand.
 //   C[Cr_v[r] + Cs_w[s]] += sign_vw * alpha * sum_k L[Lr[r] + Lk[k]] * S[Sk[k] + Sn[s]]
-// A CTA owns SK_TM rows of the long operand L and one K range.  L streams through shared
-// memory in SK_TM x SK_KC tiles (cp.async, SK_STAGES stages, 16-byte copies where two
-// neighbouring elements are contiguous and aligned; coalesced along whichever of r / k is
-// contiguous); the small operand's SK_KC x 8*NT tile sits beside it.  The k offsets of
-// both operands for a stage are staged in shared memory one stage ahead, so no copy
-// waits on a table load.  Each warp computes 32 rows x 8*NT columns on the FP64 tensor
-// cores (mma.m8n8k4: 4 x NT tiles per warp, 32 accumulators per thread), so the issue
-// slots go to the loads and not to one FMA per element pair.  A short long-extent splits
-// K over gridDim.z into ws[z][r][s], folded in a fixed order.
+// HBM (the long operand, read once) bounds large products, latency small ones.  Each warp
+// takes 32 rows and walks k in steps of 16, loading its m8n8k4 fragments straight from global
+// memory: a lane reads L at row lane/4 + 8i and k = 4u + lane%4, 64-byte runs along the rows or
+// 32-byte runs along k, whole sectors either way; the k offsets of the next step are fetched
+// while the step's loads are in flight.  The small operand comes through L1, which the warps
+// of a CTA share.  VAMEF t(fm) over 33856 rows x 4416 k (1.2 GB) takes 184 us, 6.5 TB/s, 310 us
+// with the long operand staged in shared memory and two CTAs per SM; VAMEF t(fi) of o=24
+// v=184 2.68 ms, 3.14 before.  No shared-memory stages, so 12 (NS > 16) to 20 (NS <= 8) warps per SM hide one
+// another's latencies and a product of few k costs few round trips.  The four warps of a CTA
+// are 4 / wk slots of 32 rows times wk parts of the k range, the parts added in shared memory;
+// a long K over few rows is also cut over nz CTAs into ws[z][r][s], folded in order of z.
 // ---------------------------------------------------------------------------
-constexpr int SK_THREADS = 256, SK_STAGES = 4, SK_TM = 256, SK_KC = 8;
+constexpr int SK_THREADS = 128, SK_STEP = 16, SK_ROWS = 32;
+constexpr int SK_RED = SK_ROWS + 2;           // pitch of a warp's [s][r] fragments: 2 mod 16 doubles
+constexpr int skinny_per_sm(int nt) { return nt == 1 ? 5 : nt == 2 ? 4 : 3; }
 
-template <int NT, bool LK>
-struct SkinnyShape {
-    static constexpr int MT = 4;                          // m-tiles of 8 rows per warp (8 warps x 32 rows)
-    static constexpr int LDA = SK_TM + 8;                 // [k][r] (r contiguous): 8 mod 16 doubles
-    static constexpr int A_ELEMS = LK ? SK_TM * SK_KC : SK_KC * LDA;
-    static constexpr int LDB = 8 * NT + (NT > 1 ? 8 : 0); // [k][s]: 8 mod 16 doubles
-    static constexpr int B_ELEMS = SK_KC * LDB;
-    static constexpr size_t bytes = (size_t)SK_STAGES * (A_ELEMS + B_ELEMS) * sizeof(double) +
-                                    (SK_TM + 8 * NT + 2 * SK_STAGES * SK_KC) * sizeof(int64_t);
-};
+// one CTA: row tile `rtile` (SK_ROWS * 4 / wk rows) over K range z of nz
+template <int NT>
+__device__ __forceinline__ void skinny_body(const SkinnyArgs& g, int rtile, int z, int nz) {
+    constexpr int MT = SK_ROWS / 8, U = SK_STEP / 4;
+    __shared__ double red[SK_THREADS / 32][8 * NT * SK_RED];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int fr = lane >> 2, fk = lane & 3;
+    const int wk = g.wk;
+    const int r0 = (rtile * (SK_THREADS / 32 / wk) + warp / wk) * SK_ROWS;
 
-// [r][k] tiles (k contiguous, 8 per row): k XOR 4 on every other pair of rows, so that the
-// eight rows x four k of an A fragment fall on 16 different double banks
-__device__ __forceinline__ int lk_index(int r, int k) { return r * SK_KC + (k ^ (((r >> 1) & 1) << 2)); }
+    // steps of the CTA's range, and this warp's part of them
+    const int steps = (g.K + SK_STEP - 1) / SK_STEP, per = (steps + nz - 1) / nz;
+    const int z0 = min(steps, z * per), z1 = min(steps, z0 + per);
+    const int pw = (z1 - z0 + wk - 1) / wk;
+    const int kb = min(z1, z0 + (warp % wk) * pw) * SK_STEP, ke = min(g.K, min(z1, z0 + (warp % wk + 1) * pw) * SK_STEP);
 
-// one CTA: rows [rtile * SK_TM, +SK_TM) of the long operand over K range z of nz
-template <int NT, bool LK>
-__device__ __forceinline__ void skinny_body(const SkinnyArgs& g, int rtile, int z, int nz, unsigned char* smem_raw) {
-    using Sh = SkinnyShape<NT, LK>;
-    double* As = reinterpret_cast<double*>(smem_raw);
-    double* Bs = As + SK_STAGES * Sh::A_ELEMS;
-    int64_t* sLr = reinterpret_cast<int64_t*>(Bs + SK_STAGES * Sh::B_ELEMS);
-    int64_t* sSn = sLr + SK_TM;
-    int64_t* sLk = sSn + 8 * NT;                 // [stage][k]: offsets of L, -1 past K
-    int64_t* sSk = sLk + SK_STAGES * SK_KC;      // [stage][k]: offsets of S
-
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const int r0 = rtile * SK_TM;
-    for (int i = tid; i < SK_TM; i += SK_THREADS) sLr[i] = (r0 + i < g.R) ? g.Lr[r0 + i] : -1;
-    for (int i = tid; i < 8 * NT; i += SK_THREADS) sSn[i] = (i < g.NS) ? g.Sn[i] : -1;
-
-    const int kchunks_all = (g.K + SK_KC - 1) / SK_KC;
-    const int per_split = (kchunks_all + nz - 1) / nz;
-    const int kc0 = z * per_split;
-    const int kchunks = max(0, min(kchunks_all, kc0 + per_split) - kc0);
-
-    // the k offsets of chunk c (relative to this CTA's range) into table slot c % stages
-    auto load_table = [&](int c) {
-        if (tid < 2 * SK_KC && c < kchunks) {
-            const int k = (kc0 + c) * SK_KC + (tid % SK_KC);
-            int64_t v = -1;
-            if (k < g.K) {
-                if (tid < SK_KC) v = g.lk_affine ? g.lk0 + g.lk_step * k : __ldg(g.Lk + k);
-                else v = g.sk_affine ? g.sk0 + g.sk_step * k : __ldg(g.Sk + k);
-            }
-            (tid < SK_KC ? sLk : sSk)[(c % SK_STAGES) * SK_KC + (tid % SK_KC)] = v;
-        }
-    };
-    auto load_stage = [&](int c) {
-        const int st = c % SK_STAGES;
-        double* as = As + st * Sh::A_ELEMS;
-        double* bs = Bs + st * Sh::B_ELEMS;
-        const int64_t* lk = sLk + st * SK_KC;
-        const int64_t* sk = sSk + st * SK_KC;
-        // the long operand in pairs of neighbours (rows for [k][r], k for [r][k])
+    double acc[MT][NT][2];
 #pragma unroll
-        for (int i = 0; i < (SK_TM * SK_KC / 2) / SK_THREADS; i++) {
-            const int e = tid + i * SK_THREADS;
-            int r, k, r1, k1;
-            double *d0, *d1;
-            if (LK) {
-                r = e / (SK_KC / 2);
-                k = 2 * (e % (SK_KC / 2));
-                r1 = r;
-                k1 = k + 1;
-                d0 = as + lk_index(r, k);
-                d1 = d0 + 1;
-            } else {
-                k = e / (SK_TM / 2);
-                r = 2 * (e % (SK_TM / 2));
-                r1 = r + 1;
-                k1 = k;
-                d0 = as + k * Sh::LDA + r;
-                d1 = d0 + 1;
-            }
-            const int64_t o0r = sLr[r], o1r = sLr[r1], o0k = lk[k], o1k = lk[k1];
-            const bool ok0 = o0r >= 0 && o0k >= 0, ok1 = o1r >= 0 && o1k >= 0;
-            const int64_t o0 = o0r + o0k, o1 = o1r + o1k;
-            if (ok0 && ok1 && o1 == o0 + 1 && !(o0 & 1) && !((reinterpret_cast<uintptr_t>(g.L)) & 15)) {
-                cp_async16(d0, g.L + o0);
-            } else {
-                cp_async8(d0, ok0 ? g.L + o0 : g.L, ok0);
-                cp_async8(d1, ok1 ? g.L + o1 : g.L, ok1);
-            }
-        }
-        for (int e = tid; e < SK_KC * 8 * NT; e += SK_THREADS) {
-            const int sidx = e % (8 * NT), k = e / (8 * NT);
-            const bool ok = sSn[sidx] >= 0 && sk[k] >= 0;
-            cp_async8(bs + k * Sh::LDB + sidx, ok ? g.S + sSn[sidx] + sk[k] : g.S, ok);
-        }
-    };
-
-    double acc[Sh::MT][NT][2];
-#pragma unroll
-    for (int i = 0; i < Sh::MT; i++)
+    for (int i = 0; i < MT; i++)
 #pragma unroll
         for (int j = 0; j < NT; j++) acc[i][j][0] = acc[i][j][1] = 0.0;
 
-    for (int c = 0; c < SK_STAGES; c++) load_table(c);
-    __syncthreads();
+    if (r0 < g.R && kb < ke) {
+        int64_t lr[MT], sn[NT];               // -1 past the last row / column
 #pragma unroll
-    for (int c = 0; c < SK_STAGES - 1; c++) {
-        if (c < kchunks) load_stage(c);
-        cp_commit();
-    }
-    const int wr = warp * 8 * Sh::MT;            // first row of this warp in the tile
-    const int fr = lane >> 2, fk = lane & 3;      // fragment row / k of this lane
-    for (int c = 0; c < kchunks; c++) {
-        cp_wait<SK_STAGES - 2>();
-        __syncthreads();
-        {
-            const int nc = c + SK_STAGES - 1;
-            if (nc < kchunks) load_stage(nc);
-            cp_commit();
-            load_table(c + SK_STAGES);           // the slot of chunk c, whose copies are issued
-        }
-        const double* as = As + (c % SK_STAGES) * Sh::A_ELEMS;
-        const double* bs = Bs + (c % SK_STAGES) * Sh::B_ELEMS;
+        for (int i = 0; i < MT; i++) lr[i] = r0 + 8 * i + fr < g.R ? __ldg(g.Lr + r0 + 8 * i + fr) : -1;
 #pragma unroll
-        for (int ks = 0; ks < SK_KC / 4; ks++) {
-            double a[Sh::MT], b[NT];
-            const int k = 4 * ks + fk;
+        for (int j = 0; j < NT; j++) sn[j] = 8 * j + fr < g.NS ? __ldg(g.Sn + 8 * j + fr) : -1;
+        auto offsets = [&](int k0, int64_t* lk, int64_t* sk) {
 #pragma unroll
-            for (int i = 0; i < Sh::MT; i++) {
-                const int r = wr + 8 * i + fr;
-                a[i] = LK ? as[lk_index(r, k)] : as[k * Sh::LDA + r];
+            for (int u = 0; u < U; u++) {
+                const int k = k0 + 4 * u + fk;
+                const bool ok = k < ke;
+                lk[u] = !ok ? -1 : (g.lk_affine ? g.lk0 + g.lk_step * k : __ldg(g.Lk + k));
+                sk[u] = !ok ? -1 : (g.sk_affine ? g.sk0 + g.sk_step * k : __ldg(g.Sk + k));
             }
+        };
+        int64_t lk[U], sk[U];
+        offsets(kb, lk, sk);
+        for (int k0 = kb; k0 < ke; k0 += SK_STEP) {
+            double a[U][MT], b[U][NT];
 #pragma unroll
-            for (int j = 0; j < NT; j++) b[j] = bs[k * Sh::LDB + 8 * j + fr];
+            for (int u = 0; u < U; u++) {
 #pragma unroll
-            for (int i = 0; i < Sh::MT; i++)
+                for (int i = 0; i < MT; i++) a[u][i] = (lk[u] | lr[i]) >= 0 ? __ldg(g.L + lr[i] + lk[u]) : 0.0;
 #pragma unroll
-                for (int j = 0; j < NT; j++) dmma(acc[i][j][0], acc[i][j][1], a[i], b[j]);
+                for (int j = 0; j < NT; j++) b[u][j] = (sk[u] | sn[j]) >= 0 ? __ldg(g.S + sk[u] + sn[j]) : 0.0;
+            }
+            if (k0 + SK_STEP < ke) offsets(k0 + SK_STEP, lk, sk);
+#pragma unroll
+            for (int u = 0; u < U; u++)
+#pragma unroll
+                for (int i = 0; i < MT; i++)
+#pragma unroll
+                    for (int j = 0; j < NT; j++) dmma(acc[i][j][0], acc[i][j][1], a[u][i], b[u][j]);
         }
     }
-    cp_wait<0>();
 
-    // lane holds rows wr + 8i + fr, columns 8j + 2 fk + {0, 1}
-    if (nz > 1 || g.partial) {
-        double* wz = g.ws + (int64_t)z * g.R * g.NS;
+    // lane holds rows r0 + 8i + fr, columns 8j + 2 fk + {0, 1}
+    const bool raw = nz > 1 || g.partial;
+    double* wz = raw ? g.ws + (int64_t)z * g.R * g.NS : nullptr;
+    if (wk > 1) {
+        // the parts of k through shared memory, then one thread per element: lanes along the
+        // rows of C, along the columns of a partial
 #pragma unroll
-        for (int i = 0; i < Sh::MT; i++) {
-            const int r = r0 + wr + 8 * i + fr;
+        for (int i = 0; i < MT; i++)
+#pragma unroll
+            for (int j = 0; j < NT; j++)
+#pragma unroll
+                for (int h = 0; h < 2; h++) red[warp][(8 * j + 2 * fk + h) * SK_RED + 8 * i + fr] = acc[i][j][h];
+        __syncthreads();
+        const int rows = SK_ROWS * (SK_THREADS / 32 / wk), rb = rtile * rows;
+        for (int e = threadIdx.x; e < rows * g.NS; e += SK_THREADS) {
+            const int r = raw ? e / g.NS : e % rows, s = raw ? e % g.NS : e / rows;
+            if (rb + r >= g.R) continue;
+            double v = 0.0;
+            for (int w = 0; w < wk; w++) v += red[r / SK_ROWS * wk + w][s * SK_RED + r % SK_ROWS];
+            if (raw) {
+                wz[(int64_t)(rb + r) * g.NS + s] = v;
+                continue;
+            }
+            v *= g.alpha;
+            for (int a = 0; a < g.nvr; a++)
+                for (int b = 0; b < g.nvs; b++) g.C[g.Cr[a][rb + r] + g.Cs[b][s]] += g.vsign[a * g.nvs + b] * v;
+        }
+        return;
+    }
+    if (raw) {
+#pragma unroll
+        for (int i = 0; i < MT; i++) {
+            const int r = r0 + 8 * i + fr;
             if (r >= g.R) continue;
 #pragma unroll
             for (int j = 0; j < NT; j++)
 #pragma unroll
                 for (int h = 0; h < 2; h++) {
-                    const int sidx = 8 * j + 2 * fk + h;
-                    if (sidx < g.NS) wz[(int64_t)r * g.NS + sidx] = acc[i][j][h];
+                    const int s = 8 * j + 2 * fk + h;
+                    if (s < g.NS) wz[(int64_t)r * g.NS + s] = acc[i][j][h];
                 }
         }
         return;
     }
     if (g.nvr == 1 && g.nvs == 1) {
-        // one destination per element: the reads of a row batch first, then the writes
+        // one destination per element: the reads of a row first, then its writes
         const double sc = g.alpha * g.vsign[0];
 #pragma unroll
-        for (int i = 0; i < Sh::MT; i++) {
-            const int r = r0 + wr + 8 * i + fr;
+        for (int i = 0; i < MT; i++) {
+            const int r = r0 + 8 * i + fr;
             if (r >= g.R) continue;
-            const int64_t cr = g.Cr[0][r];
+            const int64_t cr = __ldg(g.Cr[0] + r);
             int64_t off[2 * NT];
             double old[2 * NT];
 #pragma unroll
-            for (int j = 0; j < NT; j++)
-#pragma unroll
-                for (int h = 0; h < 2; h++) {
-                    const int sidx = 8 * j + 2 * fk + h;
-                    off[2 * j + h] = sidx < g.NS ? cr + g.Cs[0][sidx] : -1;
-                }
+            for (int q = 0; q < 2 * NT; q++) {
+                const int s = 8 * (q >> 1) + 2 * fk + (q & 1);
+                off[q] = s < g.NS ? cr + __ldg(g.Cs[0] + s) : -1;
+            }
 #pragma unroll
             for (int q = 0; q < 2 * NT; q++) old[q] = off[q] >= 0 ? g.C[off[q]] : 0.0;
 #pragma unroll
-            for (int j = 0; j < NT; j++)
-#pragma unroll
-                for (int h = 0; h < 2; h++)
-                    if (off[2 * j + h] >= 0) g.C[off[2 * j + h]] = old[2 * j + h] + sc * acc[i][j][h];
+            for (int q = 0; q < 2 * NT; q++)
+                if (off[q] >= 0) g.C[off[q]] = old[q] + sc * acc[i][q >> 1][q & 1];
         }
         return;
     }
 #pragma unroll
-    for (int i = 0; i < Sh::MT; i++) {
-        const int r = r0 + wr + 8 * i + fr;
+    for (int i = 0; i < MT; i++) {
+        const int r = r0 + 8 * i + fr;
         if (r >= g.R) continue;
         int64_t cr[2];
         cr[0] = g.Cr[0][r];
@@ -650,56 +598,58 @@ __device__ __forceinline__ void skinny_body(const SkinnyArgs& g, int rtile, int 
         for (int j = 0; j < NT; j++)
 #pragma unroll
             for (int h = 0; h < 2; h++) {
-                const int sidx = 8 * j + 2 * fk + h;
-                if (sidx >= g.NS) continue;
+                const int s = 8 * j + 2 * fk + h;
+                if (s >= g.NS) continue;
                 const double v = g.alpha * acc[i][j][h];
                 for (int a = 0; a < g.nvr; a++)
-                    for (int b = 0; b < g.nvs; b++) g.C[cr[a] + g.Cs[b][sidx]] += g.vsign[a * g.nvs + b] * v;
+                    for (int b = 0; b < g.nvs; b++) g.C[cr[a] + g.Cs[b][s]] += g.vsign[a * g.nvs + b] * v;
             }
     }
 }
 
-// two CTAs per SM (about 80 KB of shared memory each): 16 warps keep four stages of the
-// long operand in flight per CTA
-template <int NT, bool LK>
-__global__ void __launch_bounds__(SK_THREADS, 2) skinny_kernel(SkinnyArgs g) {
-    extern __shared__ __align__(16) unsigned char smem_raw[];
-    skinny_body<NT, LK>(g, blockIdx.x, blockIdx.z, gridDim.z, smem_raw);
+template <int NT>
+__global__ void __launch_bounds__(SK_THREADS, skinny_per_sm(NT)) skinny_kernel(SkinnyArgs g) {
+    skinny_body<NT>(g, blockIdx.x, blockIdx.y, gridDim.y);
 }
 
-// Grouped launch: the row tiles (times K ranges) of many skinny products, tile_start[p]
-// being the first CTA of problem p
-template <int NT, bool LK>
-__global__ void __launch_bounds__(SK_THREADS, 2)
-    skinny_grouped_kernel(const SkinnyArgs* __restrict__ probs, const int* __restrict__ tile_start, int nprob) {
-    extern __shared__ __align__(16) unsigned char smem_raw[];
-    __shared__ SkinnyArgs sg;
-    __shared__ int sp;
-    const int t = blockIdx.x;
-    if (threadIdx.x == 0) {
-        int lo = 0, hi = nprob - 1;
-        while (lo < hi) {
-            const int mid = (lo + hi + 1) >> 1;
-            if (tile_start[mid] <= t) lo = mid;
-            else hi = mid - 1;
-        }
-        sp = lo;
-        sg = probs[lo];
-    }
-    __syncthreads();
-    const int local = t - tile_start[sp], rt = (sg.R + SK_TM - 1) / SK_TM;
-    skinny_body<NT, LK>(sg, local % rt, local / rt, sg.nz, smem_raw);
+// Grouped launch: ctas[t] = (problem, row tile + tiles * K range) of CTA t
+template <int NT>
+__global__ void __launch_bounds__(SK_THREADS, skinny_per_sm(NT))
+    skinny_grouped_kernel(const SkinnyArgs* __restrict__ probs, const int2* __restrict__ ctas) {
+    const int2 c = ctas[blockIdx.x];
+    const SkinnyArgs& g = probs[c.x];
+    const int tiles = skinny_tiles(g);
+    skinny_body<NT>(g, c.y % tiles, c.y / tiles, g.nz);
 }
 
-__global__ void skinny_fold_kernel(SkinnyArgs g, int ks) {
+// The K ranges of a product added in order: eight threads per element take contiguous
+// ranges of z each and their sums are added in order, so that a product of many ranges and
+// few elements keeps many loads in flight (T1 residual of o=20 v=160, 3200 elements x 296
+// ranges: 53 us with one thread walking all ranges).
+__global__ void __launch_bounds__(256) skinny_fold_kernel(SkinnyArgs g, int ks) {
+    __shared__ double part[8][33];
     const int64_t rs = (int64_t)g.R * g.NS;
-    for (int64_t l = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; l < rs; l += (int64_t)gridDim.x * blockDim.x) {
+    const int lane = threadIdx.x & 31, grp = threadIdx.x >> 5;
+    const int per = (ks + 7) / 8, z0 = min(ks, grp * per), z1 = min(ks, z0 + per);
+    for (int64_t l0 = blockIdx.x * 32ll; l0 < rs; l0 += gridDim.x * 32ll) {
+        const int64_t l = l0 + lane;
         double sum = 0.0;
-        for (int z = 0; z < ks; z++) sum += g.ws[z * rs + l];
-        const int r = (int)(l / g.NS), s = (int)(l % g.NS);
-        const double v = g.alpha * sum;
-        for (int a = 0; a < g.nvr; a++)
-            for (int b = 0; b < g.nvs; b++) g.C[g.Cr[a][r] + g.Cs[b][s]] += g.vsign[a * g.nvs + b] * v;
+        if (l < rs) {
+#pragma unroll 8
+            for (int z = z0; z < z1; z++) sum += g.ws[z * rs + l];
+        }
+        part[grp][lane] = sum;
+        __syncthreads();
+        if (grp == 0 && l < rs) {
+            double v = 0.0;
+#pragma unroll
+            for (int q = 0; q < 8; q++) v += part[q][lane];
+            v *= g.alpha;
+            const int r = (int)(l / g.NS), s = (int)(l % g.NS);
+            for (int a = 0; a < g.nvr; a++)
+                for (int b = 0; b < g.nvs; b++) g.C[g.Cr[a][r] + g.Cs[b][s]] += g.vsign[a * g.nvs + b] * v;
+        }
+        __syncthreads();
     }
 }
 
@@ -814,58 +764,57 @@ void launch_short_t(const ShortDesc* d, const int* cta_start, int nprob, int tot
 // n-groups of 8 for a small extent (0: not a skinny product)
 int skinny_groups(int M, int N) {
     const int small = std::min(M, N);
-    if (small > 32) return 0;
-    return small <= 8 ? 1 : (small <= 16 ? 2 : 4);
+    return small > 32 ? 0 : (small + 7) / 8;
+}
+
+// Warps that share a row slot (wk), and CTAs (nz) that share a row tile.  wk keeps the 4 / wk
+// slots of 32 rows of a tile full (R=184: 3 tiles of 64 rows, not 2 of 128 with two warps of
+// the second idle), then splits k inside the CTA, which needs no fold, when the tiles are too
+// few and K is short; nz then balances the waves of CTAs against their prologues (about 6
+// steps) and the fold, a warp keeping 64 k or more.
+SkinnySplit skinny_split(int R, int K, int nt) {
+    SkinnySplit s;
+    auto tiles = [&](int w) { return ((int64_t)R + SK_ROWS * (4 / w) - 1) / (SK_ROWS * (4 / w)); };
+    for (int w : {2, 4})
+        if (tiles(w) * (4 / w) * 10 < tiles(s.wk) * (4 / s.wk) * 9) s.wk = w;
+    while (s.wk < 4 && K < 4096 && tiles(s.wk) < 2 * 148 && K >= s.wk * 128) s.wk *= 2;
+    const int64_t t = tiles(s.wk), slots = 148 * skinny_per_sm(nt), steps = (K + SK_STEP - 1) / SK_STEP;
+    const int64_t most = std::min<int64_t>(1024, K / (64 * s.wk));
+    if (t >= 4 * slots || most < 2) return s;
+    int64_t best = -1;
+    for (int64_t nz = 1; nz <= most; nz += std::max<int64_t>(1, nz / 8)) {
+        const int64_t per = (steps + nz - 1) / nz;
+        const int64_t cost = (t * nz + slots - 1) / slots * ((per + s.wk - 1) / s.wk + 6) + (nz > 1 ? 12 : 0);
+        if (best < 0 || cost < best) {
+            best = cost;
+            s.nz = (int)nz;
+        }
+    }
+    return s;
 }
 
 namespace {
 
-// K-ranges for the skinny kernel: about two waves of CTAs, at least 16 k-chunks each
-int skinny_ksplit(int R, int K, int nt) {
-    (void)nt;
-    const int tm = SK_TM, kc = SK_KC;
-    const int64_t tiles = (R + tm - 1) / tm;
-    if (tiles >= 2 * 148) return 1;
-    const int64_t kchunks = (K + kc - 1) / kc;
-    int64_t ks = (2 * 148 + tiles - 1) / tiles;
-    ks = std::min<int64_t>(ks, kchunks / 16);
-    ks = std::min<int64_t>(ks, 1024);
-    return (int)std::max<int64_t>(ks, 1);
-}
-
-template <int NT, bool LK>
+template <int NT>
 void launch_skinny_t(const SkinnyArgs& a, int ks, cudaStream_t s) {
-    using Sh = SkinnyShape<NT, LK>;
-    set_smem_once((const void*)skinny_kernel<NT, LK>, (int)Sh::bytes);
-    dim3 grid((a.R + SK_TM - 1) / SK_TM, 1, ks);
-    skinny_kernel<NT, LK><<<grid, SK_THREADS, Sh::bytes, s>>>(a);
-}
-
-template <int NT, bool LK>
-void launch_skinny_grouped_t(const SkinnyArgs* d, const int* tile_start, int nprob, int tiles, cudaStream_t s) {
-    using Sh = SkinnyShape<NT, LK>;
-    set_smem_once((const void*)skinny_grouped_kernel<NT, LK>, (int)Sh::bytes);
-    skinny_grouped_kernel<NT, LK><<<tiles, SK_THREADS, Sh::bytes, s>>>(d, tile_start, nprob);
+    skinny_kernel<NT><<<dim3(skinny_tiles(a), ks), SK_THREADS, 0, s>>>(a);
 }
 
 void launch_skinny(const GemmArgs& g, int nt, cudaStream_t s) {
-    bool lk;
-    SkinnyArgs a = skinny_args(g, &lk);
-    int ks = skinny_ksplit(a.R, a.K, nt);
+    SkinnyArgs a = skinny_args(g);
+    int ks = skinny_split(a.R, a.K, nt).nz;
     if (!g.ws || (int64_t)ks * a.R * a.NS > g.ws_elems) ks = 1;
     a.ws = g.ws;
-    switch (nt * 2 + (lk ? 1 : 0)) {
-        case 2: launch_skinny_t<1, false>(a, ks, s); break;
-        case 3: launch_skinny_t<1, true>(a, ks, s); break;
-        case 4: launch_skinny_t<2, false>(a, ks, s); break;
-        case 5: launch_skinny_t<2, true>(a, ks, s); break;
-        case 8: launch_skinny_t<4, false>(a, ks, s); break;
-        default: launch_skinny_t<4, true>(a, ks, s); break;
+    switch (nt) {
+        case 1: launch_skinny_t<1>(a, ks, s); break;
+        case 2: launch_skinny_t<2>(a, ks, s); break;
+        case 3: launch_skinny_t<3>(a, ks, s); break;
+        default: launch_skinny_t<4>(a, ks, s); break;
     }
     COUNT_LAUNCH();
     if (ks > 1) {
         const int64_t rs = (int64_t)a.R * a.NS;
-        const int nb = (int)std::min<int64_t>((rs + 255) / 256, 148 * 16);
+        const int nb = (int)std::min<int64_t>((rs + 31) / 32, 148 * 16);
         skinny_fold_kernel<<<nb, 256, 0, s>>>(a, ks);
         COUNT_LAUNCH();
     }
@@ -873,10 +822,9 @@ void launch_skinny(const GemmArgs& g, int nt, cudaStream_t s) {
 
 }  // namespace
 
-SkinnyArgs skinny_args(const GemmArgs& g, bool* lk_out) {
+SkinnyArgs skinny_args(const GemmArgs& g) {
     SkinnyArgs a;
     const bool long_a = g.M >= g.N;
-    bool lk;
     a.C = g.C;
     a.alpha = g.alpha;
     a.K = g.K;
@@ -885,7 +833,6 @@ SkinnyArgs skinny_args(const GemmArgs& g, bool* lk_out) {
         a.R = g.M; a.NS = g.N; a.nvr = g.nvm; a.nvs = g.nvn;
         for (int v = 0; v < 2; v++) { a.Cr[v] = g.Cm[v]; a.Cs[v] = g.Cn[v]; }
         for (int i = 0; i < 4; i++) a.vsign[i] = g.vsign[i];
-        lk = g.a_kcontig;
         a.lk_affine = g.ak_affine; a.lk0 = g.ak0; a.lk_step = g.ak_step;
         a.sk_affine = g.bk_affine; a.sk0 = g.bk0; a.sk_step = g.bk_step;
     } else {
@@ -894,25 +841,20 @@ SkinnyArgs skinny_args(const GemmArgs& g, bool* lk_out) {
         for (int v = 0; v < 2; v++) { a.Cr[v] = g.Cn[v]; a.Cs[v] = g.Cm[v]; }
         for (int r = 0; r < g.nvn; r++)
             for (int c = 0; c < g.nvm; c++) a.vsign[r * g.nvm + c] = g.vsign[c * g.nvn + r];
-        lk = g.b_kcontig;
         a.lk_affine = g.bk_affine; a.lk0 = g.bk0; a.lk_step = g.bk_step;
         a.sk_affine = g.ak_affine; a.sk0 = g.ak0; a.sk_step = g.ak_step;
     }
-    *lk_out = lk;
+    a.wk = skinny_split(a.R, a.K, skinny_groups(g.M, g.N)).wk;
     return a;
 }
 
-int skinny_tiles(int R) { return (R + SK_TM - 1) / SK_TM; }
-
-void skinny_grouped(const SkinnyArgs* d, const int* tile_start, int nprob, int tiles, int nt, bool lk, cudaStream_t s) {
-    if (nprob <= 0 || tiles <= 0) return;
-    switch (nt * 2 + (lk ? 1 : 0)) {
-        case 2: launch_skinny_grouped_t<1, false>(d, tile_start, nprob, tiles, s); break;
-        case 3: launch_skinny_grouped_t<1, true>(d, tile_start, nprob, tiles, s); break;
-        case 4: launch_skinny_grouped_t<2, false>(d, tile_start, nprob, tiles, s); break;
-        case 5: launch_skinny_grouped_t<2, true>(d, tile_start, nprob, tiles, s); break;
-        case 8: launch_skinny_grouped_t<4, false>(d, tile_start, nprob, tiles, s); break;
-        default: launch_skinny_grouped_t<4, true>(d, tile_start, nprob, tiles, s); break;
+void skinny_grouped(const SkinnyArgs* d, const int2* ctas, int nctas, int nt, cudaStream_t s) {
+    if (nctas <= 0) return;
+    switch (nt) {
+        case 1: skinny_grouped_kernel<1><<<nctas, SK_THREADS, 0, s>>>(d, ctas); break;
+        case 2: skinny_grouped_kernel<2><<<nctas, SK_THREADS, 0, s>>>(d, ctas); break;
+        case 3: skinny_grouped_kernel<3><<<nctas, SK_THREADS, 0, s>>>(d, ctas); break;
+        default: skinny_grouped_kernel<4><<<nctas, SK_THREADS, 0, s>>>(d, ctas); break;
     }
     COUNT_LAUNCH();
 }
@@ -943,7 +885,7 @@ void launch_fp64(const GemmArgs& g, cudaStream_t s) {
 // One product in a launch of its own, few output tiles and a long K: split K so that about
 // two waves of CTAs stream the operands; every split keeps at least 512 k.
 int fp64_ksplit(int M, int N, int K, bool skinny_ok) {
-    if (const int nt = skinny_ok ? skinny_groups(M, N) : 0) return skinny_ksplit(std::max(M, N), K, nt);
+    if (const int nt = skinny_ok ? skinny_groups(M, N) : 0) return skinny_split(std::max(M, N), K, nt).nz;
     const int64_t tiles = (int64_t)((M + 63) / 64) * ((N + 63) / 64);
     const int chunks = (K + BK - 1) / BK;
     const int64_t slots = 148 * Tile<64>::PER_SM;

@@ -54,3 +54,11 @@ def test_skinny_matches_reference_and_tiled(case, o, v, monkeypatch):
         scale = max(1.0, np.abs(ref).max())
         assert np.abs(out[path] - ref).max() < 1e-12 * scale, path
     assert np.abs(out["auto"] - out["tiled"]).max() < 1e-12 * max(1.0, np.abs(out["tiled"]).max())
+
+
+@pytest.mark.parametrize("o,v", [(1, 37), (3, 70), (9, 6), (17, 12), (25, 10)], ids=lambda x: str(x))
+@pytest.mark.parametrize("case", CASES, ids=[f"{c[0]}+={c[2]}*{c[4]}" for c in CASES])
+def test_skinny_edges(case, o, v, monkeypatch):
+    """One to four groups of eight columns, rows that fill a part of a 32-row slot, and warps
+    that split k among them (a K shorter than the four parts included)."""
+    test_skinny_matches_reference_and_tiled(case, o, v, monkeypatch)
