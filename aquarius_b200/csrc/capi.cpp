@@ -590,6 +590,7 @@ int ccsd_weight(ccsd_ctx ctx, ccsd_tensor A, const double* dvrt_a, const double*
                     w.len[p] = b.len[p];
                     w.d[p] = dev[sp][sc.spin[p]] + S.off[sp][sc.spin[p]][b.irrep[p]];
                 }
+                kern::weight_plan(w);
                 kern::weight_block(T.data + b.offset, w, shift, c->stream);
             }
         CCSD_CUDA(cudaStreamSynchronize(c->stream));

@@ -558,16 +558,25 @@ RunSchedule& Context::schedule(Plan& p) {
         if (kind == Step::DOT) {
             size_t e = s;
             while (e < p.steps.size() && p.steps[e].kind == Step::DOT) e++;
-            if (e - s >= 2) build_dot_run(p, rs, (int)s, (int)e);
+            build_dot_run(p, rs, (int)s, (int)e);
             s = e;
             continue;
         }
         const std::string& lab = label_of(p.steps[s]);
         size_t e = s;
         while (e < p.steps.size() && p.steps[e].kind == kind && label_of(p.steps[e]) == lab) e++;
-        if (kind == Step::GEMM || e - s >= 2) {
-            if (kind == Step::GEMM) build_run(p, rs, (int)s, (int)e);
-            else build_elementwise_run(p, rs, (int)s, (int)e);
+        if (kind == Step::GEMM) {
+            build_run(p, rs, (int)s, (int)e);
+        } else if (kind == Step::SCALE && e < p.steps.size() && p.steps[e].kind == Step::SUM && label_of(p.steps[e]) == lab) {
+            // an assignment: zeros, then sums into them
+            size_t f = e;
+            while (f < p.steps.size() && p.steps[f].kind == Step::SUM && label_of(p.steps[f]) == lab) f++;
+            const std::vector<char> fused = assigning(p, (int)s, (int)e, (int)f);
+            build_elementwise_run(p, rs, (int)s, (int)e, &fused, (int)s);
+            build_elementwise_run(p, rs, (int)e, (int)f, &fused, (int)s);
+            e = f;
+        } else {
+            build_elementwise_run(p, rs, (int)s, (int)e);
         }
         s = e;
     }
@@ -1061,11 +1070,57 @@ GemmLaunch Context::group_skinny(const std::vector<kern::SkinnyArgs>& probs, int
     return l;
 }
 
+// Which of the scalings [first, mid) and sums [mid, end) of one statement fold into an
+// assignment: a scaling of a block to zero whose first sum writes every element of the block
+// once from a tensor other than the output.  The scaling is dropped and the sum assigns: half
+// the bytes of the pair, and one launch less where every block folds.
+std::vector<char> Context::assigning(Plan& p, int first, int mid, int end) {
+    std::vector<char> fused(end - first, 0);
+    for (int i = mid; i < end; i++) {
+        const SumStep& s = p.sums[p.steps[i].idx];
+        if (s.tC == kScratch || (s.tA != kScratch && tensor(s.tA).data == tensor(s.tC).data)) return fused;
+    }
+    std::map<std::pair<int, int64_t>, int> scaled;   // block start -> its scaling to zero
+    for (int i = first; i < mid; i++) {
+        const ScaleStep& s = p.scales[p.steps[i].idx];
+        if (s.beta == 0.0 && s.n > 0) scaled[{s.tC, s.off}] = i;
+    }
+    std::map<int, std::vector<std::pair<int64_t, int64_t>>> ranges;   // tensor -> [begin, end) of its scaled blocks
+    for (auto& kv : scaled) ranges[kv.first.first].push_back({kv.first.second, kv.first.second + p.scales[p.steps[kv.second].idx].n});
+    for (int i = mid; i < end; i++) {
+        const SumStep& s = p.sums[p.steps[i].idx];
+        auto& r = ranges[s.tC];
+        auto ub = std::upper_bound(r.begin(), r.end(), std::make_pair(s.offC, INT64_MAX));
+        if (ub == r.begin() || (ub - 1)->second <= s.offC) continue;
+        const int64_t start = (ub - 1)->first;
+        auto it = scaled.find({s.tC, start});
+        if (it == scaled.end()) continue;            // a sum into this block came before
+        int64_t total = 1;
+        std::vector<std::pair<int64_t, int64_t>> pos;
+        for (int k = 0; k < s.ndim; k++) {
+            total *= s.len[k];
+            if (s.len[k] > 1) pos.push_back({s.sC[k], s.len[k]});
+        }
+        if (total <= 0) continue;
+        std::sort(pos.begin(), pos.end());
+        int64_t gapless = 1;
+        for (auto& x : pos) {
+            if (x.first != gapless) break;
+            gapless *= x.second;
+        }
+        if (s.offC == start && total == p.scales[p.steps[it->second].idx].n && gapless == total)
+            fused[it->second - first] = fused[i - first] = 1;
+        scaled.erase(it);
+    }
+    return fused;
+}
+
 // A run of permuted sums or of scalings of one statement.  Sums read their A blocks (an
 // operand or a product region, never written in the run) and write C blocks: each gets a
 // level above the last sum into the same C block, and every level is one batched launch.
-// Scalings touch distinct blocks: one launch.
-void Context::build_elementwise_run(Plan& p, RunSchedule& rs, int first, int end) {
+// Scalings touch distinct blocks: one launch.  Steps marked in fused (of the steps from fused0)
+// are the halves of an assignment: the scaling is left out, the sum assigns.
+void Context::build_elementwise_run(Plan& p, RunSchedule& rs, int first, int end, const std::vector<char>* fused, int fused0) {
     const bool is_sum = p.steps[first].kind == Step::SUM;
     std::map<int, std::vector<int64_t>> starts;
     auto block_of = [&](int h, int64_t off) -> std::pair<int, int64_t> {
@@ -1098,8 +1153,13 @@ void Context::build_elementwise_run(Plan& p, RunSchedule& rs, int first, int end
     run.end = end;
     for (int L = 0; L <= maxlvl; L++) {
         std::vector<int> idx;
-        for (int i = first; i < end; i++)
-            if (level[i - first] == L) idx.push_back(p.steps[i].idx);
+        std::vector<char> assign;
+        for (int i = first; i < end; i++) {
+            const bool f = fused && (*fused)[i - fused0];
+            if (level[i - first] != L || (f && !is_sum)) continue;
+            idx.push_back(p.steps[i].idx);
+            assign.push_back(f);
+        }
         if (idx.empty()) continue;
         GemmLaunch l;
         std::vector<int64_t> cs;
@@ -1108,9 +1168,10 @@ void Context::build_elementwise_run(Plan& p, RunSchedule& rs, int first, int end
         if (is_sum) {
             l.kind = GemmLaunch::SUM_BATCHED;
             std::vector<kern::SumDesc> d;
-            for (int k : idx) {
-                const SumStep& s = p.sums[k];
+            for (size_t j = 0; j < idx.size(); j++) {
+                const SumStep& s = p.sums[idx[j]];
                 kern::SumDesc x;
+                x.assign = assign[j];
                 x.A = data_of(p, s.tA) + s.offA;
                 x.C = data_of(p, s.tC) + s.offC;
                 x.alpha = s.alpha;
@@ -1123,10 +1184,10 @@ void Context::build_elementwise_run(Plan& p, RunSchedule& rs, int first, int end
                     x.total *= s.len[q];
                 }
                 if (x.total <= 0) continue;
-                kern::sum_plan_tiles(x);
+                kern::sum_plan(x);
                 d.push_back(x);
                 cs.push_back(chunks);
-                chunks += kern::sum_chunks(x);
+                chunks += kern::mode_chunks(x);
             }
             if (d.empty()) continue;
             l.desc_bytes = d.size() * sizeof(kern::SumDesc);
@@ -1184,12 +1245,12 @@ void Context::build_dot_run(Plan& p, RunSchedule& rs, int first, int end) {
         }
         x.alpha = d.alpha;
         if (x.total <= 0) continue;
-        kern::plan_divisors(x.len, x.ndim, x.total, x.fast, x.dmul, x.dshr);
+        kern::dot_plan(x);
         descs.push_back(x);
         cs.push_back(chunks);
-        chunks += (x.total + kern::kBatchChunk - 1) / kern::kBatchChunk;
+        chunks += kern::mode_chunks(x);
     }
-    if (descs.size() < 2) return;
+    if (descs.empty()) return;
     GemmLaunch l;
     l.kind = GemmLaunch::DOT_BATCHED;
     l.nprob = (int)descs.size();

@@ -32,6 +32,7 @@ DiisRing::~DiisRing() {
     ctx.dfree(d_e, (order + 1) * (order + 1) * sizeof(double));
     ctx.dfree(d_c, (order + 1) * sizeof(double));
     ctx.dfree(d_dots, order * sizeof(double));
+    ctx.dfree(d_segs, segs.size() * sizeof(kern::DiisSegment));
     ctx.dfree(d_state, 8 * sizeof(int));
     if (h_state) cudaFreeHost(h_state);
     if (h_c) cudaFreeHost(h_c);
@@ -83,6 +84,7 @@ void DiisRing::lay_out(const std::vector<int>& x, const std::vector<int>& dx, co
     d_e = (double*)ctx.dmalloc((order + 1) * (order + 1) * sizeof(double));
     d_c = (double*)ctx.dmalloc((order + 1) * sizeof(double));
     d_dots = (double*)ctx.dmalloc(order * sizeof(double));
+    d_segs = (kern::DiisSegment*)ctx.dmalloc(segs.size() * sizeof(kern::DiisSegment));
     d_state = (int*)ctx.dmalloc(8 * sizeof(int));
     cudaStream_t s = ctx.stream;
     for (int i = 0; i < order; i++) {
@@ -91,6 +93,7 @@ void DiisRing::lay_out(const std::vector<int>& x, const std::vector<int>& dx, co
     }
     CCSD_CUDA(cudaMemcpyAsync(d_xs, xs.data(), order * sizeof(double*), cudaMemcpyHostToDevice, s));
     CCSD_CUDA(cudaMemcpyAsync(d_dxs, dxs.data(), order * sizeof(double*), cudaMemcpyHostToDevice, s));
+    CCSD_CUDA(cudaMemcpyAsync(d_segs, segs.data(), segs.size() * sizeof(kern::DiisSegment), cudaMemcpyHostToDevice, s));
     CCSD_CUDA(cudaMemsetAsync(d_e, 0, (order + 1) * (order + 1) * sizeof(double), s));
     CCSD_CUDA(cudaMemsetAsync(d_c, 0, (order + 1) * sizeof(double), s));
     int st[8] = {0, 0, start, 0, 0, 0, 0, 0};   // head, count, start counter, singular flag
@@ -122,8 +125,7 @@ void DiisRing::extrapolate(const std::vector<int>& x, const std::vector<int>& dx
     for (size_t k = 0; k < x.size(); k++)
         kern::diis_store_segment(d_state, d_xs, d_dxs, piece_off[k], ctx.tensor(x[k]).data, ctx.tensor(dx[k]).data,
                                  piece_len[k], s);
-    CCSD_CUDA(cudaMemsetAsync(d_dots, 0, order * sizeof(double), s));
-    for (auto& sg : segs) kern::diis_dots(d_state, d_dxs, order, sg.off, sg.len, sg.w, d_dots, s);
+    kern::diis_dots(d_state, d_dxs, order, d_segs, (int)segs.size(), vec_len, d_dots, s);
     kern::diis_solve(d_state, d_e, d_c, d_dots, order, s);
     // x = sum c_i x_i, dx = sum c_i dx_i (diis.hpp:205-226); with no extrapolation c is the
     // unit vector of the stored newest pair and x, dx keep their values

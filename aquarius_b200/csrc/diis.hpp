@@ -27,17 +27,14 @@ public:
     Context& ctx;
 
 private:
-    struct Seg {
-        int64_t off, len;
-        double w;
-    };
     void lay_out(const std::vector<int>& x, const std::vector<int>& dx, const double* weights);
 
     int order, start;
     double damping;
     bool laid_out = false;
     std::vector<int64_t> piece_len, piece_off;
-    std::vector<Seg> segs;
+    std::vector<kern::DiisSegment> segs;
+    kern::DiisSegment* d_segs = nullptr;
     int64_t vec_len = 0;
     std::vector<double*> xs, dxs;
     const double** d_xs = nullptr;

@@ -399,7 +399,9 @@ public:
     kern::GemmArgs gemm_args(Plan& p, const GemmStep& g);
     RunSchedule& schedule(Plan& p);
     void build_run(Plan& p, RunSchedule& rs, int first, int end);
-    void build_elementwise_run(Plan& p, RunSchedule& rs, int first, int end);
+    void build_elementwise_run(Plan& p, RunSchedule& rs, int first, int end, const std::vector<char>* fused = nullptr,
+                               int fused0 = 0);
+    std::vector<char> assigning(Plan& p, int first, int mid, int end);
     void build_dot_run(Plan& p, RunSchedule& rs, int first, int end);
     void launch(Plan& p, const GemmLaunch& l, const std::string& label, double* dot_acc = nullptr);
     std::vector<int> constant_tensors;  // handles whose contents never change (sliced once)

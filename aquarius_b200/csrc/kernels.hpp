@@ -276,7 +276,10 @@ struct WeightArgs {
     int64_t len[8];
     const double* d[8];
     int64_t total = 1;
+    int fast = 0;                      // multiply-shift index split, as SumDesc (weight_plan)
+    uint32_t dmul[8], dshr[8];
 };
+void weight_plan(WeightArgs& w);
 void weight_block(double* X, const WeightArgs& w, double shift, cudaStream_t s);
 
 // key/value scatter: X[keys[i]] = beta*X[keys[i]] + alpha*vals[i]
@@ -284,14 +287,7 @@ void kv_write(double* X, const int64_t* keys, const double* vals, int64_t n, dou
               cudaStream_t s);
 void kv_read(const double* X, const int64_t* keys, double* vals, int64_t n, cudaStream_t s);
 
-// ---- fused CCSD update / DIIS -------------------------------------------------------
-// z = w * z_raw / den (den from per-position denominators), t += z, track max|z|;
-// blocks described by WeightArgs; results accumulated into red[0] (max)
-void update_block(double* Z, double* T, const WeightArgs& w, double* red_max, cudaStream_t s);
-
-// batched dot: out[j] += w * sum x[i]*ys[j][i], j < ny  (ys: device array of pointers)
-void dot_batch(const double* x, const double* const* ys, int ny, int64_t n, double w, double* out,
-               cudaStream_t s);
+// ---- DIIS ---------------------------------------------------------------------------
 // out[i] = sum_j c[j] * xs[j][i]  (c on device); i < n1 goes to out1, the rest to out2
 void lincomb(double* out1, int64_t n1, double* out2, int64_t n2, const double* const* xs, const double* c, int nx,
              cudaStream_t s);
@@ -304,8 +300,13 @@ void diis_advance(int* state, int order, cudaStream_t s);
 // xs[head] = [t1 | t2], dxs[head] = [z1 | z2]
 void diis_store(const int* state, const double* const* xs, const double* const* dxs, const double* t1, int64_t n1,
                 const double* t2, int64_t n2, const double* z1, const double* z2, cudaStream_t s);
-// dots[j] += w * <dxs[head][off:off+len], dxs[j][off:off+len]>,  j < order
-void diis_dots(const int* state, const double* const* dxs, int order, int64_t off, int64_t len, double w,
+// dots[j] = sum over segments of w * <dxs[head][off:off+len], dxs[j][off:off+len]>,  j < order
+// (segs: device array; total: the elements of all segments)
+struct DiisSegment {
+    int64_t off = 0, len = 0;
+    double w = 0;
+};
+void diis_dots(const int* state, const double* const* dxs, int order, const DiisSegment* segs, int nsegs, int64_t total,
                double* dots, cudaStream_t s);
 // update the error matrix with the new row, solve the bordered system and write the
 // coefficients by slot into c (unit vector at head when no extrapolation happens)
@@ -334,8 +335,10 @@ struct TauArgs {
     const double* t2 = nullptr;
     const double *t1ai = nullptr, *t1bj = nullptr, *t1aj = nullptr, *t1bi = nullptr;
     int64_t len[4] = {0, 0, 0, 0};
+    int fast = 0;                      // multiply-shift index split, as SumDesc (tau_plan)
+    uint32_t dmul[4], dshr[4];
 };
-void tau_block(const TauArgs& a, cudaStream_t s);
+void tau_plan(TauArgs& a);
 // closed-shell two-electron Fock part from dense (pq|rs) (last index fastest):
 // F[p*n + q] = sum_{i < nocc} 2 (pq|ii) - (pi|iq)
 void closed_shell_jk(const double* eri, int n, int nocc, double* F, cudaStream_t s);
@@ -361,6 +364,8 @@ struct DotDesc {
     int64_t len[8], sA[8], sB[8];
     int64_t total = 0;
     double alpha = 0;
+    int mode = 0, spr = 0, p0 = 0, pc = 0;   // as SumDesc
+    int64_t units = 0;
     int fast = 0;                      // multiply-shift index split, as SumDesc
     uint32_t dmul[8], dshr[8];
 };
@@ -400,25 +405,34 @@ struct SumDesc {
     const double* A = nullptr;
     double* C = nullptr;
     double alpha = 0;
+    int assign = 0;                    // 1: C = alpha * A (the scaling to zero before it is dropped)
     int ndim = 0;
     int64_t len[8], sA[8], sC[8];
     int64_t total = 0;
-    // permuted sums whose fastest A and C positions differ go through 32 x 32 shared-memory
-    // tiles over those two positions (coalesced reads of A and writes of C); a chunk is
-    // two tiles
-    int tiled = 0, p0 = 0, pc = 0;
-    int64_t ntiles = 0;
+    // ROWS: the fastest position is contiguous in A and in C; warps walk its rows 32 elements
+    // at a time (`spr` slots a row) and split only the row number into positions.
+    // TILES: the fastest A and C positions (p0, pc) differ: 32 x 32 tiles through shared
+    // memory, coalesced reads of A and writes of C; a chunk is two tiles.
+    // ELEMENTS: the rest, every element index split into positions.
+    enum Mode { ELEMENTS, ROWS, TILES };
+    int mode = ELEMENTS, spr = 0, p0 = 0, pc = 0;
+    int64_t units = 0;                 // slots (ROWS) or tiles (TILES)
     // every index below 2^31: the element index splits into positions by multiply-shift
     // (x / len = (umulhi(x, mul) + x) >> shr) instead of 64-bit divisions
     int fast = 0;
     uint32_t dmul[8], dshr[8];
 };
-// chunks of kBatchChunk elements (or two 32 x 32 tiles) a sum descriptor takes
-inline int64_t sum_chunks(const SumDesc& d) {
-    return d.tiled ? (d.ntiles + 1) / 2 : (d.total + kBatchChunk - 1) / kBatchChunk;
+constexpr int kRowSlots = kBatchChunk / 32;      // slots a chunk of a ROWS descriptor takes
+// chunks of kBatchChunk elements (64 slots of a row, two 32 x 32 tiles) a descriptor takes
+template <class D>
+inline int64_t mode_chunks(const D& d) {
+    if (d.mode == SumDesc::TILES) return (d.units + 1) / 2;
+    if (d.mode == SumDesc::ROWS) return (d.units + kRowSlots - 1) / kRowSlots;
+    return (d.total + kBatchChunk - 1) / kBatchChunk;
 }
-// fill the tiling fields of a descriptor (after len / sA / sC / total)
-void sum_plan_tiles(SumDesc& d);
+// merge positions and choose the mode of a descriptor (after len / sA / sC / total)
+void sum_plan(SumDesc& d);
+void dot_plan(DotDesc& d);
 struct ScaleDesc {
     double* X = nullptr;
     int64_t n = 0;

@@ -1226,38 +1226,46 @@ __global__ void axpby_kernel(const double* __restrict__ x, double* __restrict__ 
         y[i] = a * x[i] + (b == 0.0 ? 0.0 : b * y[i]);
 }
 
-__device__ __forceinline__ double den_of(const WeightArgs& w, int64_t l) {
-    double den = 0;
-    int64_t r = l;
-    for (int d = 0; d < w.ndim; d++) {
-        int64_t x = r % w.len[d];
-        r /= w.len[d];
-        den += w.d[d][x];
+// denominators of elements l[0..P) (past the end: any index below total), a position's factors
+// read once for all of them
+template <int P>
+__device__ __forceinline__ void den_of(const WeightArgs& w, const int64_t (&l)[P], double (&den)[P]) {
+#pragma unroll
+    for (int q = 0; q < P; q++) den[q] = 0;
+    if (w.fast) {
+        uint32_t r[P];
+#pragma unroll
+        for (int q = 0; q < P; q++) r[q] = (uint32_t)l[q];
+        for (int d = 0; d < w.ndim; d++) {
+            const uint32_t mul = w.dmul[d], shr = w.dshr[d], len = (uint32_t)w.len[d];
+            const double* e = w.d[d];
+#pragma unroll
+            for (int q = 0; q < P; q++) {
+                const uint32_t t = (uint32_t)(((uint64_t)__umulhi(r[q], mul) + r[q]) >> shr);
+                den[q] += __ldg(e + (r[q] - t * len));
+                r[q] = t;
+            }
+        }
+        return;
     }
-    return den;
+#pragma unroll
+    for (int q = 0; q < P; q++) {
+        int64_t r = l[q];
+        for (int d = 0; d < w.ndim; d++) {
+            int64_t x = r % w.len[d];
+            r /= w.len[d];
+            den[q] += w.d[d][x];
+        }
+    }
 }
 
 __global__ void weight_kernel(double* X, WeightArgs w, double shift) {
     for (int64_t l = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; l < w.total;
          l += (int64_t)gridDim.x * blockDim.x) {
-        double den = den_of(w, l) + shift;
-        X[l] = fabs(den) < 1e-4 ? 0.0 : X[l] / den;
+        double den[1];
+        den_of<1>(w, {l}, den);
+        X[l] = fabs(den[0] + shift) < 1e-4 ? 0.0 : X[l] / (den[0] + shift);
     }
-}
-
-// z = z/den (0 if |den| < 1e-4), t += z, block max |z|
-__global__ void update_kernel(double* __restrict__ Z, double* __restrict__ T, WeightArgs w, double* partial) {
-    double mx = 0;
-    for (int64_t l = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; l < w.total;
-         l += (int64_t)gridDim.x * blockDim.x) {
-        double den = den_of(w, l);
-        double z = fabs(den) < 1e-4 ? 0.0 : Z[l] / den;
-        Z[l] = z;
-        T[l] += z;
-        mx = fmax(mx, fabs(z));
-    }
-    mx = block_max(mx);
-    if (threadIdx.x == 0) partial[blockIdx.x] = mx;
 }
 
 __global__ void kv_write_kernel(double* X, const int64_t* keys, const double* vals, int64_t n, double a, double b) {
@@ -1273,40 +1281,88 @@ __global__ void kv_read_kernel(const double* X, const int64_t* keys, double* val
 }
 
 // batched dot: partial[b * ny + j] = sum over the block's range of x * ys[j]
-__global__ void dot_batch_kernel(const double* __restrict__ x, const double* const* ys, int ny, int64_t n,
-                                 double* partial) {
-    double s[16];
-    for (int j = 0; j < 16; j++) s[j] = 0;
-    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
-        double xv = x[i];
-        for (int j = 0; j < ny; j++) s[j] += xv * ys[j][i];
-    }
-    for (int j = 0; j < ny; j++) {
-        double t = block_sum(s[j]);
-        if (threadIdx.x == 0) partial[blockIdx.x * ny + j] = t;
-    }
+// out[j] = sum of partial[b][j] over b, one CTA per j
+__global__ void fold_batch_kernel(const double* partial, int nb, int ny, double* out) {
+    const int j = blockIdx.x;
+    double s = 0;
+#pragma unroll 4
+    for (int b = threadIdx.x; b < nb; b += blockDim.x) s += partial[b * ny + j];
+    s = block_sum(s);
+    if (threadIdx.x == 0) out[j] = s;
 }
 
-__global__ void fold_batch_kernel(const double* partial, int nb, int ny, double w, double* out) {
-    for (int j = 0; j < ny; j++) {
-        double s = 0;
-        for (int b = threadIdx.x; b < nb; b += blockDim.x) s += partial[b * ny + j];
-        s = block_sum(s);
-        if (threadIdx.x == 0) out[j] += w * s;
+// sum_j c[j] xs[j][i] of two elements at a time, the vectors' loads in flight together (a
+// vector with c[j] = 0 is not read).  HBM bounds it: T2 of o=20 v=144 with eight vectors (1.8 GB)
+// took 310 us with one load in flight per thread and takes 265.
+template <int N, class Out>
+__device__ __forceinline__ void lincomb_body(int64_t n, const double* const* xs, int64_t off, const double* c, Out out) {
+    __shared__ const double* sx[N];
+    __shared__ double sc[N];
+    if (threadIdx.x < N) {
+        sx[threadIdx.x] = xs[threadIdx.x] + off;
+        sc[threadIdx.x] = c[threadIdx.x];
     }
-}
-
-__global__ void lincomb_kernel(double* __restrict__ out1, int64_t n1, double* __restrict__ out2, int64_t n2,
-                               const double* const* xs, const double* c, int nx) {
-    const int64_t n = n1 + n2;
-    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
-        double s = 0;
-        for (int j = 0; j < nx; j++) {
-            double cj = c[j];
-            if (cj != 0.0) s += cj * xs[j][i];
+    __syncthreads();
+    const int64_t step = (int64_t)gridDim.x * blockDim.x;
+    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += 2 * step) {
+        const int64_t i1 = i + step;
+        const bool two = i1 < n;
+        double v[2][N];
+#pragma unroll
+        for (int j = 0; j < N; j++) {
+            const bool use = sc[j] != 0.0;
+            v[0][j] = use ? __ldg(sx[j] + i) : 0.0;
+            v[1][j] = use && two ? __ldg(sx[j] + i1) : 0.0;
         }
-        if (i < n1) out1[i] = s;
-        else out2[i - n1] = s;
+        double s0 = 0, s1 = 0;
+#pragma unroll
+        for (int j = 0; j < N; j++) {
+            s0 += sc[j] * v[0][j];
+            s1 += sc[j] * v[1][j];
+        }
+        out(i, s0);
+        if (two) out(i1, s1);
+    }
+}
+
+template <int N>
+__global__ void __launch_bounds__(EW_THREADS) lincomb_kernel(double* __restrict__ out1, int64_t n1, double* __restrict__ out2,
+                                                             int64_t n2, const double* const* xs, const double* c) {
+    lincomb_body<N>(n1 + n2, xs, 0, c, [&](int64_t i, double v) {
+        if (i < n1) out1[i] = v;
+        else out2[i - n1] = v;
+    });
+}
+
+// out[i] = sum_j c[j] * xs[j][off + i]
+template <int N>
+__global__ void __launch_bounds__(EW_THREADS) lincomb_segment_kernel(double* __restrict__ out, int64_t len,
+                                                                     const double* const* xs, int64_t off,
+                                                                     const double* c) {
+    lincomb_body<N>(len, xs, off, c, [&](int64_t i, double v) { out[i] = v; });
+}
+
+// f(std::integral_constant<int, n>) for a ring of n vectors
+template <class F>
+void for_vectors(int n, F f) {
+    switch (n) {
+        case 1: f(std::integral_constant<int, 1>()); break;
+        case 2: f(std::integral_constant<int, 2>()); break;
+        case 3: f(std::integral_constant<int, 3>()); break;
+        case 4: f(std::integral_constant<int, 4>()); break;
+        case 5: f(std::integral_constant<int, 5>()); break;
+        case 6: f(std::integral_constant<int, 6>()); break;
+        case 7: f(std::integral_constant<int, 7>()); break;
+        case 8: f(std::integral_constant<int, 8>()); break;
+        case 9: f(std::integral_constant<int, 9>()); break;
+        case 10: f(std::integral_constant<int, 10>()); break;
+        case 11: f(std::integral_constant<int, 11>()); break;
+        case 12: f(std::integral_constant<int, 12>()); break;
+        case 13: f(std::integral_constant<int, 13>()); break;
+        case 14: f(std::integral_constant<int, 14>()); break;
+        case 15: f(std::integral_constant<int, 15>()); break;
+        case 16: f(std::integral_constant<int, 16>()); break;
+        default: throw std::runtime_error("a DIIS ring holds 1 to 16 vectors");
     }
 }
 
@@ -1335,117 +1391,207 @@ double* partial_buffer(cudaStream_t s) {
 
 namespace {
 
+// the problem that chunk c belongs to (every thread gets it): a warp probes 32 first chunks at
+// a time, so that thousands of blocks take three dependent loads instead of twelve
 __device__ __forceinline__ int find_problem(const int64_t* __restrict__ cs, int n, int64_t c) {
-    int lo = 0, hi = n - 1;
-    while (lo < hi) {
-        const int mid = (lo + hi + 1) >> 1;
-        if (cs[mid] <= c) lo = mid;
-        else hi = mid - 1;
+    __shared__ int sp;
+    if (threadIdx.x < 32) {
+        int lo = 0, m = n;
+        while (m > 1) {
+            const int step = (m + 31) >> 5, i = lo + (int)threadIdx.x * step;
+            const unsigned below = __ballot_sync(0xffffffffu, i < lo + m && cs[min(i, n - 1)] <= c);
+            const int hit = __popc(below) - 1;
+            m = min(step, m - hit * step);
+            lo += hit * step;
+        }
+        if (threadIdx.x == 0) sp = lo;
     }
-    return lo;
+    __syncthreads();
+    return sp;
 }
 
-__global__ void __launch_bounds__(256) sum_batched_kernel(const SumDesc* __restrict__ d, const int64_t* __restrict__ cs,
-                                                          int n) {
-    __shared__ int sp;
-    __shared__ double tile[32][33];
-    const int64_t c = blockIdx.x;
-    if (threadIdx.x == 0) sp = find_problem(cs, n, c);
-    __syncthreads();
-    const SumDesc& D = d[sp];
-    if (D.tiled) {
-        // two 32 x 32 tiles over (p0, pc): read along p0 (A-contiguous), write along pc
-        const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;   // 32 x 8 threads
-        const int64_t l0 = D.len[D.p0], lc = D.len[D.pc];
-        const int64_t t0n = (l0 + 31) / 32, tcn = (lc + 31) / 32;
-        for (int tt = 0; tt < 2; tt++) {
-            const int64_t t = (c - cs[sp]) * 2 + tt;
-            if (t >= D.ntiles) break;   // uniform across the CTA
-            int64_t r = t;
-            const int64_t t0 = r % t0n;
-            r /= t0n;
-            const int64_t tc = r % tcn;
-            r /= tcn;
-            int64_t oa = 0, oc = 0;
-            for (int k = 0; k < D.ndim; k++) {
-                if (k == D.p0 || k == D.pc) continue;
-                const int64_t x = r % D.len[k];
-                r /= D.len[k];
-                oa += x * D.sA[k];
-                oc += x * D.sC[k];
-            }
-            const int64_t x0 = t0 * 32 + tx;
+// a descriptor into shared memory (its fields are read in every loop); sync before use
+template <class D>
+__device__ __forceinline__ void stage_desc(D* dst, const D* __restrict__ src) {
+    static_assert(sizeof(D) % 8 == 0, "copied in 8-byte words");
+    for (int i = threadIdx.x; i < (int)(sizeof(D) / 8); i += blockDim.x)
+        reinterpret_cast<uint64_t*>(dst)[i] = __ldg(reinterpret_cast<const unsigned long long*>(src) + i);
+}
+
+// x / len[k] of a descriptor's position k
+template <class D>
+__device__ __forceinline__ int64_t div_pos(const D& d, int k, int64_t x) {
+    if (d.fast) return (uint32_t)(((uint64_t)__umulhi((uint32_t)x, d.dmul[k]) + (uint32_t)x) >> d.dshr[k]);
+    return x / d.len[k];
+}
+
+// Offsets of kPer elements of this thread in half h (of two) of chunk c, -1 past the end: of
+// A and of the other operand (strides sX).  ROWS: a warp walks eight consecutive slots of 32
+// neighbours and splits the row number only when the row changes.
+constexpr int kPer = 4;
+template <class D>
+__device__ __forceinline__ void chunk_offsets(const D& d, const int64_t* sX, int64_t c, int h, int64_t (&oa)[kPer],
+                                              int64_t (&ox)[kPer]) {
+    if (d.mode == SumDesc::ROWS) {
+        const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+        const int64_t slot = c * kRowSlots + warp * (2 * kPer) + h * kPer;
+        int64_t row = slot / d.spr;
+        int seg = (int)(slot - row * d.spr);
+        bool fresh = true;
+        int64_t ra = 0, rx = 0;
 #pragma unroll
-            for (int q = 0; q < 4; q++) {
-                const int64_t xc = tc * 32 + ty + 8 * q;
-                tile[ty + 8 * q][tx] = (x0 < l0 && xc < lc) ? D.A[oa + x0 * D.sA[D.p0] + xc * D.sA[D.pc]] : 0.0;
+        for (int q = 0; q < kPer; q++) {
+            if (fresh) {
+                ra = rx = 0;
+                int64_t r = row;
+                for (int k = 1; k < d.ndim; k++) {
+                    const int64_t t = div_pos(d, k, r), x = r - t * d.len[k];
+                    ra += x * d.sA[k];
+                    rx += x * sX[k];
+                    r = t;
+                }
+                fresh = false;
             }
-            __syncthreads();
-            const int64_t xc = tc * 32 + tx;
-#pragma unroll
-            for (int q = 0; q < 4; q++) {
-                const int64_t y0 = t0 * 32 + ty + 8 * q;
-                if (y0 < l0 && xc < lc) D.C[oc + y0 * D.sC[D.p0] + xc * D.sC[D.pc]] += D.alpha * tile[tx][ty + 8 * q];
+            const int64_t x = seg * 32 + lane;
+            const bool ok = slot + q < d.units && x < d.len[0];
+            oa[q] = ok ? ra + x : -1;
+            ox[q] = ok ? rx + x : -1;
+            if (++seg == d.spr) {
+                seg = 0;
+                row++;
+                fresh = true;
             }
-            __syncthreads();
         }
         return;
     }
-    // a thread's elements in batches of four: the offsets, then the loads, then the stores,
-    // so that the loads of a batch are in flight together (batches of four keep the
-    // registers, and with them the occupancy of the tiled path of this kernel, low)
-    constexpr int PER = 4;
-    for (int half = 0; half < kBatchChunk / (256 * PER); half++) {
-    const int64_t base = (c - cs[sp]) * kBatchChunk + half * 256 * PER;
-    int64_t oa[PER], oc[PER];
+    const int64_t l0 = c * kBatchChunk + h * 256 * kPer + threadIdx.x;
 #pragma unroll
-    for (int q = 0; q < PER; q++) {
-        const int64_t l = base + threadIdx.x + q * 256;
-        oa[q] = -1;
-        oc[q] = 0;
-        if (l >= D.total) continue;
-        int64_t a = 0, cc = 0;
-        if (D.fast) {
-            uint32_t r = (uint32_t)l;
-            for (int k = 0; k < D.ndim; k++) {
-                const uint32_t qq = (uint32_t)(((uint64_t)__umulhi(r, D.dmul[k]) + r) >> D.dshr[k]);
-                const uint32_t x = r - qq * (uint32_t)D.len[k];
-                a += (int64_t)x * D.sA[k];
-                cc += (int64_t)x * D.sC[k];
-                r = qq;
-            }
-        } else {
-            int64_t r = l;
-            for (int k = 0; k < D.ndim; k++) {
-                const int64_t x = r % D.len[k];
-                r /= D.len[k];
-                a += x * D.sA[k];
-                cc += x * D.sC[k];
+    for (int q = 0; q < kPer; q++) oa[q] = ox[q] = l0 + q * 256 < d.total ? 0 : -1;
+    if (d.fast) {
+        uint32_t r[kPer];
+#pragma unroll
+        for (int q = 0; q < kPer; q++) r[q] = (uint32_t)(l0 + q * 256);
+        for (int k = 0; k < d.ndim; k++) {
+            const uint32_t mul = d.dmul[k], shr = d.dshr[k], len = (uint32_t)d.len[k];
+            const int64_t sa = d.sA[k], sx = sX[k];
+#pragma unroll
+            for (int q = 0; q < kPer; q++) {
+                const uint32_t t = (uint32_t)(((uint64_t)__umulhi(r[q], mul) + r[q]) >> shr), x = r[q] - t * len;
+                if (oa[q] >= 0) {
+                    oa[q] += x * sa;
+                    ox[q] += x * sx;
+                }
+                r[q] = t;
             }
         }
-        oa[q] = a;
-        oc[q] = cc;
-    }
-    double va[PER], vc[PER];
-#pragma unroll
-    for (int q = 0; q < PER; q++) {
-        va[q] = oa[q] >= 0 ? D.A[oa[q]] : 0.0;
-        vc[q] = oa[q] >= 0 ? D.C[oc[q]] : 0.0;
+        return;
     }
 #pragma unroll
-    for (int q = 0; q < PER; q++)
-        if (oa[q] >= 0) D.C[oc[q]] = vc[q] + D.alpha * va[q];
+    for (int q = 0; q < kPer; q++) {
+        if (oa[q] < 0) continue;
+        int64_t r = l0 + q * 256;
+        for (int k = 0; k < d.ndim; k++) {
+            const int64_t t = r / d.len[k], x = r - t * d.len[k];
+            oa[q] += x * d.sA[k];
+            ox[q] += x * sX[k];
+            r = t;
+        }
+    }
+}
+
+// Tile t of a TILES descriptor (32 x 32 over the fastest positions p0 of A and pc of the other
+// operand): its corner (past the extents where t is past the end) and the operands' offsets
+template <class D>
+__device__ __forceinline__ void tile_corner(const D& d, const int64_t* sX, int64_t t, int64_t& x0, int64_t& xc,
+                                            int64_t& oa, int64_t& ox) {
+    const int64_t l0 = d.len[d.p0], lc = d.len[d.pc];
+    const int64_t t0n = (l0 + 31) / 32, tcn = (lc + 31) / 32;
+    oa = ox = 0;
+    x0 = l0;
+    xc = lc;
+    if (t >= d.units) return;
+    int64_t r = t / t0n;
+    x0 = (t - r * t0n) * 32;
+    const int64_t u = r / tcn;
+    xc = (r - u * tcn) * 32;
+    r = u;
+    for (int k = 0; k < d.ndim; k++) {
+        if (k == d.p0 || k == d.pc) continue;
+        const int64_t v = div_pos(d, k, r), x = r - v * d.len[k];
+        oa += x * d.sA[k];
+        ox += x * sX[k];
+        r = v;
+    }
+}
+
+// Permuted sums (antisymmetriser images, copies): HBM bounds them, 24 bytes per element (16
+// where the sum assigns).  Copies and sums of equal layouts merge to one long row.  o=24 v=184: the
+// copy of <am||ei> (117M elements) 860 us as a scaling and a sum that splits every index, 434
+// as an assignment; images of the ring (39M elements) 247 -> 147.
+__global__ void __launch_bounds__(256) sum_batched_kernel(const SumDesc* __restrict__ d, const int64_t* __restrict__ cs,
+                                                          int n) {
+    __shared__ SumDesc D;
+    __shared__ double tile[2][32][33];
+    const int p = find_problem(cs, n, blockIdx.x);
+    stage_desc(&D, d + p);
+    const int64_t c = blockIdx.x - cs[p];
+    __syncthreads();
+    if (D.mode == SumDesc::TILES) {
+        // two 32 x 32 tiles over (p0, pc): read along p0 (A-contiguous), write along pc; the
+        // reads of both tiles and of C are in flight together
+        const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;   // 32 x 8 threads
+        const int64_t l0 = D.len[D.p0], lc = D.len[D.pc];
+        const int64_t sa0 = D.sA[D.p0], sac = D.sA[D.pc], sc0 = D.sC[D.p0], scc = D.sC[D.pc];
+        double va[2][4], vc[2][4];
+        int64_t oc[2], x0[2], xc[2];
+#pragma unroll
+        for (int tt = 0; tt < 2; tt++) {
+            int64_t oa;
+            tile_corner(D, D.sC, c * 2 + tt, x0[tt], xc[tt], oa, oc[tt]);
+#pragma unroll
+            for (int q = 0; q < 4; q++) {
+                const int64_t y0 = x0[tt] + tx, yc = xc[tt] + ty + 8 * q;
+                va[tt][q] = y0 < l0 && yc < lc ? __ldg(D.A + oa + y0 * sa0 + yc * sac) : 0.0;
+                const int64_t z0 = x0[tt] + ty + 8 * q, zc = xc[tt] + tx;
+                vc[tt][q] = !D.assign && z0 < l0 && zc < lc ? D.C[oc[tt] + z0 * sc0 + zc * scc] : 0.0;
+            }
+        }
+#pragma unroll
+        for (int tt = 0; tt < 2; tt++)
+#pragma unroll
+            for (int q = 0; q < 4; q++) tile[tt][ty + 8 * q][tx] = va[tt][q];
+        __syncthreads();
+#pragma unroll
+        for (int tt = 0; tt < 2; tt++)
+#pragma unroll
+            for (int q = 0; q < 4; q++) {
+                const int64_t z0 = x0[tt] + ty + 8 * q, zc = xc[tt] + tx;
+                if (z0 < l0 && zc < lc) D.C[oc[tt] + z0 * sc0 + zc * scc] = vc[tt][q] + D.alpha * tile[tt][tx][ty + 8 * q];
+            }
+        return;
+    }
+#pragma unroll
+    for (int h = 0; h < 2; h++) {
+        int64_t oa[kPer], oc[kPer];
+        chunk_offsets(D, D.sC, c, h, oa, oc);
+        double va[kPer], vc[kPer];
+#pragma unroll
+        for (int q = 0; q < kPer; q++) {
+            va[q] = oa[q] >= 0 ? __ldg(D.A + oa[q]) : 0.0;
+            vc[q] = oa[q] >= 0 && !D.assign ? D.C[oc[q]] : 0.0;
+        }
+#pragma unroll
+        for (int q = 0; q < kPer; q++)
+            if (oa[q] >= 0) D.C[oc[q]] = vc[q] + D.alpha * va[q];
     }
 }
 
 __global__ void __launch_bounds__(256) scale_batched_kernel(const ScaleDesc* __restrict__ d,
                                                             const int64_t* __restrict__ cs, int n) {
-    __shared__ int sp;
-    const int64_t c = blockIdx.x;
-    if (threadIdx.x == 0) sp = find_problem(cs, n, c);
-    __syncthreads();
-    const ScaleDesc& D = d[sp];
-    const int64_t base = (c - cs[sp]) * kBatchChunk;
+    const int p = find_problem(cs, n, blockIdx.x);
+    const ScaleDesc D = d[p];
+    const int64_t base = (blockIdx.x - cs[p]) * kBatchChunk;
+#pragma unroll 4
     for (int i = threadIdx.x; i < kBatchChunk; i += blockDim.x) {
         const int64_t l = base + i;
         if (l >= D.n) break;
@@ -1453,107 +1599,144 @@ __global__ void __launch_bounds__(256) scale_batched_kernel(const ScaleDesc* __r
     }
 }
 
-// Tau of one chunk of one block (tau_kernel's arithmetic)
+// Tau of one chunk of one block; HBM bounds it, 16 bytes per element
 __global__ void __launch_bounds__(256) tau_batched_kernel(const TauArgs* __restrict__ d, const int64_t* __restrict__ cs,
                                                           int n) {
-    __shared__ int sp;
-    const int64_t c = blockIdx.x;
-    if (threadIdx.x == 0) sp = find_problem(cs, n, c);
+    __shared__ TauArgs a;
+    const int p = find_problem(cs, n, blockIdx.x);
+    stage_desc(&a, d + p);
+    const int64_t base = (blockIdx.x - cs[p]) * kBatchChunk;
     __syncthreads();
-    const TauArgs& a = d[sp];
-    const int64_t la = a.len[0], lb = a.len[1], li = a.len[2], lj = a.len[3];
-    const int64_t total = la * lb * li * lj;
-    const int64_t base = (c - cs[sp]) * kBatchChunk;
-    for (int i = threadIdx.x; i < kBatchChunk; i += blockDim.x) {
-        const int64_t l = base + i;
-        if (l >= total) break;
-        int64_t r = l;
-        const int64_t x = r % la;
-        r /= la;
-        const int64_t y = r % lb;
-        r /= lb;
-        const int64_t ii = r % li;
-        const int64_t j = r / li;
-        double v = a.t2[l];
-        if (a.t1ai) v += a.t1ai[x + la * ii] * a.t1bj[y + lb * j];
-        if (a.t1aj) v -= a.t1aj[x + la * j] * a.t1bi[y + lb * ii];
-        a.tau[l] = v;
+    const int64_t la = a.len[0], lb = a.len[1], total = la * lb * a.len[2] * a.len[3];
+    const double *ai = a.t1ai, *bj = a.t1bj, *aj = a.t1aj, *bi = a.t1bi;
+    const bool fast = a.fast != 0;
+    const uint32_t n0 = (uint32_t)la, n1 = (uint32_t)lb, n2 = (uint32_t)a.len[2];
+    const uint32_t m0 = a.dmul[0], m1 = a.dmul[1], m2 = a.dmul[2], s0 = a.dshr[0], s1 = a.dshr[1], s2 = a.dshr[2];
+    constexpr int P = kBatchChunk / 256;
+    double v[P];
+#pragma unroll
+    for (int q = 0; q < P; q++) {
+        const int64_t l = base + q * 256 + threadIdx.x;
+        v[q] = l < total ? __ldg(a.t2 + l) : 0.0;
+    }
+#pragma unroll
+    for (int q = 0; q < P; q++) {
+        const int64_t l = base + q * 256 + threadIdx.x;
+        if (l >= total) continue;
+        if (ai || aj) {
+            int64_t x, y, i, j;
+            if (fast) {
+                uint32_t r = (uint32_t)l, t = (uint32_t)(((uint64_t)__umulhi(r, m0) + r) >> s0);
+                x = r - t * n0;
+                r = t;
+                t = (uint32_t)(((uint64_t)__umulhi(r, m1) + r) >> s1);
+                y = r - t * n1;
+                r = t;
+                t = (uint32_t)(((uint64_t)__umulhi(r, m2) + r) >> s2);
+                i = r - t * n2;
+                j = t;
+            } else {
+                x = l % la;
+                y = l / la % lb;
+                i = l / (la * lb) % a.len[2];
+                j = l / (la * lb) / a.len[2];
+            }
+            if (ai) v[q] += __ldg(ai + x + la * i) * __ldg(bj + y + lb * j);
+            if (aj) v[q] -= __ldg(aj + x + la * j) * __ldg(bi + y + lb * i);
+        }
+        a.tau[l] = v[q];
     }
 }
 
 // Jacobi update of one chunk of one block; the residual max goes to red_max through an
-// atomic max on the bits of non-negative doubles (order-independent)
+// atomic max on the bits of non-negative doubles (order-independent).  HBM bounds it, 32
+// bytes per element.
 __global__ void __launch_bounds__(256) update_batched_kernel(const UpdateDesc* __restrict__ d,
                                                              const int64_t* __restrict__ cs, int n, double* red_max) {
-    __shared__ int sp;
-    const int64_t c = blockIdx.x;
-    if (threadIdx.x == 0) sp = find_problem(cs, n, c);
+    __shared__ UpdateDesc D;
+    const int p = find_problem(cs, n, blockIdx.x);
+    stage_desc(&D, d + p);
+    const int64_t base = (blockIdx.x - cs[p]) * kBatchChunk;
     __syncthreads();
-    const UpdateDesc& D = d[sp];
-    const int64_t base = (c - cs[sp]) * kBatchChunk;
     double mx = 0;
-    for (int i = threadIdx.x; i < kBatchChunk; i += blockDim.x) {
-        const int64_t l = base + i;
-        if (l >= D.w.total) break;
-        const double den = den_of(D.w, l);
-        const double z = fabs(den) < 1e-4 ? 0.0 : D.Z[l] / den;
-        D.Z[l] = z;
-        D.T[l] += z;
-        mx = fmax(mx, fabs(z));
+#pragma unroll
+    for (int h = 0; h < 2; h++) {
+        double z[kPer], t[kPer];
+#pragma unroll
+        for (int q = 0; q < kPer; q++) {
+            const int64_t l = base + (h * kPer + q) * 256 + threadIdx.x;
+            z[q] = l < D.w.total ? D.Z[l] : 0.0;
+            t[q] = l < D.w.total ? D.T[l] : 0.0;
+        }
+        int64_t l[kPer];
+        double den[kPer];
+#pragma unroll
+        for (int q = 0; q < kPer; q++) l[q] = min(base + (h * kPer + q) * 256 + threadIdx.x, D.w.total - 1);
+        den_of<kPer>(D.w, l, den);
+#pragma unroll
+        for (int q = 0; q < kPer; q++) {
+            if (base + (h * kPer + q) * 256 + threadIdx.x >= D.w.total) continue;
+            const double x = fabs(den[q]) < 1e-4 ? 0.0 : z[q] / den[q];
+            D.Z[l[q]] = x;
+            D.T[l[q]] = t[q] + x;
+            mx = fmax(mx, fabs(x));
+        }
     }
     mx = block_max(mx);
     if (threadIdx.x == 0 && mx > 0.0)
         atomicMax(reinterpret_cast<unsigned long long*>(red_max), (unsigned long long)__double_as_longlong(mx));
 }
 
-// dot of one chunk of one block into part[c]
+// dot of one chunk of one block into part[c]; HBM bounds it, 16 bytes per element (the energy of
+// o=24 v=184, 117M elements through a permuted view: 1060 us element by element, 446 by tiles)
 __global__ void __launch_bounds__(256) dot_batched_kernel(const DotDesc* __restrict__ d, const int64_t* __restrict__ cs,
                                                           int n, double* part) {
-    __shared__ int sp;
-    const int64_t c = blockIdx.x;
-    if (threadIdx.x == 0) sp = find_problem(cs, n, c);
+    __shared__ DotDesc D;
+    __shared__ double tile[2][32][33];
+    const int p = find_problem(cs, n, blockIdx.x);
+    stage_desc(&D, d + p);
+    const int64_t c = blockIdx.x - cs[p];
     __syncthreads();
-    const DotDesc& D = d[sp];
-    const int64_t base = (c - cs[sp]) * kBatchChunk;
     double acc = 0;
-    // batches of four elements: the offsets first, then the loads (in flight together)
-    constexpr int PER = 4;
-    for (int half = 0; half < kBatchChunk / (256 * PER); half++) {
-    int64_t oa[PER], ob[PER];
+    if (D.mode == SumDesc::TILES) {
+        // as the sum's tiles: A read along p0, B along pc
+        const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
+        const int64_t l0 = D.len[D.p0], lc = D.len[D.pc];
+        const int64_t sa0 = D.sA[D.p0], sac = D.sA[D.pc], sb0 = D.sB[D.p0], sbc = D.sB[D.pc];
+        double va[2][4], vb[2][4];
 #pragma unroll
-    for (int q = 0; q < PER; q++) {
-        const int64_t l = base + half * 256 * PER + threadIdx.x + q * 256;
-        oa[q] = -1;
-        ob[q] = 0;
-        if (l >= D.total) continue;
-        int64_t a = 0, b = 0;
-        if (D.fast) {
-            uint32_t r = (uint32_t)l;
-            for (int k = 0; k < D.ndim; k++) {
-                const uint32_t qq = (uint32_t)(((uint64_t)__umulhi(r, D.dmul[k]) + r) >> D.dshr[k]);
-                const uint32_t x = r - qq * (uint32_t)D.len[k];
-                a += (int64_t)x * D.sA[k];
-                b += (int64_t)x * D.sB[k];
-                r = qq;
-            }
-        } else {
-            int64_t r = l;
-            for (int k = 0; k < D.ndim; k++) {
-                const int64_t x = r % D.len[k];
-                r /= D.len[k];
-                a += x * D.sA[k];
-                b += x * D.sB[k];
+        for (int tt = 0; tt < 2; tt++) {
+            int64_t x0, xc, oa, ob;
+            tile_corner(D, D.sB, c * 2 + tt, x0, xc, oa, ob);
+#pragma unroll
+            for (int q = 0; q < 4; q++) {
+                const int64_t y0 = x0 + tx, yc = xc + ty + 8 * q;
+                va[tt][q] = y0 < l0 && yc < lc ? __ldg(D.A + oa + y0 * sa0 + yc * sac) : 0.0;
+                const int64_t z0 = x0 + ty + 8 * q, zc = xc + tx;
+                vb[tt][q] = z0 < l0 && zc < lc ? __ldg(D.B + ob + z0 * sb0 + zc * sbc) : 0.0;
             }
         }
-        oa[q] = a;
-        ob[q] = b;
-    }
 #pragma unroll
-    for (int q = 0; q < PER; q++)
-        if (oa[q] >= 0) acc += D.A[oa[q]] * D.B[ob[q]];
+        for (int tt = 0; tt < 2; tt++)
+#pragma unroll
+            for (int q = 0; q < 4; q++) tile[tt][ty + 8 * q][tx] = va[tt][q];
+        __syncthreads();
+#pragma unroll
+        for (int tt = 0; tt < 2; tt++)
+#pragma unroll
+            for (int q = 0; q < 4; q++) acc += vb[tt][q] * tile[tt][tx][ty + 8 * q];
+    } else {
+#pragma unroll
+    for (int h = 0; h < 2; h++) {
+        int64_t oa[kPer], ob[kPer];
+        chunk_offsets(D, D.sB, c, h, oa, ob);
+#pragma unroll
+        for (int q = 0; q < kPer; q++)
+            if (oa[q] >= 0) acc += __ldg(D.A + oa[q]) * __ldg(D.B + ob[q]);
+    }
     }
     acc = block_sum(acc);
-    if (threadIdx.x == 0) part[c] = D.alpha * acc;
+    if (threadIdx.x == 0) part[blockIdx.x] = D.alpha * acc;
 }
 
 }  // namespace
@@ -1576,22 +1759,70 @@ void plan_divisors(const int64_t* lens, int ndim, int64_t total, int& fast, uint
     }
 }
 
-void sum_plan_tiles(SumDesc& d) {
-    d.tiled = 0;
+namespace {
+// Positions in order of the stride sX, extents of 1 dropped, neighbours that run through both
+// operands without a gap merged; ROWS where the fastest position is contiguous in both and a
+// row fills half of a warp or more, TILES where the fastest positions differ and fill a
+// quarter of a tile's side.
+template <class D>
+void plan_positions(D& d, int64_t* sX) {
+    int n = 0;
+    for (int k = 0; k < d.ndim; k++) {
+        if (d.len[k] == 1) continue;
+        const int64_t len = d.len[k], sa = d.sA[k], sx = sX[k];
+        int at = n++;
+        for (; at > 0 && sX[at - 1] > sx; at--) {
+            d.len[at] = d.len[at - 1];
+            d.sA[at] = d.sA[at - 1];
+            sX[at] = sX[at - 1];
+        }
+        d.len[at] = len;
+        d.sA[at] = sa;
+        sX[at] = sx;
+    }
+    d.ndim = 0;
+    for (int k = 0; k < n; k++) {
+        const int j = d.ndim - 1;
+        if (j >= 0 && d.sA[k] == d.sA[j] * d.len[j] && sX[k] == sX[j] * d.len[j]) {
+            d.len[j] *= d.len[k];
+            continue;
+        }
+        d.len[d.ndim] = d.len[k];
+        d.sA[d.ndim] = d.sA[k];
+        sX[d.ndim++] = sX[k];
+    }
     plan_divisors(d.len, d.ndim, d.total, d.fast, d.dmul, d.dshr);
+    d.mode = SumDesc::ELEMENTS;
+    if (d.ndim > 0 && d.sA[0] == 1 && sX[0] == 1 && d.len[0] >= 16 && d.len[0] < ((int64_t)1 << 31)) {
+        d.mode = SumDesc::ROWS;
+        d.spr = (int)((d.len[0] + 31) / 32);
+        d.units = d.total / d.len[0] * d.spr;
+        return;
+    }
     if (d.ndim < 2) return;
     int p0 = 0, pc = 0;
     for (int k = 1; k < d.ndim; k++) {
         if (d.sA[k] < d.sA[p0]) p0 = k;
-        if (d.sC[k] < d.sC[pc]) pc = k;
+        if (sX[k] < sX[pc]) pc = k;
     }
     if (p0 == pc || d.len[p0] < 8 || d.len[pc] < 8) return;
-    d.tiled = 1;
+    d.mode = SumDesc::TILES;
     d.p0 = p0;
     d.pc = pc;
-    d.ntiles = ((d.len[p0] + 31) / 32) * ((d.len[pc] + 31) / 32);
+    d.units = ((d.len[p0] + 31) / 32) * ((d.len[pc] + 31) / 32);
     for (int k = 0; k < d.ndim; k++)
-        if (k != p0 && k != pc) d.ntiles *= d.len[k];
+        if (k != p0 && k != pc) d.units *= d.len[k];
+}
+}  // namespace
+
+void sum_plan(SumDesc& d) { plan_positions(d, d.sC); }
+
+void dot_plan(DotDesc& d) { plan_positions(d, d.sB); }
+
+void weight_plan(WeightArgs& w) { plan_divisors(w.len, w.ndim, w.total, w.fast, w.dmul, w.dshr); }
+
+void tau_plan(TauArgs& a) {
+    plan_divisors(a.len, 4, a.len[0] * a.len[1] * a.len[2] * a.len[3], a.fast, a.dmul, a.dshr);
 }
 
 void sum_batched(const SumDesc* d, const int64_t* chunk_start, int n, int64_t chunks, cudaStream_t s) {
@@ -1690,16 +1921,6 @@ void weight_block(double* X, const WeightArgs& w, double shift, cudaStream_t s) 
     COUNT_LAUNCH();
 }
 
-void update_block(double* Z, double* T, const WeightArgs& w, double* red_max, cudaStream_t s) {
-    if (w.total <= 0) return;
-    int nb = ew_blocks(w.total);
-    double* part = partial_buffer(s);
-    update_kernel<<<nb, EW_THREADS, 0, s>>>(Z, T, w, part);
-    fold_norm_kernel<<<1, 1024, 0, s>>>(part, nb, 0, 1.0, red_max);
-    COUNT_LAUNCH();
-    COUNT_LAUNCH();
-}
-
 void kv_write(double* X, const int64_t* keys, const double* vals, int64_t n, double alpha, double beta,
               cudaStream_t s) {
     if (n <= 0) return;
@@ -1713,21 +1934,12 @@ void kv_read(const double* X, const int64_t* keys, double* vals, int64_t n, cuda
     COUNT_LAUNCH();
 }
 
-void dot_batch(const double* x, const double* const* ys, int ny, int64_t n, double w, double* out,
-               cudaStream_t s) {
-    if (n <= 0 || ny <= 0) return;
-    int nb = ew_blocks(n);
-    double* part = partial_buffer(s);
-    dot_batch_kernel<<<nb, EW_THREADS, 0, s>>>(x, ys, ny, n, part);
-    fold_batch_kernel<<<1, 1024, 0, s>>>(part, nb, ny, w, out);
-    COUNT_LAUNCH();
-    COUNT_LAUNCH();
-}
-
 void lincomb(double* out1, int64_t n1, double* out2, int64_t n2, const double* const* xs, const double* c, int nx,
              cudaStream_t s) {
     if (n1 + n2 <= 0) return;
-    lincomb_kernel<<<ew_blocks(n1 + n2), EW_THREADS, 0, s>>>(out1, n1, out2, n2, xs, c, nx);
+    for_vectors(nx, [&](auto N) {
+        lincomb_kernel<decltype(N)::value><<<ew_blocks((n1 + n2 + 1) / 2), EW_THREADS, 0, s>>>(out1, n1, out2, n2, xs, c);
+    });
     COUNT_LAUNCH();
 }
 
@@ -1759,20 +1971,42 @@ __global__ void diis_store_kernel(const int* st, const double* const* xs, const 
     }
 }
 
-__global__ void diis_dots_kernel(const int* st, const double* const* dxs, int order, int64_t off, int64_t len,
-                                 double* partial) {
-    const double* x = dxs[st[0]] + off;
-    double s[16];
-    for (int j = 0; j < 16; j++) s[j] = 0;
-    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < len; i += (int64_t)gridDim.x * blockDim.x) {
-        double xv = x[i];
+// <dxs[head], dxs[j]> of every vector over all weighted segments, a partial per CTA.  HBM
+// bounds it (each vector once); two elements of every vector are in flight per thread.
+template <int N>
+__global__ void __launch_bounds__(EW_THREADS) diis_dots_kernel(const int* st, const double* const* dxs,
+                                                               const DiisSegment* __restrict__ segs, int nsegs,
+                                                               double* partial) {
+    __shared__ const double* sx[N];
+    __shared__ const double* shead;
+    if (threadIdx.x < N) sx[threadIdx.x] = dxs[threadIdx.x];
+    if (threadIdx.x == 0) shead = dxs[st[0]];
+    __syncthreads();
+    double s[N];
 #pragma unroll
-        for (int j = 0; j < 16; j++)
-            if (j < order) s[j] += xv * dxs[j][off + i];
+    for (int j = 0; j < N; j++) s[j] = 0;
+    const int64_t step = (int64_t)gridDim.x * blockDim.x;
+    for (int q = 0; q < nsegs; q++) {
+        const DiisSegment g = segs[q];
+        const int64_t end = g.off + g.len;
+        for (int64_t i = g.off + blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < end; i += 2 * step) {
+            const int64_t i1 = i + step;
+            const bool two = i1 < end;
+            double v[2][N];
+            const double x0 = g.w * __ldg(shead + i), x1 = two ? g.w * __ldg(shead + i1) : 0.0;
+#pragma unroll
+            for (int j = 0; j < N; j++) {
+                v[0][j] = __ldg(sx[j] + i);
+                v[1][j] = two ? __ldg(sx[j] + i1) : 0.0;
+            }
+#pragma unroll
+            for (int j = 0; j < N; j++) s[j] += x0 * v[0][j] + x1 * v[1][j];
+        }
     }
-    for (int j = 0; j < order; j++) {
-        double t = block_sum(s[j]);
-        if (threadIdx.x == 0) partial[blockIdx.x * order + j] = t;
+#pragma unroll
+    for (int j = 0; j < N; j++) {
+        const double t = block_sum(s[j]);
+        if (threadIdx.x == 0) partial[blockIdx.x * N + j] = t;
     }
 }
 
@@ -1870,19 +2104,6 @@ __global__ void diis_store_segment_kernel(const int* st, const double* const* xs
     }
 }
 
-// out[i] = sum_j c[j] * xs[j][off + i]
-__global__ void lincomb_segment_kernel(double* __restrict__ out, int64_t len, const double* const* xs, int64_t off,
-                                       const double* c, int nx) {
-    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < len; i += (int64_t)gridDim.x * blockDim.x) {
-        double s = 0;
-        for (int j = 0; j < nx; j++) {
-            double cj = c[j];
-            if (cj != 0.0) s += cj * xs[j][off + i];
-        }
-        out[i] = s;
-    }
-}
-
 // diis.hpp:155-161: while the start counter is above 1 (and two vectors are stored), the
 // stored newest x becomes (damping - 1) x_0 + damping x_1
 __global__ void diis_damp_kernel(const int* st, const double* const* xs, int order, int64_t len, double damping) {
@@ -1938,23 +2159,6 @@ __global__ void pack_vvvv_kernel(double* V, int kab, int kcd, int n0, int n1, in
 }  // namespace
 
 namespace {
-__global__ void tau_kernel(TauArgs a) {
-    const int64_t la = a.len[0], lb = a.len[1], li = a.len[2], lj = a.len[3];
-    const int64_t n = la * lb * li * lj;
-    for (int64_t l = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; l < n; l += (int64_t)gridDim.x * blockDim.x) {
-        int64_t r = l;
-        const int64_t x = r % la;
-        r /= la;
-        const int64_t y = r % lb;
-        r /= lb;
-        const int64_t i = r % li;
-        const int64_t j = r / li;
-        double v = a.t2[l];
-        if (a.t1ai) v += a.t1ai[x + la * i] * a.t1bj[y + lb * j];
-        if (a.t1aj) v -= a.t1aj[x + la * j] * a.t1bi[y + lb * i];
-        a.tau[l] = v;
-    }
-}
 // 32 x 32 tiles of one matrix per blockIdx.z, 32 x 8 threads
 __global__ void transpose_factor_kernel(const double* __restrict__ in, double* __restrict__ out, int n) {
     __shared__ double tile[32][33];
@@ -2021,13 +2225,6 @@ void closed_shell_jk(const double* eri, int n, int nocc, double* F, cudaStream_t
     COUNT_LAUNCH();
 }
 
-void tau_block(const TauArgs& a, cudaStream_t s) {
-    const int64_t n = a.len[0] * a.len[1] * a.len[2] * a.len[3];
-    if (n <= 0) return;
-    tau_kernel<<<ew_blocks(n), EW_THREADS, 0, s>>>(a);
-    COUNT_LAUNCH();
-}
-
 void pack_vvvv(double* V, int kind_ab, int kind_cd, int n0, int n1, int n2, int n3, int64_t scd, const double* tJ,
                const double* tK, int a0, int a1, bool J, bool K, cudaStream_t s) {
     int64_t ncd = kind_cd == 1 ? (int64_t)n2 * (n2 - 1) / 2 : (int64_t)n2 * n3;
@@ -2049,13 +2246,14 @@ void diis_store(const int* state, const double* const* xs, const double* const* 
     COUNT_LAUNCH();
 }
 
-void diis_dots(const int* state, const double* const* dxs, int order, int64_t off, int64_t len, double w,
+void diis_dots(const int* state, const double* const* dxs, int order, const DiisSegment* segs, int nsegs, int64_t total,
                double* dots, cudaStream_t s) {
-    if (len <= 0) return;
-    int nb = ew_blocks(len);
+    const int nb = std::min(ew_blocks((total + 1) / 2), 148 * 8);
     double* part = partial_buffer(s);
-    diis_dots_kernel<<<nb, EW_THREADS, 0, s>>>(state, dxs, order, off, len, part);
-    fold_batch_kernel<<<1, 1024, 0, s>>>(part, nb, order, w, dots);
+    for_vectors(order, [&](auto N) {
+        diis_dots_kernel<decltype(N)::value><<<nb, EW_THREADS, 0, s>>>(state, dxs, segs, nsegs, part);
+    });
+    fold_batch_kernel<<<order, 256, 0, s>>>(part, nb, order, dots);
     COUNT_LAUNCH();
     COUNT_LAUNCH();
 }
@@ -2075,7 +2273,9 @@ void diis_store_segment(const int* state, const double* const* xs, const double*
 void lincomb_segment(double* out, int64_t len, const double* const* xs, int64_t off, const double* c, int nx,
                      cudaStream_t s) {
     if (len <= 0) return;
-    lincomb_segment_kernel<<<ew_blocks(len), EW_THREADS, 0, s>>>(out, len, xs, off, c, nx);
+    for_vectors(nx, [&](auto N) {
+        lincomb_segment_kernel<decltype(N)::value><<<ew_blocks((len + 1) / 2), EW_THREADS, 0, s>>>(out, len, xs, off, c);
+    });
     COUNT_LAUNCH();
 }
 

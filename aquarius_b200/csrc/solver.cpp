@@ -346,6 +346,7 @@ kern::WeightArgs Solver::weight_args(const Tensor& T, int cs, const Block& b) co
         w.len[p] = b.len[p];
         w.d[p] = den[sp][s] + ctx.spaces.off[sp][s][b.irrep[p]];
     }
+    kern::weight_plan(w);
     return w;
 }
 
@@ -402,17 +403,18 @@ void Solver::build_tau_blocks() {
                     a.t1bi = t1.data + y->offset;
                 }
             }
+            kern::tau_plan(a);
             tau_blocks.push_back(a);
         }
     }
-    // descriptors of the one-launch form
+    // the launch's descriptors
     std::vector<int64_t> cs;
     tau_chunks = 0;
     for (auto& a : tau_blocks) {
         cs.push_back(tau_chunks);
         tau_chunks += (a.len[0] * a.len[1] * a.len[2] * a.len[3] + kern::kBatchChunk - 1) / kern::kBatchChunk;
     }
-    if (tau_blocks.size() > 1) {
+    if (!tau_blocks.empty()) {
         d_tau = (kern::TauArgs*)alloc(tau_blocks.size() * sizeof(kern::TauArgs));
         d_tau_cs = (int64_t*)alloc(cs.size() * sizeof(int64_t));
         ctx.stage_h2d(d_tau, tau_blocks.data(), tau_blocks.size() * sizeof(kern::TauArgs));
@@ -421,9 +423,7 @@ void Solver::build_tau_blocks() {
 }
 
 void Solver::launch_tau() {
-    if (d_tau) kern::tau_batched(d_tau, d_tau_cs, (int)tau_blocks.size(), tau_chunks, ctx.stream);
-    else
-        for (auto& a : tau_blocks) kern::tau_block(a, ctx.stream);
+    kern::tau_batched(d_tau, d_tau_cs, (int)tau_blocks.size(), tau_chunks, ctx.stream);
 }
 
 // Z.weight(D); T += Z; conv = Z.norm(00) over every block of Z1 and Z2, one launch
@@ -927,8 +927,10 @@ void Solver::build_diis() {
     d_e = (double*)alloc((n + 1) * (n + 1) * sizeof(double));
     d_c = (double*)alloc((n + 1) * sizeof(double));
     d_dots = (double*)alloc(n * sizeof(double));
+    d_segs = (kern::DiisSegment*)alloc(segs.size() * sizeof(kern::DiisSegment));
     d_state = (int*)alloc(8 * sizeof(int));
     if (ctx.host_only) return;
+    ctx.stage_h2d(d_segs, segs.data(), segs.size() * sizeof(kern::DiisSegment));
     for (int i = 0; i < n; i++) {
         CCSD_CUDA(cudaMemsetAsync(xs[i], 0, vec_len * sizeof(double), ctx.stream));
         CCSD_CUDA(cudaMemsetAsync(dxs[i], 0, vec_len * sizeof(double), ctx.stream));
@@ -970,8 +972,7 @@ void Solver::diis_step() {
     // copy x, dx into the head slot (device-side slot index)
     kern::diis_store(d_state, d_xs, d_dxs, t1.data, t1.total, t2.data, t2.total, z1.data, z2.data, s);
     // new error-matrix row: <dx_head, dx_j> for all slots (absent slots are zero vectors)
-    CCSD_CUDA(cudaMemsetAsync(d_dots, 0, n * sizeof(double), s));
-    for (auto& sg : segs) kern::diis_dots(d_state, d_dxs, n, sg.off, sg.len, sg.w, d_dots, s);
+    kern::diis_dots(d_state, d_dxs, n, d_segs, (int)segs.size(), vec_len, d_dots, s);
     // bordered system, solve, coefficients by slot
     kern::diis_solve(d_state, d_e, d_c, d_dots, n, s);
     // x = sum c_j x_j (diis.hpp:205-226).  The reference also extrapolates dx into Z; every

@@ -11,11 +11,6 @@ void options_default(ccsd_options* o);
 // the slice autotuner's rule: 1 for the statements that take one slice fewer
 std::vector<int> slice_choice(const std::vector<double>& dE, double budget);
 
-struct DiisSegment {
-    int64_t off, len;
-    double w;
-};
-
 class Solver {
 public:
     Context& ctx;
@@ -52,7 +47,8 @@ public:
     double *d_e = nullptr, *d_c = nullptr, *d_dots = nullptr;
     int* d_state = nullptr;
     int64_t vec_len = 0;
-    std::vector<DiisSegment> segs;
+    std::vector<kern::DiisSegment> segs;
+    kern::DiisSegment* d_segs = nullptr;
     // graph
     cudaGraph_t graph = nullptr;
     cudaGraphExec_t graph_exec = nullptr;
