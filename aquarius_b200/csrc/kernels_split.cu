@@ -15,9 +15,10 @@
 //   s1*s2 + s2*s1 apart, exact over 512 k).
 //
 // INT8 slices (3, 4 or 5):  x = (max/127) * (q1 + q2/254 + q3/254^2 ...),  q_t in [-127,127],
-//   the whole signed 8-bit range: y = x * 127/max lies in [-127,127]; q1 = rint(y) and each
-//   further slice is rint of the remainder (in [-1/2,1/2]) times 254, so every slice
-//   carries log2(254) = 7.99 bits.  The tcgen05 GEMM (kind::i8, twice the BF16 rate)
+//   the whole signed 8-bit range: y = x * 127/max lies in [-127,127] and is rounded to a
+//   multiple of 254^-(NS-1), whose digits of base 254 (offset by 127) are the slices, so every
+//   slice carries log2(254) = 7.99 bits and the first ns slices are an ns-slice slicing (the
+//   rest is within half a unit of the last one).  The tcgen05 GEMM (kind::i8, twice the BF16 rate)
 //   accumulates every level t = i+j of the kept products q_i*q_j (i+j < NS) in its own
 //   INT32 accumulator, which is exact (|q_i q_j| <= 127^2 < 2^14, at most 5 products per
 //   level: a drained chunk of 16384 k stays below 2^31); the epilogue weights level t by
@@ -495,6 +496,21 @@ __device__ __forceinline__ int64_t next_tile(unsigned long long* ctr, int64_t* s
     return *s_next;
 }
 
+// Maxima over the warp of eight values per lane: lanes halve the values they still hold with
+// each exchange (nine exchanges, not eight reductions of five); lanes 4 i .. 4 i + 3 get value i's.
+__device__ __forceinline__ double row_max8(const double (&v)[SPER], int lane) {
+    static_assert(SPER == 8, "eight rows per warp");
+    double a[4], b[2];
+    const bool h = lane & 16, g = lane & 8, f = lane & 4;
+#pragma unroll
+    for (int i = 0; i < 4; i++) a[i] = fmax(h ? v[i + 4] : v[i], __shfl_xor_sync(0xffffffffu, h ? v[i] : v[i + 4], 16));
+#pragma unroll
+    for (int i = 0; i < 2; i++) b[i] = fmax(g ? a[i + 2] : a[i], __shfl_xor_sync(0xffffffffu, g ? a[i] : a[i + 2], 8));
+    double m = fmax(f ? b[1] : b[0], __shfl_xor_sync(0xffffffffu, f ? b[0] : b[1], 4));
+    m = fmax(m, __shfl_xor_sync(0xffffffffu, m, 2));
+    return fmax(m, __shfl_xor_sync(0xffffffffu, m, 1));
+}
+
 template <bool KC>
 __global__ void __launch_bounds__(STHREADS, 6) rowmax_kernel(const double* __restrict__ X, const int64_t* __restrict__ R,
                                                           const int64_t* __restrict__ Kt, int nrows, int K, int tiles_r,
@@ -521,14 +537,10 @@ __global__ void __launch_bounds__(STHREADS, 6) rowmax_kernel(const double* __res
         const int r0 = (int)(t % tiles_r) * SR;
         if (KC) {
             // element i of a warp: one row (warp / 2 + 4 i), 32 consecutive k
-#pragma unroll
-            for (int i = 0; i < SPER; i++) {
-                double m = v[i];
-                for (int o = 16; o > 0; o >>= 1) m = fmax(m, __shfl_xor_sync(0xffffffffu, m, o));
-                const int row = r0 + (warp >> 1) + 4 * i;
-                if (lane == 0 && row < nrows && m > 0.0)
-                    atomicMax(&rowmax[row], (unsigned long long)__double_as_longlong(m));
-            }
+            const double m = row_max8(v, lane);
+            const int row = r0 + (warp >> 1) + 4 * (lane >> 2);
+            if ((lane & 3) == 0 && row < nrows && m > 0.0)
+                atomicMax(&rowmax[row], (unsigned long long)__double_as_longlong(m));
         } else {
             // every element of a thread sits in row `lane`: fold them, then across the warps
             double m = 0.0;
@@ -546,19 +558,73 @@ __global__ void __launch_bounds__(STHREADS, 6) rowmax_kernel(const double* __res
     }
 }
 
+// A tile of the operand in shared memory: position of k in its row.  Four neighbours in k are
+// 20 apart, so that a thread reads four of them for one packed store and neither the reads
+// (16 lanes on consecutive positions) nor the writes of either orientation (along k, or along
+// the rows, whose pitch is odd) meet on a bank.
+constexpr int SPITCH = 77;
+__device__ __forceinline__ int slice_pos(int k) { return (k & 3) * 20 + (k >> 2); }
+
 __device__ __forceinline__ unsigned short bf16_bits(double v) {
     __nv_bfloat16 b = __float2bfloat16_rn((float)v);
     return *reinterpret_cast<unsigned short*>(&b);
 }
 
+// rint of |t| < 2^31 (0 for a NaN) without a conversion instruction: 1.5 * 2^52 leaves the
+// integer in the low word of the sum
+__device__ __forceinline__ int round_int(double t) {
+    return fabs(t) < 2147483648.0 ? __double2loint(t + 6755399441055744.0) : 0;
+}
+
+// INT8 slices.  127 * 254^3 < 2^31: up to four digits of base 254 are one 32-bit integer, so x
+// is rounded once, to a multiple of 254^-(NS-1), and the digits come from integer divisions by
+// 254 (the running remainder took a double rounding and a conversion per slice, which run at
+// a quarter of the rate of a sum).  Digits are 0..253 (the leading one 0..254) after an
+// offset of 127 each, so every slice lies in [-127, 127].
+//   five slices: two digits of the rounded value, three of its remainder
+template <int NS>
+struct I8Digits {
+    static constexpr int HI = NS == 5 ? 2 : NS, LO = NS - HI;
+    // the factor of a row with 127 / max: 254^(HI-1)
+    static constexpr double SCALE = HI == 2 ? 254.0 : HI == 3 ? 64516.0 : 16387064.0;
+    static constexpr unsigned OFFSET = HI == 2 ? 127u * 255u : HI == 3 ? 127u * 64771u : 127u * 16451835u;
+    __device__ static __forceinline__ void put(double x, double mul, unsigned (&w)[NS], int at) {
+        const double t = x * mul;
+        const int n = round_int(t);
+        unsigned u = (unsigned)n + OFFSET;
+#pragma unroll
+        for (int q = HI - 1; q > 0; q--) {
+            const unsigned r = u / 254u;
+            w[q] |= ((u - r * 254u + 129u) & 255u) << (8 * at);   // - 127 in a byte
+            u = r;
+        }
+        w[0] |= ((u + 129u) & 255u) << (8 * at);
+        if constexpr (LO > 0) {
+            // the remainder, in [-1/2, 1/2], as three digits
+            unsigned v = (unsigned)round_int((t - (double)n) * 16387064.0) + 127u * 64771u;
+#pragma unroll
+            for (int q = NS - 1; q > HI; q--) {
+                const unsigned r = v / 254u;
+                w[q] |= ((v - r * 254u + 129u) & 255u) << (8 * at);
+                v = r;
+            }
+            w[HI] |= ((v + 129u) & 255u) << (8 * at);
+        }
+    }
+};
+
+// HBM bounds the slicing: 8 bytes read and NS (INT8) or 2 NS (BF16) written per element.
+// 4416 x 4416 of gathered amplitudes to four INT8 slices (234 MB): 139 -> 120 us where neighbours in
+// memory are neither in a row nor in k, 90 -> 60 us else, with packed stores and the digits
+// from one rounding; before, a store per byte and eight quarter-rate conversions per element.
 template <bool KC, int NS, bool I8>
 __global__ void __launch_bounds__(STHREADS, 6)
     slice_kernel(const double* __restrict__ X, const int64_t* __restrict__ R, const int64_t* __restrict__ Kt, int nrows,
                  int K, int tiles_r, int64_t ntiles, const unsigned long long* __restrict__ rowmax, int rows_p, int kpad,
                  uint8_t* __restrict__ out_bytes, double* __restrict__ scale, unsigned long long* ctr) {
-    __shared__ double tile[SR][SK + 1];
+    __shared__ double tile[SR][SPITCH];
     __shared__ int64_t sR[2][SR], sK[2][SK];
-    __shared__ double sMul[SR];      // per row: 127 / max (INT8) or 2^(6 - e) (BF16); 0 for a zero row
+    __shared__ double sMul[SR];      // per row: 127 / max in units of the last digit (INT8) or 2^(6 - e) (BF16); 0 for a zero row
     __shared__ int64_t s_next;
     const size_t plane = (size_t)rows_p * kpad;
     int b = 0;
@@ -581,7 +647,7 @@ __global__ void __launch_bounds__(STHREADS, 6)
             double mul = 0.0, sc = 0.0;
             if (mx > 1e-290) {   // below that a row counts as zero (127 / max would overflow)
                 if constexpr (I8) {
-                    mul = 127.0 / mx;
+                    mul = 127.0 / mx * I8Digits<NS>::SCALE;
                     sc = mx / 127.0;
                 } else {
                     mul = ldexp(1.0, 6 - ilogb(mx));          // mx in [2^e, 2^(e+1))
@@ -597,44 +663,45 @@ __global__ void __launch_bounds__(STHREADS, 6)
         for (int i = 0; i < SPER; i++) {
             int r, k;
             slice_rk<KC>(i, r, k);
-            tile[r][k] = v[i];
+            tile[r][slice_pos(k)] = v[i];
         }
         __syncthreads();
         // BF16: x = 2^(e-6) (s1 + s2 + ...), s1 in [-128,128], slice t carries weight 2^-8t
         // INT8: x = (max/127) (q1 + q2/254 + ...), q_t in [-127,127]
 #pragma unroll
-        for (int i = 0; i < SPER; i++) {
+        for (int i = 0; i < SPER / 4; i++) {
             const int e = threadIdx.x + i * STHREADS;
-            const int k = e % SK, r = e / SK;
+            const int kq = e % (SK / 4), r = e / (SK / 4);    // four neighbours from 4 kq
             const int row = r0 + r;
             const double mul = sMul[r];
-            uint16_t bits[NS];
+            const size_t o = (size_t)row * kpad + (size_t)(k0 + 4 * kq);
+            if constexpr (I8) {
+                unsigned w[NS];
 #pragma unroll
-            for (int q = 0; q < NS; q++) bits[q] = 0;
-            if (mul > 0.0) {
-                double y = tile[r][k] * mul;                 // |y| <= 127 (INT8), < 2^7 + 1 (BF16)
-                double w = 1.0;                              // BF16 weight of slice q: 2^(-8q)
+                for (int q = 0; q < NS; q++) w[q] = 0;
 #pragma unroll
-                for (int q = 0; q < NS; q++) {
-                    const double st = rint(y);               // an integer of at most 8 significant bits
-                    if constexpr (I8) {
-                        bits[q] = (uint16_t)(uint8_t)(int8_t)(int)st;
-                        y = (y - st) * 254.0;                // remainder in [-1/2, 1/2] -> [-127, 127]
-                    } else {
-                        bits[q] = bf16_bits(st * w);
+                for (int j = 0; j < 4; j++) I8Digits<NS>::put(tile[r][j * 20 + kq], mul, w, j);
+#pragma unroll
+                for (int q = 0; q < NS; q++) *reinterpret_cast<unsigned*>(out_bytes + q * plane + o) = w[q];
+            } else {
+                uint16_t bits[NS][4];
+#pragma unroll
+                for (int j = 0; j < 4; j++) {
+                    double y = tile[r][j * 20 + kq] * mul;       // |y| < 2^7 + 1
+                    double w = 1.0;                              // weight of slice q: 2^(-8q)
+#pragma unroll
+                    for (int q = 0; q < NS; q++) {
+                        const double st = rint(y);               // an integer of at most 8 significant bits
+                        bits[q][j] = mul > 0.0 ? bf16_bits(st * w) : 0;
                         y = (y - st) * 256.0;
                         w *= 0.00390625;
                     }
                 }
-            }
-            const size_t o = (size_t)row * kpad + (size_t)(k0 + k);
-            if constexpr (I8) {
-#pragma unroll
-                for (int q = 0; q < NS; q++) out_bytes[q * plane + o] = (uint8_t)bits[q];
-            } else {
                 uint16_t* out = reinterpret_cast<uint16_t*>(out_bytes);
 #pragma unroll
-                for (int q = 0; q < NS; q++) out[q * plane + o] = bits[q];
+                for (int q = 0; q < NS; q++)
+                    *reinterpret_cast<uint2*>(out + q * plane + o) =
+                        make_uint2(bits[q][0] | (unsigned)bits[q][1] << 16, bits[q][2] | (unsigned)bits[q][3] << 16);
             }
         }
         __syncthreads();   // the tile, sMul and the next tables
@@ -913,13 +980,11 @@ __global__ void __launch_bounds__(split::STHREADS) rect_rowmax_kernel(const Rect
         const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
         if (d.kc) {
 #pragma unroll
-            for (int i = 0; i < SPER; i++) {
-                double m = fabs(v[i]);
-                for (int o = 16; o > 0; o >>= 1) m = fmax(m, __shfl_xor_sync(0xffffffffu, m, o));
-                const int r = (warp >> 1) + 4 * i;
-                if (lane == 0 && r0 + r < d.nrows && m > 0.0)
-                    atomicMax(&rm[d.row0 + r0 + r], (unsigned long long)__double_as_longlong(m));
-            }
+            for (int i = 0; i < SPER; i++) v[i] = fabs(v[i]);
+            const double m = row_max8(v, lane);
+            const int r = (warp >> 1) + 4 * (lane >> 2);
+            if ((lane & 3) == 0 && r0 + r < d.nrows && m > 0.0)
+                atomicMax(&rm[d.row0 + r0 + r], (unsigned long long)__double_as_longlong(m));
         } else {
             double m = 0.0;
 #pragma unroll
@@ -943,7 +1008,7 @@ __global__ void __launch_bounds__(split::STHREADS) rect_slice_kernel(const RectD
                                                                      int rows_p0, int kpad0, uint8_t* out0,
                                                                      double* scale0) {
     using namespace split;
-    __shared__ double tile[SR][SK + 1];
+    __shared__ double tile[SR][SPITCH];
     __shared__ int64_t sR[SR], sK[SK];
     __shared__ double sMul[SR];
     __shared__ int sp;
@@ -966,30 +1031,40 @@ __global__ void __launch_bounds__(split::STHREADS) rect_slice_kernel(const RectD
             const bool in = r0 + (int)threadIdx.x < d.nrows;
             const double mx = in ? __longlong_as_double((long long)rowmax[row]) : 0.0;
             const bool nz = mx > 1e-290;
-            sMul[threadIdx.x] = nz ? 127.0 / mx : 0.0;
+            sMul[threadIdx.x] = nz ? 127.0 / mx * I8Digits<NS>::SCALE : 0.0;
             if (in && d.k0 == 0 && k0 == 0) scale[row] = nz ? mx / 127.0 : 0.0;   // the row's first rectangle
         }
 #pragma unroll
         for (int i = 0; i < SPER; i++) {
             const int e = threadIdx.x + i * STHREADS;
             const int r = d.kc ? e / SK : e % SR, k = d.kc ? e % SK : e / SR;
-            tile[r][k] = v[i];
+            tile[r][slice_pos(k)] = v[i];
         }
         __syncthreads();
         const size_t plane = (size_t)rows_p * kpad;
-#pragma unroll
-        for (int i = 0; i < SPER; i++) {
-            const int e = threadIdx.x + i * STHREADS;
-            const int k = e % SK, r = e / SK;
-            if (r0 + r >= d.nrows || k0 + k >= d.nk) continue;
+        // four neighbours of the merged operand per store; a rectangle may start at any k, so its
+        // words start up to three elements before it and the outer ones are stored by byte
+        const int lead = d.k0 & 3, words = lead ? SK / 4 + 1 : SK / 4;
+        const int rows = min(SR, d.nrows - r0), kn = min(SK, d.nk - k0);
+        for (int e = threadIdx.x; e < rows * words; e += STHREADS) {
+            const int r = e / words, kb = 4 * (e % words) - lead;
+            if (kb >= kn) continue;
             const double mul = sMul[r];
-            const size_t o = (size_t)(d.row0 + r0 + r) * kpad + (size_t)(d.k0 + k0 + k);
-            double y = tile[r][k] * mul;
+            unsigned w[NS];
 #pragma unroll
-            for (int q = 0; q < NS; q++) {
-                const double st = mul > 0.0 ? rint(y) : 0.0;
-                out[q * plane + o] = (uint8_t)(int8_t)(int)st;
-                y = (y - st) * 254.0;
+            for (int q = 0; q < NS; q++) w[q] = 0;
+#pragma unroll
+            for (int j = 0; j < 4; j++)
+                if (kb + j >= 0 && kb + j < kn) I8Digits<NS>::put(tile[r][slice_pos(kb + j)], mul, w, j);
+            uint8_t* o = out + (size_t)(d.row0 + r0 + r) * kpad + (size_t)(d.k0 + k0) + kb;
+            if (kb >= 0 && kb + 4 <= kn) {
+#pragma unroll
+                for (int q = 0; q < NS; q++) *reinterpret_cast<unsigned*>(o + q * plane) = w[q];
+            } else {
+#pragma unroll
+                for (int q = 0; q < NS; q++)
+                    for (int j = 0; j < 4; j++)
+                        if (kb + j >= 0 && kb + j < kn) o[q * plane + j] = (uint8_t)(w[q] >> (8 * j));
             }
         }
         __syncthreads();   // the tile, the tables and the row factors are reused by the next tile

@@ -613,7 +613,7 @@ void Context::run_merged(Plan& p, MergedProduct& m, const std::string& label) {
                 c = alloc_sliced(rows, m.K, ns, kind);
                 phase("slice-cached", [&] { kern::rect_slice(d, ts, n, tiles, ns, c, stream); });
             }
-            // the first ns slices of a deeper slicing are the ns-slice slicing
+            // the first ns slices of a deeper slicing are an ns-slice slicing
             kern::SlicedOperand v = c;
             v.nslices = ns;
             return v;

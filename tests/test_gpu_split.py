@@ -104,3 +104,19 @@ def test_refinement_moves_to_four_slices_and_converges(precision):
         assert c < 1e-10
         assert abs(e - e_ref) < 1e-10, (e, e_ref)
         s.close()
+
+
+@pytest.mark.parametrize("slices", [3, 4, 5])
+@pytest.mark.parametrize("o,v", [(3, 11), (5, 27), (7, 34)], ids=lambda x: str(x))
+def test_int8_slices_at_odd_extents(o, v, slices):
+    """Rows and k that end inside a packed group of four, both orientations of the gather.  An
+    operand is off by at most half a unit of its last slice (max / 127 / 254^(n-1) / 2), and the
+    products left out (levels of n slices and more, n - 1 of them at the first) by at most
+    127^2 254^-n each in units of (max / 127)^2."""
+    K = max(o * v, v * v) * 4
+    for sa, ia, sb, ib, sc, ic in (("amei", "amei", "abij", "ebjm", "abij", "abij"),
+                                   ("amef", "amef", "abij", "efij", "amij", "amij")):
+        ref = _contract("fp64", o, v, ia, sa, ib, sb, ic, sc, 5, False)
+        got = _contract("split_i8", o, v, ia, sa, ib, sb, ic, sc, 5, False, slices=slices)
+        bound = K * 0.05 * 6 * 0.01 * 6 * (254.0 ** (1 - slices) / 127 + 2 * slices * 254.0 ** -slices)
+        assert np.abs(got - ref).max() <= bound, (sa, np.abs(got - ref).max(), bound)
