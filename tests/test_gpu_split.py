@@ -106,6 +106,9 @@ def test_refinement_moves_to_four_slices_and_converges(precision):
         s.close()
 
 
+SHAPES.update(amef=((1, 1), (2, 0)), amij=((1, 1), (0, 2)))
+
+
 @pytest.mark.parametrize("slices", [3, 4, 5])
 @pytest.mark.parametrize("o,v", [(3, 11), (5, 27), (7, 34)], ids=lambda x: str(x))
 def test_int8_slices_at_odd_extents(o, v, slices):
