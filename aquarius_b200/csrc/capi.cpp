@@ -382,8 +382,8 @@ int ccsd_tensor_read_block(ccsd_ctx ctx, ccsd_tensor t, const int alpha[4], cons
         Tensor& T = c->tensor(t);
         int cs;
         const Block& b = block_at(T, alpha, irreps, cs);
-        CCSD_CUDA(cudaStreamSynchronize(c->stream));
         if (T.view_of) {
+            CCSD_CUDA(cudaStreamSynchronize(c->stream));   // the copy below is not on the stream
             std::vector<int64_t> ord = block_order(b);
             std::vector<double> buf(b.size);
             CCSD_CUDA(cudaMemcpy(buf.data(), T.data + b.offset, b.size * sizeof(double), cudaMemcpyDeviceToHost));

@@ -359,7 +359,10 @@ void Context::collect_profile() {
 }
 
 void Context::upload(Plan& p) {
-    bool any = false;
+    // a plan's steps do not change once it runs: a statement of thousands of block products
+    // (0.5 ms to walk, D2h o=16 v=96) is looked through once, not on every call
+    const bool reserve = split_precision() && !p.split_reserved && (host_only || kern::split_supported());
+    if (p.tables_ready && !reserve) return;
     if (p.scratch_elems > 0 && !p.scratch) p.scratch = (double*)dmalloc(p.scratch_elems * sizeof(double));
     // split-K workspace of the FP64 GEMM, grown before any capture
     int64_t need = 0;
@@ -423,7 +426,6 @@ void Context::upload(Plan& p) {
     for (auto& g : p.gemms) {
         if (g.uploaded) continue;
         g.uploaded = true;
-        any = true;
         // k tables that are arithmetic progressions let the kernels compute the offsets
         auto affine = [](const std::vector<int64_t>& t, int64_t& b0, int64_t& st) {
             if (t.empty()) return false;
@@ -438,14 +440,15 @@ void Context::upload(Plan& p) {
     }
     // tables are uploaded from pageable host memory; make sure the copies have been
     // staged before the host vectors could change
-    if (split_precision() && !p.split_reserved && (host_only || kern::split_supported())) {
+    if (reserve) {
         reserve_split(p);
         p.split_reserved = true;
     }
-    (void)any;   // staged copies need no synchronisation (the host tables stay with the plan)
+    p.tables_ready = true;
 }
 
 void Context::release(Plan& p) {
+    p.tables_ready = false;
     if (p.scratch) dfree(p.scratch, p.scratch_elems * sizeof(double));
     p.scratch = nullptr;
     for (auto& t : p.table_pool) dfree(t.first, t.second);

@@ -260,6 +260,7 @@ struct Plan {
     int64_t scratch_elems = 0;         // doubles of scratch the steps need (products X)
     double* scratch = nullptr;         // allocated at upload
     bool split_reserved = false;       // split-path workspace sized for this plan
+    bool tables_ready = false;         // tables, scratch and workspaces of every step are in place
     std::vector<std::pair<void*, size_t>> table_pool;   // device buffers holding the steps' tables
     std::vector<Step> steps;
     std::vector<GemmStep> gemms;

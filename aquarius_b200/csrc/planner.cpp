@@ -49,6 +49,7 @@ void Plan::append(Plan&& o) {
     for (auto& g : o.scales) scales.push_back(g);
     for (auto& g : o.dots) dots.push_back(g);
     scratch_elems = std::max(scratch_elems, o.scratch_elems);
+    tables_ready = false;
 }
 
 namespace {
