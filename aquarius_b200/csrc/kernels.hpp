@@ -202,8 +202,6 @@ void gemm_split(const SlicedOperand& a, const SlicedOperand& b, int M, int N, in
 // K-ranges for a split GEMM: enough CTAs for about two waves when the output has few
 // tiles (1 = none)
 int split_ksplit(int M, int N, int K, int nslices = 3, int kind = SLICE_BF16);
-// alpha * sum_z ws[z][m][n] scattered into every destination variant of g (fixed order)
-void splitk_fold(const GemmArgs& g, int ks, cudaStream_t s);
 
 // Merged products of a symmetry-blocked statement: the block products of one irrep class
 // form one dense GEMM.  Its operands are rectangles (a block product's rows x its k range)
@@ -243,8 +241,13 @@ struct ScatterDesc {
     double alpha = 0;
     int nrows = 0, ncols = 0, row0 = 0, col0 = 0;
 };
-// C += alpha * sum_z ws[z] over each rectangle (chunks of kBatchChunk elements)
-void rect_scatter(const ScatterDesc* d, const int64_t* chunk_start, int n, int64_t chunks, const double* ws, int ldn,
+// C += alpha * sum_z ws[z] over each rectangle (ws: [column][row], ldm rows; chunks of 64 rows x
+// 32 columns)
+constexpr int kScatterRows = 64, kScatterCols = 32;
+inline int64_t scatter_chunks(int nrows, int ncols) {
+    return (int64_t)((nrows + kScatterRows - 1) / kScatterRows) * ((ncols + kScatterCols - 1) / kScatterCols);
+}
+void rect_scatter(const ScatterDesc* d, const int64_t* chunk_start, int n, int64_t chunks, const double* ws, int ldm,
                   int64_t zstride, int ks, cudaStream_t s);
 bool split_supported();
 // nonzero if a split-GEMM wait expired (1..4 = which wait); reset clears it

@@ -911,14 +911,6 @@ void gemm_fp64(const GemmArgs& g, cudaStream_t s) {
     }
 }
 
-void splitk_fold(const GemmArgs& g, int ks, cudaStream_t s) {
-    const int64_t mn = (int64_t)g.M * g.N;
-    if (mn <= 0 || ks <= 1) return;
-    const int nb = (int)std::min<int64_t>((mn + 255) / 256, 148 * 16);
-    splitk_fold_kernel<<<nb, 256, 0, s>>>(g, ks);
-    COUNT_LAUNCH();
-}
-
 int fp64_tile_rows(int M, int N) {
     // 64 unless 32 x 32 tiles cover the product with at most three fifths of the area
     auto area = [&](int64_t r) { return ((M + r - 1) / r) * ((N + r - 1) / r) * r * r; };

@@ -119,11 +119,11 @@ struct Params {
     double vsign[4];
     int* err;
     // split-K over gridDim.y: K-block range blockIdx.y of ks, partials (scales applied,
-    // alpha not) to ws[z][m][n], folded into C by the FP64 fold kernel
+    // alpha not) to ws[z][n][m], folded into C by split_fold_kernel
     int ks;
     int kb_per;                    // K blocks per range (a multiple of the exact chunk)
     double* ws;
-    int dense;                     // write ws[z][m][n] even without split-K (merged products)
+    int dense;                     // write ws[z][n][m] even without split-K (merged products)
 };
 
 __device__ __forceinline__ uint32_t smem_u32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
@@ -392,11 +392,12 @@ __global__ void __launch_bounds__(THREADS, 1)
             const int m = m0 + q * 32 + lane;
             if (m < p.M) {
                 const double sa = p.scaleA[m];
-                double* wz = p.ws + ((int64_t)blockIdx.y * p.M + m) * p.N;
+                // [n][m]: the lanes of a warp write 32 consecutive rows
+                double* wz = p.ws + (int64_t)blockIdx.y * p.M * p.N + m;
 #pragma unroll
                 for (int j = 0; j < COLS; j++) {
                     const int n = n0 + h * COLS + j;
-                    if (n < p.N) wz[n] = sa * p.scaleB[n] * acc[j];
+                    if (n < p.N) wz[(int64_t)n * p.M] = sa * p.scaleB[n] * acc[j];
                 }
             }
         } else if (ok && p.nvm == 1 && p.nvn == 1) {
@@ -819,6 +820,90 @@ void slice_rows(const double* X, const int64_t* R, const int64_t* Kt, int nrows,
     g_launches += 2;
 }
 
+// ---------------------------------------------------------------------------
+// dense products into C
+// ---------------------------------------------------------------------------
+namespace {
+
+// the problem that chunk c belongs to; called by one warp, 32 first chunks probed at a time
+__device__ __forceinline__ int find_chunk(const int64_t* __restrict__ cs, int n, int64_t c) {
+    int lo = 0, m = n;
+    while (m > 1) {
+        const int step = (m + 31) >> 5, i = lo + (int)(threadIdx.x & 31) * step;
+        const unsigned below = __ballot_sync(0xffffffffu, i < lo + m && cs[min(i, n - 1)] <= c);
+        const int hit = __popc(below) - 1;
+        m = min(step, m - hit * step);
+        lo += hit * step;
+    }
+    return lo;
+}
+
+// C[Cm_a[m] + Cn_b[n]] += vsign_ab * alpha * sum_z ws[z][col0 + n][row0 + m] for one tile of 64 rows x
+// 32 columns of a rectangle.  HBM and L2 bound it: the product is read along its rows; where
+// the columns of C are the contiguous ones (and the rows are not) the tile is turned in shared
+// memory, so that C is read and written in whole sectors either way.
+// D2h o=24 v=180: the 600 scatters of four iterations 12.1 -> 7.1 ms; a lane wrote a sector of its own
+// before, in the product and in C.
+__device__ __forceinline__ void scatter_tile(const ScatterDesc& d, int64_t chunk, const double* __restrict__ ws, int ldm,
+                                             int64_t zstride, int ks) {
+    constexpr int PER = kScatterRows * kScatterCols / 256;
+    __shared__ double tile[kScatterCols][kScatterRows + 1];
+    const int tiles_r = (d.nrows + kScatterRows - 1) / kScatterRows;
+    const int r0 = (int)(chunk % tiles_r) * kScatterRows, c0 = (int)(chunk / tiles_r) * kScatterCols;
+    const int64_t *Cm = d.Cm[0], *Cn = d.Cn[0];
+    const bool turn = d.ncols > 1 && __ldg(Cn + 1) - __ldg(Cn) == 1 && (d.nrows == 1 || __ldg(Cm + 1) - __ldg(Cm) != 1);
+    double v[PER];
+#pragma unroll
+    for (int q = 0; q < PER; q++) {
+        const int e = threadIdx.x + 256 * q, m = r0 + e % kScatterRows, c = c0 + e / kScatterRows;
+        v[q] = m < d.nrows && c < d.ncols ? __ldg(ws + (int64_t)(d.col0 + c) * ldm + d.row0 + m) : 0.0;
+    }
+    for (int z = 1; z < ks; z++)
+#pragma unroll
+        for (int q = 0; q < PER; q++) {
+            const int e = threadIdx.x + 256 * q, m = r0 + e % kScatterRows, c = c0 + e / kScatterRows;
+            if (m < d.nrows && c < d.ncols) v[q] += __ldg(ws + z * zstride + (int64_t)(d.col0 + c) * ldm + d.row0 + m);
+        }
+    if (turn) {
+#pragma unroll
+        for (int q = 0; q < PER; q++) {
+            const int e = threadIdx.x + 256 * q;
+            tile[e / kScatterRows][e % kScatterRows] = v[q];
+        }
+        __syncthreads();
+#pragma unroll
+        for (int q = 0; q < PER; q++) {
+            const int e = threadIdx.x + 256 * q;
+            v[q] = tile[e % kScatterCols][e / kScatterCols];
+        }
+    }
+    for (int a = 0; a < d.nvm; a++)
+        for (int b = 0; b < d.nvn; b++) {
+            const double f = d.alpha * d.vsign[a * d.nvn + b];
+            int64_t off[PER];
+            double old[PER];
+#pragma unroll
+            for (int q = 0; q < PER; q++) {
+                const int e = threadIdx.x + 256 * q;
+                const int m = r0 + (turn ? e / kScatterCols : e % kScatterRows);
+                const int c = c0 + (turn ? e % kScatterCols : e / kScatterRows);
+                off[q] = m < d.nrows && c < d.ncols ? __ldg(d.Cm[a] + m) + __ldg(d.Cn[b] + c) : -1;
+            }
+#pragma unroll
+            for (int q = 0; q < PER; q++) old[q] = off[q] >= 0 ? d.C[off[q]] : 0.0;
+#pragma unroll
+            for (int q = 0; q < PER; q++)
+                if (off[q] >= 0) d.C[off[q]] = old[q] + f * v[q];
+        }
+}
+
+__global__ void __launch_bounds__(256) split_fold_kernel(ScatterDesc d, const double* __restrict__ ws, int ldm,
+                                                         int64_t zstride, int ks) {
+    scatter_tile(d, blockIdx.x, ws, ldm, zstride, ks);
+}
+
+}  // namespace
+
 namespace {
 struct SchemeInfo {
     int tbn, bke, kbb, chunk, grain;
@@ -912,7 +997,22 @@ void gemm_split(const SlicedOperand& a, const SlicedOperand& b, int M, int N, in
         else split_gemm_kernel<4, false><<<grid, THREADS, si.smem, s>>>(ma, mb, p);
     }
     g_launches++;
-    if (ks > 1 && !g.dense_out) splitk_fold(g, ks, s);
+    if (ks > 1 && !g.dense_out) {
+        ScatterDesc d;
+        d.C = g.C;
+        for (int v = 0; v < 2; v++) {
+            d.Cm[v] = g.Cm[v];
+            d.Cn[v] = g.Cn[v];
+        }
+        d.nvm = g.nvm;
+        d.nvn = g.nvn;
+        for (int i = 0; i < 4; i++) d.vsign[i] = g.vsign[i];
+        d.alpha = g.alpha;
+        d.nrows = M;
+        d.ncols = N;
+        split_fold_kernel<<<(unsigned)scatter_chunks(M, N), 256, 0, s>>>(d, g.ws, M, (int64_t)M * N, ks);
+        g_launches++;
+    }
 }
 
 // ---------------------------------------------------------------------------
@@ -1071,29 +1171,17 @@ __global__ void __launch_bounds__(split::STHREADS) rect_slice_kernel(const RectD
     }
 }
 
-// C[Cm_a[m] + Cn_b[n]] += vsign_ab * alpha * sum_z ws[z][row0 + m][col0 + n] for one
-// rectangle's chunk of kBatchChunk elements per CTA
 __global__ void __launch_bounds__(256) rect_scatter_kernel(const ScatterDesc* __restrict__ sd,
                                                            const int64_t* __restrict__ cs, int n,
-                                                           const double* __restrict__ ws, int ldn, int64_t zstride,
+                                                           const double* __restrict__ ws, int ldm, int64_t zstride,
                                                            int ks) {
     __shared__ int sp;
-    if (threadIdx.x == 0) sp = find_rect(cs, n, blockIdx.x);
-    __syncthreads();
-    const ScatterDesc& d = sd[sp];
-    const int64_t base = (blockIdx.x - cs[sp]) * (int64_t)kBatchChunk;
-    const int64_t total = (int64_t)d.nrows * d.ncols;
-    for (int i = threadIdx.x; i < kBatchChunk; i += blockDim.x) {
-        const int64_t l = base + i;
-        if (l >= total) break;
-        const int m = (int)(l / d.ncols), c = (int)(l % d.ncols);
-        const int64_t w = (int64_t)(d.row0 + m) * ldn + d.col0 + c;
-        double v = 0.0;
-        for (int z = 0; z < ks; z++) v += ws[z * zstride + w];
-        v *= d.alpha;
-        for (int a = 0; a < d.nvm; a++)
-            for (int b = 0; b < d.nvn; b++) d.C[d.Cm[a][m] + d.Cn[b][c]] += d.vsign[a * d.nvn + b] * v;
+    if (threadIdx.x < 32) {
+        const int p = find_chunk(cs, n, blockIdx.x);
+        if (threadIdx.x == 0) sp = p;
     }
+    __syncthreads();
+    scatter_tile(sd[sp], blockIdx.x - cs[sp], ws, ldm, zstride, ks);
 }
 
 }  // namespace
@@ -1128,10 +1216,10 @@ void rect_slice_batched(const RectDesc* d, const int64_t* tile_start, int n, int
     g_launches += 2;
 }
 
-void rect_scatter(const ScatterDesc* d, const int64_t* chunk_start, int n, int64_t chunks, const double* ws, int ldn,
+void rect_scatter(const ScatterDesc* d, const int64_t* chunk_start, int n, int64_t chunks, const double* ws, int ldm,
                   int64_t zstride, int ks, cudaStream_t s) {
     if (n <= 0 || chunks <= 0) return;
-    rect_scatter_kernel<<<(unsigned)chunks, 256, 0, s>>>(d, chunk_start, n, ws, ldn, zstride, ks);
+    rect_scatter_kernel<<<(unsigned)chunks, 256, 0, s>>>(d, chunk_start, n, ws, ldm, zstride, ks);
     g_launches++;
 }
 

@@ -402,7 +402,7 @@ void Context::build_merged(Plan& p, GemmRun& run, int first, int end, std::vecto
             std::vector<int64_t> cs;
             for (auto& s : l) {
                 cs.push_back(L.chunks);
-                L.chunks += ((int64_t)s.nrows * s.ncols + kern::kBatchChunk - 1) / kern::kBatchChunk;
+                L.chunks += kern::scatter_chunks(s.nrows, s.ncols);
             }
             L.n = (int)l.size();
             L.d = (kern::ScatterDesc*)dmalloc(l.size() * sizeof(kern::ScatterDesc));
@@ -639,7 +639,7 @@ void Context::run_merged(Plan& p, MergedProduct& m, const std::string& label) {
     phase("gemm", [&] { kern::gemm_split(va, vb, m.M, m.N, m.K, a, stream, ks); });
     phase("scatter", [&] {
         for (auto& L : m.levels)
-            kern::rect_scatter(L.d, L.cs, L.n, L.chunks, merged_ws, m.N, (int64_t)m.M * m.N, ks, stream);
+            kern::rect_scatter(L.d, L.cs, L.n, L.chunks, merged_ws, m.M, (int64_t)m.M * m.N, ks, stream);
     });
 }
 
