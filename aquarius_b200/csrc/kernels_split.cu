@@ -25,7 +25,7 @@
 //   254^-t in FP64.  Per product the error is ~254^-NS / 2 of row max x column max
 //   (3.7e-8, 1.5e-10, 5.7e-13 for 3, 4, 5 slices).
 //
-// Kernel structure (one 128 x TBN output tile per CTA, 320 threads):
+// Kernel structure (one CTA per SM walks 128 x TBN output tiles, 320 threads):
 //   warp 0      TMA producer: NS A-slice + NS B-slice tiles of 128-byte k-blocks per
 //               stage (128-byte swizzle), 2 stages, mbarrier full/empty ring;
 //   warp 1      TMEM allocation and the single-thread MMA issuer: one MMA per kept slice
@@ -33,7 +33,11 @@
 //               finished chunk;
 //   warps 2..9  epilogue: TMEM accumulator sets (double-buffered where two fit) are
 //               drained per chunk into FP64 registers; the scaled result is scattered
-//               into the destination through the planner's offset tables at the end.
+//               into the destination through the planner's offset tables while the next
+//               tile's products run (the accumulators are free once they are drained).
+//               A CTA per tile left the pipe idle from the drain to the next CTA's first
+//               stage, 10 to 25 us of a 90 us tile at K=4416; D2h o=24 v=180, products of a
+//               few hundred rows: 18.7 -> 16.4 ms of four iterations.
 // Every mbarrier wait is bounded (about 2 s); on expiry the kernel records an error
 // code, stops issuing work and returns after releasing its TMEM.
 #include <algorithm>
@@ -118,7 +122,8 @@ struct Params {
     int nvm, nvn;
     double vsign[4];
     int* err;
-    // split-K over gridDim.y: K-block range blockIdx.y of ks, partials (scales applied,
+    int tiles;                     // output tiles
+    // split-K: K-block range z of ks, partials (scales applied,
     // alpha not) to ws[z][n][m], folded into C by split_fold_kernel
     int ks;
     int kb_per;                    // K blocks per range (a multiple of the exact chunk)
@@ -242,13 +247,16 @@ __global__ void __launch_bounds__(THREADS, 1)
     volatile int* abort_flag = (volatile int*)(tmem_slot + 1);
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int tile = blockIdx.x;
-    const int tm = tile / p.tiles_n, tn = tile % p.tiles_n;
-    const int m0 = tm * BM, n0 = tn * TBN;
-    // this CTA's K blocks [kb0, kb0 + nkb)
-    const int kb0 = blockIdx.y * p.kb_per;
-    const int nkb = max(0, min(p.Kp / Sh::BKE, kb0 + p.kb_per) - kb0);
-    const int nchunks = (nkb + Sh::CHUNK - 1) / Sh::CHUNK;
+    // work item w: tile w % tiles of K range w / tiles; its K blocks are [kb0, kb0 + nkb)
+    const int total = p.tiles * p.ks;
+    auto work = [&](int w, int& m0, int& n0, int& z, int& kb0, int& nkb) {
+        const int tile = w % p.tiles;
+        z = w / p.tiles;
+        m0 = tile / p.tiles_n * BM;
+        n0 = tile % p.tiles_n * TBN;
+        kb0 = z * p.kb_per;
+        nkb = max(0, min(p.Kp / Sh::BKE, kb0 + p.kb_per) - kb0);
+    };
 
     if (threadIdx.x == 0) {
         for (int s = 0; s < STAGES; s++) {
@@ -275,68 +283,85 @@ __global__ void __launch_bounds__(THREADS, 1)
     if (warp == 0) {
         if (lane == 0) {
             // ---------------- TMA producer ----------------
-            for (int kb = 0; kb < nkb && !*abort_flag; kb++) {
-                const int s = kb % STAGES;
-                if (kb >= STAGES && !mbar_wait(&empty[s], ((kb / STAGES) - 1) & 1, abort_flag, p.err, 1)) break;
-                mbar_expect_tx(&full[s], Sh::STAGE);
-                uint8_t* base = stages + (size_t)s * Sh::STAGE;
-                // x = k-block start in elements: a multiple of 128 bytes
-                for (int i = 0; i < NS; i++)
-                    tma_load_2d(base + i * Sh::TILE_A, &tmA, (kb0 + kb) * Sh::BKE, i * p.Mp + m0, &full[s]);
-                for (int i = 0; i < NS; i++)
-                    tma_load_2d(base + NS * Sh::TILE_A + i * Sh::TILE_B, &tmB, (kb0 + kb) * Sh::BKE,
-                                i * p.Np + n0, &full[s]);
+            int it = 0;                  // K blocks of all tiles so far: stage and phase
+            bool ok = true;
+            for (int w = blockIdx.x, m0, n0, z, kb0, nkb; w < total && ok; w += gridDim.x) {
+                work(w, m0, n0, z, kb0, nkb);
+                for (int kb = 0; kb < nkb && !*abort_flag; kb++, it++) {
+                    const int s = it % STAGES;
+                    if (it >= STAGES && !mbar_wait(&empty[s], ((it / STAGES) - 1) & 1, abort_flag, p.err, 1)) {
+                        ok = false;
+                        break;
+                    }
+                    mbar_expect_tx(&full[s], Sh::STAGE);
+                    uint8_t* base = stages + (size_t)s * Sh::STAGE;
+                    // x = k-block start in elements: a multiple of 128 bytes
+                    for (int i = 0; i < NS; i++)
+                        tma_load_2d(base + i * Sh::TILE_A, &tmA, (kb0 + kb) * Sh::BKE, i * p.Mp + m0, &full[s]);
+                    for (int i = 0; i < NS; i++)
+                        tma_load_2d(base + NS * Sh::TILE_A + i * Sh::TILE_B, &tmB, (kb0 + kb) * Sh::BKE,
+                                    i * p.Np + n0, &full[s]);
+                }
+                ok = ok && !*abort_flag;
             }
         }
     } else if (warp == 1) {
         if (lane == 0) {
             // ---------------- MMA issuer ----------------
-            int kb = 0;
-            for (int c = 0; c < nchunks && !*abort_flag; c++) {
-                const int b = c % NBUF;
-                if (c >= NBUF && !mbar_wait(&tempty[b], ((c / NBUF) - 1) & 1, abort_flag, p.err, 2)) break;
-                tc_fence_after();
-                const uint32_t dbase = tmem + b * Sh::BUF;
-                const int kb_end = min(nkb, (c + 1) * Sh::CHUNK);
-                bool first = true;
-                bool ok = true;
-                for (; kb < kb_end; kb++) {
-                    const int s = kb % STAGES;
-                    if (!mbar_wait(&full[s], (kb / STAGES) & 1, abort_flag, p.err, 3)) {
+            int it = 0, cc = 0;          // K blocks and chunks of all tiles so far
+            bool ok = true;
+            for (int w = blockIdx.x, m0, n0, z, kb0, nkb; w < total && ok; w += gridDim.x) {
+                work(w, m0, n0, z, kb0, nkb);
+                int kb = 0;
+                for (int kb_end; kb < nkb && !*abort_flag; cc++) {
+                    const int b = cc % NBUF;
+                    if (cc >= NBUF && !mbar_wait(&tempty[b], ((cc / NBUF) - 1) & 1, abort_flag, p.err, 2)) {
                         ok = false;
                         break;
                     }
                     tc_fence_after();
-                    const uint8_t* base = stages + (size_t)s * Sh::STAGE;
-                    uint64_t ad[NS], bd[NS];
+                    const uint32_t dbase = tmem + b * Sh::BUF;
+                    kb_end = min(nkb, kb + Sh::CHUNK);
+                    bool first = true;
+                    for (; kb < kb_end; kb++, it++) {
+                        const int s = it % STAGES;
+                        if (!mbar_wait(&full[s], (it / STAGES) & 1, abort_flag, p.err, 3)) {
+                            ok = false;
+                            break;
+                        }
+                        tc_fence_after();
+                        const uint8_t* base = stages + (size_t)s * Sh::STAGE;
+                        uint64_t ad[NS], bd[NS];
 #pragma unroll
-                    for (int i = 0; i < NS; i++) {
-                        ad[i] = sdesc<Sh::KBB>(base + i * Sh::TILE_A);
-                        bd[i] = sdesc<Sh::KBB>(base + NS * Sh::TILE_A + i * Sh::TILE_B);
+                        for (int i = 0; i < NS; i++) {
+                            ad[i] = sdesc<Sh::KBB>(base + i * Sh::TILE_A);
+                            bd[i] = sdesc<Sh::KBB>(base + NS * Sh::TILE_A + i * Sh::TILE_B);
+                        }
+#pragma unroll
+                        for (int kk = 0; kk < Sh::KSTEPS; kk++) {
+                            // one MMA covers 32 bytes of K (16 BF16 or 32 INT8 values)
+                            const uint64_t o = (uint64_t)(kk * 32) >> 4;
+                            // slice products (i, t - i) with t < NS into accumulator t (INT8) or
+                            // min(t, NACC - 1) (BF16)
+                            bool fresh[Sh::NACC];
+#pragma unroll
+                            for (int j = 0; j < Sh::NACC; j++) fresh[j] = first;
+#pragma unroll
+                            for (int t = 0; t < NS; t++)
+#pragma unroll
+                                for (int i = 0; i <= t; i++) {
+                                    const int j = t < Sh::NACC - 1 ? t : Sh::NACC - 1;
+                                    umma<I8>(dbase + j * TBN, ad[i] + o, bd[t - i] + o, Sh::IDESC, fresh[j] ? 0u : 1u);
+                                    fresh[j] = false;
+                                }
+                            first = false;
+                        }
+                        umma_commit(&empty[s]);
                     }
-#pragma unroll
-                    for (int kk = 0; kk < Sh::KSTEPS; kk++) {
-                        // one MMA covers 32 bytes of K (16 BF16 or 32 INT8 values)
-                        const uint64_t o = (uint64_t)(kk * 32) >> 4;
-                        // slice products (i, t - i) with t < NS into accumulator t (INT8) or
-                        // min(t, NACC - 1) (BF16)
-                        bool fresh[Sh::NACC];
-#pragma unroll
-                        for (int j = 0; j < Sh::NACC; j++) fresh[j] = first;
-#pragma unroll
-                        for (int t = 0; t < NS; t++)
-#pragma unroll
-                            for (int i = 0; i <= t; i++) {
-                                const int j = t < Sh::NACC - 1 ? t : Sh::NACC - 1;
-                                umma<I8>(dbase + j * TBN, ad[i] + o, bd[t - i] + o, Sh::IDESC, fresh[j] ? 0u : 1u);
-                                fresh[j] = false;
-                            }
-                        first = false;
-                    }
-                    umma_commit(&empty[s]);
+                    if (!ok) break;
+                    umma_commit(&tfull[b]);
                 }
-                if (!ok) break;
-                umma_commit(&tfull[b]);
+                ok = ok && !*abort_flag;
             }
         }
     } else {
@@ -345,104 +370,109 @@ __global__ void __launch_bounds__(THREADS, 1)
         const int q = warp & 3;          // TMEM lane quadrant this warp may access
         const int h = ew >> 2;           // column half
         double acc[COLS];
-#pragma unroll
-        for (int j = 0; j < COLS; j++) acc[j] = 0.0;
         bool ok = true;
-        for (int c = 0; c < nchunks; c++) {
-            const int b = c % NBUF;
-            if (!mbar_wait(&tfull[b], (c / NBUF) & 1, abort_flag, p.err, 4)) {
-                ok = false;
-                break;
-            }
-            tc_fence_after();
-            const uint32_t base = tmem + ((uint32_t)(q * 32) << 16) + b * Sh::BUF + h * COLS;
+        int cc = 0;                      // chunks of all tiles so far
+        for (int w = blockIdx.x, m0, n0, z, kb0, nkb; w < total && ok; w += gridDim.x) {
+            work(w, m0, n0, z, kb0, nkb);
+            const int nchunks = (nkb + Sh::CHUNK - 1) / Sh::CHUNK;
 #pragma unroll
-            for (int j4 = 0; j4 < COLS / 16; j4++) {
-                if constexpr (I8) {
-                    // one level at a time (fewer live registers): level j weighs 254^-j
+            for (int j = 0; j < COLS; j++) acc[j] = 0.0;
+            for (int c = 0; c < nchunks; c++, cc++) {
+                const int b = cc % NBUF;
+                if (!mbar_wait(&tfull[b], (cc / NBUF) & 1, abort_flag, p.err, 4)) {
+                    ok = false;
+                    break;
+                }
+                tc_fence_after();
+                const uint32_t base = tmem + ((uint32_t)(q * 32) << 16) + b * Sh::BUF + h * COLS;
 #pragma unroll
-                    for (int j = 0; j < Sh::NACC; j++) {
-                        uint32_t r[16];
-                        tmem_ld16(base + j * TBN + j4 * 16, r);
+                for (int j4 = 0; j4 < COLS / 16; j4++) {
+                    if constexpr (I8) {
+                        // one level at a time (fewer live registers): level j weighs 254^-j
+#pragma unroll
+                        for (int j = 0; j < Sh::NACC; j++) {
+                            uint32_t r[16];
+                            tmem_ld16(base + j * TBN + j4 * 16, r);
+                            tmem_wait_ld();
+                            const double w = j == 0 ? 1.0 : j == 1 ? 1.0 / 254.0 : j == 2 ? 1.0 / 64516.0
+                                           : j == 3 ? 1.0 / 16387064.0 : 1.0 / 4162314256.0;
+#pragma unroll
+                            for (int t = 0; t < 16; t++) acc[j4 * 16 + t] += (double)(int)r[t] * w;
+                        }
+                    } else {
+                        uint32_t r[Sh::NACC][16];
+#pragma unroll
+                        for (int j = 0; j < Sh::NACC; j++) tmem_ld16(base + j * TBN + j4 * 16, r[j]);
                         tmem_wait_ld();
-                        const double w = j == 0 ? 1.0 : j == 1 ? 1.0 / 254.0 : j == 2 ? 1.0 / 64516.0
-                                       : j == 3 ? 1.0 / 16387064.0 : 1.0 / 4162314256.0;
 #pragma unroll
-                        for (int t = 0; t < 16; t++) acc[j4 * 16 + t] += (double)(int)r[t] * w;
-                    }
-                } else {
-                    uint32_t r[Sh::NACC][16];
+                        for (int t = 0; t < 16; t++) {
+                            double v = 0.0;
 #pragma unroll
-                    for (int j = 0; j < Sh::NACC; j++) tmem_ld16(base + j * TBN + j4 * 16, r[j]);
-                    tmem_wait_ld();
-#pragma unroll
-                    for (int t = 0; t < 16; t++) {
-                        double v = 0.0;
-#pragma unroll
-                        for (int j = 0; j < Sh::NACC; j++) v += (double)__uint_as_float(r[j][t]);
-                        acc[j4 * 16 + t] += v;
+                            for (int j = 0; j < Sh::NACC; j++) v += (double)__uint_as_float(r[j][t]);
+                            acc[j4 * 16 + t] += v;
+                        }
                     }
                 }
+                tc_fence_before();
+                __syncwarp();
+                if (lane == 0) mbar_arrive(&tempty[b]);
             }
-            tc_fence_before();
-            __syncwarp();
-            if (lane == 0) mbar_arrive(&tempty[b]);
-        }
-        if (ok && (p.ks > 1 || p.dense)) {
-            const int m = m0 + q * 32 + lane;
-            if (m < p.M) {
-                const double sa = p.scaleA[m];
-                // [n][m]: the lanes of a warp write 32 consecutive rows
-                double* wz = p.ws + (int64_t)blockIdx.y * p.M * p.N + m;
+            if (ok && (p.ks > 1 || p.dense)) {
+                const int m = m0 + q * 32 + lane;
+                if (m < p.M) {
+                    const double sa = p.scaleA[m];
+                    // [n][m]: the lanes of a warp write 32 consecutive rows
+                    double* wz = p.ws + (int64_t)z * p.M * p.N + m;
 #pragma unroll
-                for (int j = 0; j < COLS; j++) {
-                    const int n = n0 + h * COLS + j;
-                    if (n < p.N) wz[(int64_t)n * p.M] = sa * p.scaleB[n] * acc[j];
-                }
-            }
-        } else if (ok && p.nvm == 1 && p.nvn == 1) {
-            // one destination per element: read EB destinations, then write them, so that
-            // the read-modify-writes of a thread overlap instead of running one by one
-            constexpr int EB = 8;
-            const int m = m0 + q * 32 + lane;
-            if (m < p.M) {
-                const double sa = p.alpha * p.vsign[0] * p.scaleA[m];
-                const int64_t cm0 = p.Cm0[m];
-#pragma unroll
-                for (int j0 = 0; j0 < COLS; j0 += EB) {
-                    int64_t off[EB];
-                    double old[EB];
-#pragma unroll
-                    for (int t = 0; t < EB; t++) {
-                        const int n = n0 + h * COLS + j0 + t;
-                        off[t] = n < p.N ? cm0 + p.Cn0[n] : -1;
-                    }
-#pragma unroll
-                    for (int t = 0; t < EB; t++) old[t] = off[t] >= 0 ? p.C[off[t]] : 0.0;
-#pragma unroll
-                    for (int t = 0; t < EB; t++) {
-                        const int n = n0 + h * COLS + j0 + t;
-                        if (off[t] >= 0) p.C[off[t]] = old[t] + sa * p.scaleB[n] * acc[j0 + t];
+                    for (int j = 0; j < COLS; j++) {
+                        const int n = n0 + h * COLS + j;
+                        if (n < p.N) wz[(int64_t)n * p.M] = sa * p.scaleB[n] * acc[j];
                     }
                 }
-            }
-        } else if (ok) {
-            const int m = m0 + q * 32 + lane;
-            if (m < p.M) {
-                const double sa = p.alpha * p.scaleA[m];
-                const int64_t cm0 = p.Cm0[m];
-                const int64_t cm1 = p.nvm > 1 ? p.Cm1[m] : 0;
+            } else if (ok && p.nvm == 1 && p.nvn == 1) {
+                // one destination per element: read EB destinations, then write them, so that
+                // the read-modify-writes of a thread overlap instead of running one by one
+                constexpr int EB = 8;
+                const int m = m0 + q * 32 + lane;
+                if (m < p.M) {
+                    const double sa = p.alpha * p.vsign[0] * p.scaleA[m];
+                    const int64_t cm0 = p.Cm0[m];
 #pragma unroll
-                for (int j = 0; j < COLS; j++) {
-                    const int n = n0 + h * COLS + j;
-                    if (n < p.N) {
-                        const double v = sa * p.scaleB[n] * acc[j];
-                        const int64_t cn0 = p.Cn0[n];
-                        p.C[cm0 + cn0] += p.vsign[0] * v;
-                        if (p.nvn > 1) p.C[cm0 + p.Cn1[n]] += p.vsign[1] * v;
-                        if (p.nvm > 1) {
-                            p.C[cm1 + cn0] += p.vsign[p.nvn] * v;
-                            if (p.nvn > 1) p.C[cm1 + p.Cn1[n]] += p.vsign[3] * v;
+                    for (int j0 = 0; j0 < COLS; j0 += EB) {
+                        int64_t off[EB];
+                        double old[EB];
+#pragma unroll
+                        for (int t = 0; t < EB; t++) {
+                            const int n = n0 + h * COLS + j0 + t;
+                            off[t] = n < p.N ? cm0 + p.Cn0[n] : -1;
+                        }
+#pragma unroll
+                        for (int t = 0; t < EB; t++) old[t] = off[t] >= 0 ? p.C[off[t]] : 0.0;
+#pragma unroll
+                        for (int t = 0; t < EB; t++) {
+                            const int n = n0 + h * COLS + j0 + t;
+                            if (off[t] >= 0) p.C[off[t]] = old[t] + sa * p.scaleB[n] * acc[j0 + t];
+                        }
+                    }
+                }
+            } else if (ok) {
+                const int m = m0 + q * 32 + lane;
+                if (m < p.M) {
+                    const double sa = p.alpha * p.scaleA[m];
+                    const int64_t cm0 = p.Cm0[m];
+                    const int64_t cm1 = p.nvm > 1 ? p.Cm1[m] : 0;
+#pragma unroll
+                    for (int j = 0; j < COLS; j++) {
+                        const int n = n0 + h * COLS + j;
+                        if (n < p.N) {
+                            const double v = sa * p.scaleB[n] * acc[j];
+                            const int64_t cn0 = p.Cn0[n];
+                            p.C[cm0 + cn0] += p.vsign[0] * v;
+                            if (p.nvn > 1) p.C[cm0 + p.Cn1[n]] += p.vsign[1] * v;
+                            if (p.nvm > 1) {
+                                p.C[cm1 + cn0] += p.vsign[p.nvn] * v;
+                                if (p.nvn > 1) p.C[cm1 + p.Cn1[n]] += p.vsign[3] * v;
+                            }
                         }
                     }
                 }
@@ -986,8 +1016,8 @@ void gemm_split(const SlicedOperand& a, const SlicedOperand& b, int M, int N, in
     p.dense = g.dense_out ? 1 : 0;
     if (g.dense_out && (!g.ws || (int64_t)ks * M * N > g.ws_elems))
         throw std::runtime_error("merged split product: dense output workspace too small");
-    const int tiles = (a.rows / BM) * p.tiles_n;
-    const dim3 grid(tiles, ks);
+    p.tiles = (a.rows / BM) * p.tiles_n;
+    const int grid = (int)std::min<int64_t>((int64_t)p.tiles * ks, 148);
     if (kind == SLICE_INT8) {
         if (ns == 3) split_gemm_kernel<3, true><<<grid, THREADS, si.smem, s>>>(ma, mb, p);
         else if (ns == 4) split_gemm_kernel<4, true><<<grid, THREADS, si.smem, s>>>(ma, mb, p);
