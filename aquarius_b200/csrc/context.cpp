@@ -52,9 +52,7 @@ Context::~Context() {
     cudaFree(d_scalar);
     cudaFree(splitk_ws);
     cudaFree(merged_ws);
-    for (double* q : merged_retired) cudaFree(q);
     cudaFree(tile_ws);
-    for (double* q : tile_retired) cudaFree(q);
     for (auto& p : pending) {
         cudaEventDestroy(p.second.first);
         cudaEventDestroy(p.second.second);
@@ -377,11 +375,7 @@ void Context::upload(Plan& p) {
                 if (kss > 1) need = std::max<int64_t>(need, (int64_t)kss * g.M * g.N);
             }
     }
-    if (need > splitk_elems) {
-        if (splitk_ws) dfree(splitk_ws, splitk_elems * sizeof(double));
-        splitk_ws = (double*)dmalloc(need * sizeof(double));
-        splitk_elems = need;
-    }
+    grow_ws(splitk_ws, splitk_elems, need);
     // every table of the steps not yet uploaded goes into ONE device buffer with one copy:
     // a symmetry-blocked plan has hundreds of thousands of tables, and an allocation and a
     // copy per table cost seconds alone and minutes when several solves share the driver
@@ -1018,12 +1012,18 @@ void Context::build_run(Plan& p, RunSchedule& rs, int first, int end) {
     rs.runs.push_back(std::move(run));
 }
 
-void Context::ensure_tile_ws(int64_t elems) {
-    if (elems <= tile_ws_elems) return;
-    // a captured graph may hold the old buffer: it lives as long as the context
-    if (tile_ws) tile_retired.push_back(tile_ws);
-    tile_ws = (double*)dmalloc(elems * sizeof(double));
-    tile_ws_elems = elems;
+// a shared workspace of at least `need` doubles; the old one is freed in stream order, after the
+// work that is queued on it
+void Context::grow_ws(double*& ws, int64_t& elems, int64_t need) {
+    if (need <= elems) return;
+    if (ws) {
+        dfree(ws, elems * sizeof(double));
+        ws_moves++;
+    }
+    ws = nullptr;
+    elems = 0;
+    ws = (double*)dmalloc(need * sizeof(double));
+    elems = need;
 }
 
 // one launch of the tiled kernel over these problems, its work laid out and uploaded
@@ -1040,7 +1040,7 @@ GemmLaunch Context::group_tiles(const std::vector<kern::GemmArgs>& probs, int ro
     l.nctas = (int)w.seg_start.size() - 1;
     l.nfolds = (int)w.folds.size();
     l.slots = w.slots;
-    if (w.slots > 0) ensure_tile_ws(kern::tile_ws_elems(w.slots, rows));
+    if (w.slots > 0) grow_ws(tile_ws, tile_ws_elems, kern::tile_ws_elems(w.slots, rows));
     l.d_probs = (kern::GemmArgs*)dmalloc(probs.size() * sizeof(kern::GemmArgs));
     stage_h2d(l.d_probs, probs.data(), probs.size() * sizeof(kern::GemmArgs));
     l.at_start = w.segs.size() * sizeof(kern::TileSeg);

@@ -323,11 +323,13 @@ public:
     kern::SlicedOperand ws_view[2];                        // workspace views of the current call
     double* merged_ws = nullptr;                           // dense products of merged launches
     int64_t merged_ws_elems = 0;
-    std::vector<double*> merged_retired;                   // outgrown, kept until the context goes
     double* tile_ws = nullptr;                             // partial tiles of grouped FP64 launches
     int64_t tile_ws_elems = 0;
-    std::vector<double*> tile_retired;                     // outgrown, kept until the context goes
-    void ensure_tile_ws(int64_t elems);
+    // Every plan of the context shares splitk_ws, split_ws, merged_ws and tile_ws, and the first
+    // launch of a larger plan moves them.  A captured graph holds their addresses by value: it
+    // keeps the count it was captured at, and a solver whose graph is older captures anew.
+    int64_t ws_moves = 0;
+    void grow_ws(double*& ws, int64_t& elems, int64_t need);
     GemmLaunch group_tiles(const std::vector<kern::GemmArgs>& probs, int rows, bool ak, bool bk);
     GemmLaunch group_skinny(const std::vector<kern::SkinnyArgs>& probs, int nt);
     void build_merged(Plan& p, GemmRun& run, int first, int end, std::vector<char>& merged,

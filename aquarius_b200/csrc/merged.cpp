@@ -416,13 +416,7 @@ void Context::build_merged(Plan& p, GemmRun& run, int first, int end, std::vecto
         for (int ns = 3; ns <= 5; ns++)
             need = std::max<int64_t>(need, (int64_t)kern::split_ksplit((int)M, (int)N, (int)K, ns, kern::SLICE_INT8) *
                                                M * N);
-        if (need > merged_ws_elems) {
-            // a smaller buffer stays allocated until the context goes: a captured graph of an
-            // earlier plan may still name it
-            if (merged_ws) merged_retired.push_back(merged_ws);
-            merged_ws = (double*)dmalloc(need * sizeof(double));
-            merged_ws_elems = need;
-        }
+        grow_ws(merged_ws, merged_ws_elems, need);
         // the slice workspaces too are sized here, before any capture
         ensure_ws(split_ws.a, (int)M, (int)K);
         ensure_ws(split_ws.b, (int)N, (int)K);

@@ -270,8 +270,7 @@ Solver::~Solver() { teardown(); }
 void Solver::teardown() {
     if (source) source->lambda_users--;
     source = nullptr;
-    if (graph_exec) cudaGraphExecDestroy(graph_exec);
-    if (graph) cudaGraphDestroy(graph);
+    drop_graph();
     ctx.release(iter_plan);
     ctx.release(tau_plan);
     ctx.release(energy_plan);
@@ -291,6 +290,13 @@ void Solver::teardown() {
         auto it = std::find(ctx.constant_tensors.begin(), ctx.constant_tensors.end(), t);
         if (it != ctx.constant_tensors.end()) ctx.constant_tensors.erase(it);
     }
+}
+
+void Solver::drop_graph() {
+    if (graph_exec) cudaGraphExecDestroy(graph_exec);
+    if (graph) cudaGraphDestroy(graph);
+    graph_exec = nullptr;
+    graph = nullptr;
 }
 
 void* Solver::alloc(size_t bytes) {
@@ -1075,10 +1081,7 @@ void Solver::iterate_async() {
             // hold the extrapolated residual at that mode's floor until they age out of the
             // ring: restart the subspace from the current amplitudes
             if (opts.diis_order > 1) CCSD_CUDA(cudaMemsetAsync(d_state + 1, 0, sizeof(int), ctx.stream));
-            if (graph_exec) cudaGraphExecDestroy(graph_exec);
-            if (graph) cudaGraphDestroy(graph);
-            graph_exec = nullptr;
-            graph = nullptr;
+            drop_graph();
             captured_once = false;
         }
     }
@@ -1088,6 +1091,8 @@ void Solver::iterate_async() {
         !ctx.host_only)
         autotune_slices();
     if (opts.use_graph) {
+        // another plan of this context has moved a workspace that the graph points into
+        if (graph_exec && graph_ws_moves != ctx.ws_moves) drop_graph();
         if (!graph_exec) {
             // the first iteration runs eagerly (it also warms every kernel), the graph is
             // captured from the second one on
@@ -1103,6 +1108,7 @@ void Solver::iterate_async() {
                 }
                 CCSD_CUDA(cudaStreamEndCapture(ctx.stream, &graph));
                 CCSD_CUDA(cudaGraphInstantiate(&graph_exec, graph, 0));
+                graph_ws_moves = ctx.ws_moves;
             } else {
                 launch_iteration();
                 captured_once = true;

@@ -53,6 +53,7 @@ public:
     cudaGraph_t graph = nullptr;
     cudaGraphExec_t graph_exec = nullptr;
     bool captured_once = false;
+    int64_t graph_ws_moves = 0;        // Context::ws_moves at the capture
     bool refined = false;           // moved to a more accurate contraction mode (refine_tol reached)
     // this solver's contraction mode (precision, slices): the context's routing fields are
     // shared by every solver on it, so each entry point that launches contractions first
@@ -125,6 +126,7 @@ private:
     void setup();
     void setup_or_teardown();
     void teardown();
+    void drop_graph();
     std::vector<int> constants() const;
     std::vector<int> owned_tensors() const;
     void launch_iteration();

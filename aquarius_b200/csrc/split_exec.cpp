@@ -80,7 +80,10 @@ void Context::ensure_ws(kern::SlicedOperand& w, int rows, int K) {
     if (w.data && w.bytes >= need && w.rows >= rp) return;
     const int keep_rows = std::max(rp, w.rows);
     const int64_t keep_bytes = std::max(need, w.bytes);
-    if (w.data) free_sliced(w);
+    if (w.data) {
+        free_sliced(w);
+        ws_moves++;
+    }
     w.rows = keep_rows;
     w.bytes = keep_bytes;
     w.data = (uint8_t*)dmalloc(keep_bytes);

@@ -89,3 +89,45 @@ def test_converges_like_oracle():
         s.close()
     finally:
         ctx.close()
+
+
+@pytest.mark.parametrize("precision", ["fp64", "split_i8"])
+def test_graph_outlives_a_larger_plan_on_its_context(precision):
+    """A captured iteration, then a contraction on the same context that needs more split-K and slicing
+    workspace than the iteration, then the iteration again: the same energies, residuals and amplitudes
+    as of a solver left alone, and tensors that took their memory in between keep their zeros."""
+    o, v, seed = 3, 10, 7
+    eps, B, *_ = A.synth_problem(seed, o, v)
+
+    def solve(disturb):
+        with A.Context(0) as ctx:
+            ctx.set_spaces(vrt=[v], occ=[o])
+            ctx.set_split_routing("all")
+            H = ctx.hamiltonian_from_factor(B, eps)
+            s = ctx.solver(H, diis_order=8, precision=precision, slices=4 if precision != "fp64" else 0,
+                           use_graph=True)
+            out = [s.iterate() for _ in range(4)]
+            held = []
+            if disturb:
+                if precision != "fp64":
+                    ctx.set_precision(precision, slices=4)
+                # 1000 = v^3 rows of <ab||cd> against one column, and <ab||cd> squared
+                big = [ctx.tensor(n, (2, 0), (2, 0), plain=True) for n in "xyz"]
+                before = ctx.device_bytes()
+                ctx.contract(1.0, big[0], "abef", big[1], "efcd", 0.0, big[2], "abcd")
+                fa = ctx.tensor("f", (1, 0), (1, 0), plain=True)
+                ctx.contract(1.0, big[0], "afbe", big[1], "cfbe", 0.0, fa, "ac")
+                assert ctx.device_bytes() > before
+                for k in range(24):
+                    held.append(ctx.tensor("h%d" % k, (2, 0), (k % 3, 2 - k % 3), plain=True) if k % 3 != 1
+                                else ctx.tensor("h%d" % k, (1, 1), (1, 1), plain=True))
+            out += [s.iterate() for _ in range(4)]
+            for t in held:
+                assert not t.to_full().any()
+            res = out, s.T1.to_full(), s.T2.to_full()
+            s.close()
+            return res
+
+    alone, beside = solve(False), solve(True)
+    assert alone[0] == beside[0]
+    assert np.array_equal(alone[1], beside[1]) and np.array_equal(alone[2], beside[2])
