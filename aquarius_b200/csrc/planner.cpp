@@ -254,53 +254,134 @@ void enumerate_dim(const std::vector<Unit>& units, const std::vector<Var>& vars,
 
 constexpr int kMaxVars = 32;   // C positions + internal letters of one statement (at most 8 + 8)
 
+// The k order of a skinny product.  Units follow A's positions, so where the other operand runs
+// along a later unit (VAMEF[amef] tau[efim]: k = m, then e, f) every element of it is a sector
+// of its own.  Four neighbours along that unit become the fastest index (next to four along
+// the first unit where that one is contiguous in an operand), so that the fragment loads of
+// both operands take whole 32-byte sectors, and the walk along the first unit goes on inside.
+// T1 residual, o=24 v=184 (184 x 24 over 812k): 619 -> 337 us; the case of few k is left alone (its
+// operands stay in L2).  Symmetry-blocked plans are too: merged products share their k tables.
+struct KOrder {
+    size_t p = 0;      // the unit whose neighbours come first, in fours (0: enumerate_dim's order)
+    size_t run = 1;    // neighbours along the first unit that stay together
+};
+
+KOrder skinny_k_order(const std::vector<Unit>& ku, const Operand& A, const Operand& B) {
+    auto fastest = [&](const Operand& op) -> int {   // the unit this operand is contiguous along, -1: a row index
+        int v = -1;
+        for (size_t q = 0; q < op.var.size(); q++)
+            if (op.blk->pair_of((int)q) < 0 && op.blk->stride[q] == 1 && op.blk->len[q] > 1) v = op.var[q];
+        for (auto& pr : op.blk->pairs)
+            if (pr.stride == 1) v = op.var[pr.p];
+        for (size_t u = 0; u < ku.size(); u++)
+            if (ku[u].v0 == v) return (int)u;
+        return -1;
+    };
+    const int fa = fastest(A), fb = fastest(B), p = std::max(fa, fb);
+    KOrder k;
+    if (p <= 0 || ku[p].size < 4) return k;
+    int64_t before = 1;
+    for (int u = 0; u < p; u++) before *= ku[u].size;
+    if (before < 2) return k;
+    k.p = p;
+    k.run = std::min(fa, fb) == 0 ? 4 : 1;
+    return k;
+}
+
 // Offset table of a GEMM dimension: out[k] = base + f(values at point k), points ordered as
-// enumerate_dim orders them (first unit fastest).  Every offset this planner tabulates is a
-// sum of one term per unit: an operand position depends on one variable, and a packed or
-// swapped pair on the two variables of one restricted-pair unit.  So each unit's terms are
-// evaluated once (f at that unit's values, all other variables 0, minus f at all zeros) and
+// enumerate_dim orders them (first unit fastest) or as `order` says.  Every offset this planner
+// tabulates is a sum of one term per unit: an operand position depends on one variable, and a
+// packed or swapped pair on the two variables of one restricted-pair unit.  So each unit's terms
+// are evaluated once (f at that unit's values, all other variables 0, minus f at all zeros) and
 // the table is their Kronecker sum: O(points) additions instead of O(points x positions).
 template <class F>
 void fill_table(std::vector<int64_t>& out, const std::vector<Unit>& units, const std::vector<Var>& vars, int64_t base,
-                F f) {
+                F f, const KOrder& order = KOrder()) {
     // per-thread scratch: planning runs statements on several threads, and the tables of a
     // large plan are filled a few million times
     thread_local std::vector<int64_t> val, cur, next, term;
     val.assign(vars.size(), 0);
     const int64_t f0 = f(val);
-    cur.assign(1, base + f0);
-    for (const Unit& u : units) {
-        term.resize(u.size);
-        // the unit's points in enumerate_dim's order: a value, a rectangle pair (first
-        // variable fastest) or a triangle pair x < y (y outer, x inner)
-        if (u.v1 < 0) {
-            for (int64_t c = 0; c < u.size; c++) {
-                val[u.v0] = c;
-                term[c] = f(val) - f0;
-            }
-        } else if (u.tri) {
-            int64_t c = 0;
-            for (int64_t y = 0; y < vars[u.v0].len; y++)
-                for (int64_t x = 0; x < y; x++) {
-                    val[u.v0] = x;
-                    val[u.v1] = y;
-                    term[c++] = f(val) - f0;
+    // Kronecker sum of units [u0, u1) into cur, which holds its starting value
+    auto sum_units = [&](size_t u0, size_t u1) {
+        for (size_t i = u0; i < u1; i++) {
+            const Unit& u = units[i];
+            term.resize(u.size);
+            // the unit's points in enumerate_dim's order: a value, a rectangle pair (first
+            // variable fastest) or a triangle pair x < y (y outer, x inner)
+            if (u.v1 < 0) {
+                for (int64_t c = 0; c < u.size; c++) {
+                    val[u.v0] = c;
+                    term[c] = f(val) - f0;
                 }
-        } else {
-            const int64_t n0 = vars[u.v0].len;
-            for (int64_t c = 0; c < u.size; c++) {
-                val[u.v0] = c % n0;
-                val[u.v1] = c / n0;
-                term[c] = f(val) - f0;
+            } else if (u.tri) {
+                int64_t c = 0;
+                for (int64_t y = 0; y < vars[u.v0].len; y++)
+                    for (int64_t x = 0; x < y; x++) {
+                        val[u.v0] = x;
+                        val[u.v1] = y;
+                        term[c++] = f(val) - f0;
+                    }
+            } else {
+                const int64_t n0 = vars[u.v0].len;
+                for (int64_t c = 0; c < u.size; c++) {
+                    val[u.v0] = c % n0;
+                    val[u.v1] = c / n0;
+                    term[c] = f(val) - f0;
+                }
+            }
+            val[u.v0] = 0;
+            if (u.v1 >= 0) val[u.v1] = 0;
+            next.resize(cur.size() * term.size());
+            for (size_t j = 0; j < term.size(); j++)
+                for (size_t t = 0; t < cur.size(); t++) next[j * cur.size() + t] = cur[t] + term[j];
+            cur.swap(next);
+        }
+    };
+    if (order.p == 0) {
+        cur.assign(1, base + f0);
+        sum_units(0, units.size());
+        out.assign(cur.begin(), cur.end());
+        return;
+    }
+    // the first unit, those before p, p and those after it apart, then the points in their order (a
+    // finished table permuted in a pass of its own took the planning of F(mi) += <mn||ef> t(ef,in) at
+    // o=20 v=160 from 14 to 19 ms)
+    thread_local std::vector<int64_t> first, mid, along, after;
+    auto part = [&](std::vector<int64_t>& t, size_t u0, size_t u1, int64_t start) {
+        cur.assign(1, start);
+        sum_units(u0, u1);
+        t.assign(cur.begin(), cur.end());
+    };
+    part(first, 0, 1, base + f0);
+    part(mid, 1, order.p, 0);
+    part(along, order.p, order.p + 1, 0);
+    part(after, order.p + 1, units.size(), 0);
+    const int64_t n0 = first.size(), np = along.size(), run = order.run;
+    cur.resize(n0 * mid.size() * np * after.size());
+    int64_t* at = cur.data();
+    const int64_t *f1 = first.data(), *fp = along.data();
+    for (const int64_t a : after)
+        for (int64_t y0 = 0; y0 < np; y0 += 4) {
+            const int64_t w = std::min<int64_t>(4, np - y0);
+            for (const int64_t m : mid) {
+                if (run == 1 && w == 4) {
+                    const int64_t s0 = m + a + fp[y0], s1 = m + a + fp[y0 + 1], s2 = m + a + fp[y0 + 2], s3 = m + a + fp[y0 + 3];
+                    for (int64_t i = 0; i < n0; i++, at += 4) {
+                        at[0] = f1[i] + s0;
+                        at[1] = f1[i] + s1;
+                        at[2] = f1[i] + s2;
+                        at[3] = f1[i] + s3;
+                    }
+                    continue;
+                }
+                for (int64_t i0 = 0; i0 < n0; i0 += run) {
+                    const int64_t i1 = std::min(n0, i0 + run);
+                    for (int64_t y = y0; y < y0 + w; y++)
+                        for (int64_t i = i0; i < i1; i++) *at++ = f1[i] + (fp[y] + m + a);
+                }
             }
         }
-        val[u.v0] = 0;
-        if (u.v1 >= 0) val[u.v1] = 0;
-        next.resize(cur.size() * term.size());
-        for (size_t j = 0; j < term.size(); j++)
-            for (size_t t = 0; t < cur.size(); t++) next[j * cur.size() + t] = cur[t] + term[j];
-        cur.swap(next);
-    }
     out.assign(cur.begin(), cur.end());
 }
 
@@ -323,48 +404,6 @@ int64_t operand_offset(const Operand& op, const std::vector<int64_t>& val, const
         if (up) off += pair_off(b, pr, val[vp], val[vq]);
     }
     return off;
-}
-
-// The k order of a skinny product.  Units follow A's positions, so where the other operand runs
-// along a later unit (VAMEF[amef] tau[efim]: k = m, then e, f) every element of it is a sector
-// of its own.  Four neighbours along that unit become the fastest index (next to four along
-// the first unit where that one is contiguous in an operand), so that the fragment loads of
-// both operands take whole 32-byte sectors, and the walk along the first unit goes on inside.
-// T1 residual, o=24 v=184 (184 x 24 over 812k): 619 -> 337 us; the case of few k is left alone (its
-// operands stay in L2).  Symmetry-blocked plans are too: merged products share their k tables.
-void block_k(GemmStep& g, const std::vector<Unit>& ku, const Operand& A, const Operand& B) {
-    auto fastest = [&](const Operand& op) -> int {   // the unit this operand is contiguous along, -1: a row index
-        int v = -1;
-        for (size_t q = 0; q < op.var.size(); q++)
-            if (op.blk->pair_of((int)q) < 0 && op.blk->stride[q] == 1 && op.blk->len[q] > 1) v = op.var[q];
-        for (auto& pr : op.blk->pairs)
-            if (pr.stride == 1) v = op.var[pr.p];
-        for (size_t u = 0; u < ku.size(); u++)
-            if (ku[u].v0 == v) return (int)u;
-        return -1;
-    };
-    const int fa = fastest(A), fb = fastest(B), p = std::max(fa, fb);
-    if (p <= 0) return;
-    const int64_t run = std::min(fa, fb) == 0 ? 4 : 1;   // neighbours along the first unit that stay together
-    int64_t n0 = ku[0].size, mid = 1, outer = 1;
-    const int64_t np = ku[p].size;
-    for (int u = 1; u < p; u++) mid *= ku[u].size;
-    for (size_t u = p + 1; u < ku.size(); u++) outer *= ku[u].size;
-    if (np < 4 || n0 * mid < 2) return;
-    std::vector<int64_t> a(g.hAk.size()), b(g.hBk.size());
-    size_t at = 0;
-    for (int64_t o = 0; o < outer; o++)
-        for (int64_t pc = 0; pc < np; pc += 4)
-            for (int64_t m = 0; m < mid; m++)
-                for (int64_t ic = 0; ic < n0; ic += run)
-                    for (int64_t y = pc; y < std::min(np, pc + 4); y++)
-                        for (int64_t i = ic; i < std::min(n0, ic + run); i++, at++) {
-                            const size_t k = ((o * np + y) * mid + m) * n0 + i;
-                            a[at] = g.hAk[k];
-                            b[at] = g.hBk[k];
-                        }
-    g.hAk.swap(a);
-    g.hBk.swap(b);
 }
 
 struct Term {
@@ -540,10 +579,11 @@ void lower_gemm(Context& ctx, Term& t, int hA, int hB, int hC, int cc, std::set<
     const Block& bB = *t.B.blk;
     const Block& bC = *t.bC;
     fill_table(g.hAm, mu, vars, bA.offset, [&](const std::vector<int64_t>& val) { return operand_offset(t.A, val, all_m); });
-    fill_table(g.hAk, ku, vars, 0, [&](const std::vector<int64_t>& val) { return operand_offset(t.A, val, all_k); });
-    fill_table(g.hBk, ku, vars, 0, [&](const std::vector<int64_t>& val) { return operand_offset(t.B, val, all_k); });
+    KOrder order;
+    if (ctx.spaces.nirrep == 1 && std::min(M, N) <= 32 && K >= 512) order = skinny_k_order(ku, t.A, t.B);
+    fill_table(g.hAk, ku, vars, 0, [&](const std::vector<int64_t>& val) { return operand_offset(t.A, val, all_k); }, order);
+    fill_table(g.hBk, ku, vars, 0, [&](const std::vector<int64_t>& val) { return operand_offset(t.B, val, all_k); }, order);
     fill_table(g.hBn, nu, vars, bB.offset, [&](const std::vector<int64_t>& val) { return operand_offset(t.B, val, all_n); });
-    if (ctx.spaces.nirrep == 1 && std::min(M, N) <= 32 && K >= 512) block_k(g, ku, t.A, t.B);
     if (dest_x) {
         // plain column-major scratch product: no variants
         g.nvm = g.nvn = 1;

@@ -148,3 +148,32 @@ def test_export_without_a_statement_is_an_error(tmp_path):
     with _ctx(1) as ctx:
         with pytest.raises(A.CcsdError):
             ctx.plan_export(tmp_path / "plan.txt")
+
+
+# products of one extent <= 32 over a long k walk it in another order than their units (four
+# neighbours along the unit that the other operand is contiguous in come first)
+LONG_K = [("mi", "mi", "mnef", "mnef", "abij", "efin"), ("ai", "ai", "amef", "amef", "abij", "efim")]
+
+
+@pytest.mark.parametrize("o,v", [(5, 13), (7, 11), (6, 16)], ids=["o5v13", "o7v11", "o6v16"])
+@pytest.mark.parametrize("case", LONG_K, ids=[f"{c[0]}+={c[2]}*{c[4]}" for c in LONG_K])
+def test_long_k_order_replays_to_reference(case, o, v, tmp_path):
+    """Every k of a long skinny product once, in the same order for both operands: extents that four
+    does and does not divide, along the first unit and along the other."""
+    cs, ic, as_, ia, bs, ib = case
+    rng = np.random.default_rng(o * v)
+    with A.Context(-1) as ctx:
+        ctx.set_spaces(vrt=[v], occ=[o])
+        tA, tB, tC = ctx.tensor("A", *SHAPES[as_]), ctx.tensor("B", *SHAPES[bs]), ctx.tensor("C", *SHAPES[cs])
+        fa, fb, fc = (random_so(ctx, *SHAPES[x], rng) for x in (as_, bs, cs))
+        ctx.contract(0.5, tA, ia, tB, ib, 1.0, tC, ic)
+        ctx.plan_export(tmp_path / "plan.txt")
+        dump, store = _replay_one(ctx, None, {tA.h: fa, tB.h: fb, tC.h: fc}, tmp_path / "plan.txt")
+        gemms = [g for g in dump.steps if g[0] == "gemm" and min(g[4:6]) <= 32 and g[6] >= 512]
+        # the order is in use: neighbours of B first, where A's units begin with another letter
+        assert any((np.diff(g[11][t][:4]) == 1).all() for g in gemms for t in ("Ak", "Bk"))
+        want = R.to_storage(ctx, dump.tensors[tC.h], reference_contract(0.5, fa, ia, fb, ib, 1.0, fc, ic, tC.group))
+        # sums of K terms in two orders differ by at most 2 (K + 1) u sum |a b|, u = 2^-53, at most four
+        # products add to an element
+        K = max(g[6] for g in gemms)
+        assert np.abs(store[tC.h] - want).max() <= 4 * 2.0**-52 * (K + 1) * K * np.abs(fa).max() * np.abs(fb).max()
