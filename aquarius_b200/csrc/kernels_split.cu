@@ -25,7 +25,7 @@
 //   254^-t in FP64.  Per product the error is ~254^-NS / 2 of row max x column max
 //   (3.7e-8, 1.5e-10, 5.7e-13 for 3, 4, 5 slices).
 //
-// Kernel structure (one CTA per SM walks 128 x TBN output tiles, 320 threads):
+// Kernel structure (one CTA per SM walks several 128 x TBN output tiles, 320 threads):
 //   warp 0      TMA producer: NS A-slice + NS B-slice tiles of 128-byte k-blocks per
 //               stage (128-byte swizzle), 2 stages, mbarrier full/empty ring;
 //   warp 1      TMEM allocation and the single-thread MMA issuer: one MMA per kept slice
@@ -69,6 +69,13 @@ constexpr int EPI_WARPS = 8;
 constexpr int THREADS = 32 * (2 + EPI_WARPS);
 constexpr long long WAIT_CYCLES = 4000000000ll;     // ~2 s at 1.9 GHz
 constexpr int SMEM_LIMIT = 227 * 1024;
+constexpr int SMS = 148;
+// How long a CTA keeps its SM: as many tiles as make 40960 k, 16 at most (0.3 to 1 ms), so that work of
+// another stream, one of higher priority above all, gets SMs before the product ends.  D2h o=24 v=180
+// beside o=31 v=255 on a stream of lower priority (ms per iteration of the small one, 95th percentile):
+// 77 and 111; 85 and 123 with CTAs that walk the whole product, 70 and 97 with a CTA per tile.  Alone,
+// four iterations of o=24 v=184 take 215.3 ms; 214.0 and 223.8 with those.
+constexpr int HOLD_K = 40960, HOLD_TILES = 16;
 
 // Kernel shape per scheme.  A stage holds NS A tiles and NS B tiles of one k-block (a
 // 128- or 64-byte row segment); as many stages as fit in shared memory (at most 4).
@@ -123,6 +130,7 @@ struct Params {
     double vsign[4];
     int* err;
     int tiles;                     // output tiles
+    int stride, steps, gens;       // work items per step, steps, and CTAs that share a lane's steps
     // split-K: K-block range z of ks, partials (scales applied,
     // alpha not) to ws[z][n][m], folded into C by split_fold_kernel
     int ks;
@@ -247,8 +255,11 @@ __global__ void __launch_bounds__(THREADS, 1)
     volatile int* abort_flag = (volatile int*)(tmem_slot + 1);
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    // work item w: tile w % tiles of K range w / tiles; its K blocks are [kb0, kb0 + nkb)
-    const int total = p.tiles * p.ks;
+    // work item w: tile w % tiles of K range w / tiles; its K blocks are [kb0, kb0 + nkb).  Step s
+    // of a lane is item s * stride + lane; CTA generation g takes steps [g, g + 1) * steps / gens
+    const int gen = blockIdx.x / p.stride, lane0 = blockIdx.x % p.stride;
+    const int first = (int)((int64_t)p.steps * gen / p.gens) * p.stride + lane0;
+    const int total = min(p.tiles * p.ks, (int)((int64_t)p.steps * (gen + 1) / p.gens) * p.stride);
     auto work = [&](int w, int& m0, int& n0, int& z, int& kb0, int& nkb) {
         const int tile = w % p.tiles;
         z = w / p.tiles;
@@ -285,7 +296,7 @@ __global__ void __launch_bounds__(THREADS, 1)
             // ---------------- TMA producer ----------------
             int it = 0;                  // K blocks of all tiles so far: stage and phase
             bool ok = true;
-            for (int w = blockIdx.x, m0, n0, z, kb0, nkb; w < total && ok; w += gridDim.x) {
+            for (int w = first, m0, n0, z, kb0, nkb; w < total && ok; w += p.stride) {
                 work(w, m0, n0, z, kb0, nkb);
                 for (int kb = 0; kb < nkb && !*abort_flag; kb++, it++) {
                     const int s = it % STAGES;
@@ -310,7 +321,7 @@ __global__ void __launch_bounds__(THREADS, 1)
             // ---------------- MMA issuer ----------------
             int it = 0, cc = 0;          // K blocks and chunks of all tiles so far
             bool ok = true;
-            for (int w = blockIdx.x, m0, n0, z, kb0, nkb; w < total && ok; w += gridDim.x) {
+            for (int w = first, m0, n0, z, kb0, nkb; w < total && ok; w += p.stride) {
                 work(w, m0, n0, z, kb0, nkb);
                 int kb = 0;
                 for (int kb_end; kb < nkb && !*abort_flag; cc++) {
@@ -372,7 +383,7 @@ __global__ void __launch_bounds__(THREADS, 1)
         double acc[COLS];
         bool ok = true;
         int cc = 0;                      // chunks of all tiles so far
-        for (int w = blockIdx.x, m0, n0, z, kb0, nkb; w < total && ok; w += gridDim.x) {
+        for (int w = first, m0, n0, z, kb0, nkb; w < total && ok; w += p.stride) {
             work(w, m0, n0, z, kb0, nkb);
             const int nchunks = (nkb + Sh::CHUNK - 1) / Sh::CHUNK;
 #pragma unroll
@@ -1017,7 +1028,14 @@ void gemm_split(const SlicedOperand& a, const SlicedOperand& b, int M, int N, in
     if (g.dense_out && (!g.ws || (int64_t)ks * M * N > g.ws_elems))
         throw std::runtime_error("merged split product: dense output workspace too small");
     p.tiles = (a.rows / BM) * p.tiles_n;
-    const int grid = (int)std::min<int64_t>((int64_t)p.tiles * ks, 148);
+    const int64_t items = (int64_t)p.tiles * ks;
+    p.stride = (int)std::min<int64_t>(items, SMS);
+    p.steps = (int)((items + p.stride - 1) / p.stride);
+    // gens CTAs in turn take a lane's steps, hold each: the steps are dealt out in whole waves, so the
+    // number of waves stays that of a single walk
+    const int hold = std::max(1, std::min(HOLD_TILES, HOLD_K / (std::min(nkb, p.kb_per) * si.bke)));
+    p.gens = (p.steps + hold - 1) / hold;
+    const unsigned grid = (unsigned)(p.stride * p.gens);
     if (kind == SLICE_INT8) {
         if (ns == 3) split_gemm_kernel<3, true><<<grid, THREADS, si.smem, s>>>(ma, mb, p);
         else if (ns == 4) split_gemm_kernel<4, true><<<grid, THREADS, si.smem, s>>>(ma, mb, p);

@@ -6,6 +6,8 @@ INT8 slices carry 7 bits each (3e-5, 3e-7, 3e-9 for three, four, five).  A full 
 agrees with the FP64 oracle to |dE| <= 1e-8 Eh and max|dT| <= 1e-7 at every iteration with
 three BF16 or four INT8 slices.
 """
+import time
+
 import numpy as np
 import pytest
 
@@ -123,3 +125,41 @@ def test_int8_slices_at_odd_extents(o, v, slices):
         got = _contract("split_i8", o, v, ia, sa, ib, sb, ic, sc, 5, False, slices=slices)
         bound = K * 0.05 * 6 * 0.01 * 6 * (254.0 ** (1 - slices) / 127 + 2 * slices * 254.0 ** -slices)
         assert np.abs(got - ref).max() <= bound, (sa, np.abs(got - ref).max(), bound)
+
+
+def test_a_small_product_gets_in_beside_a_large_one():
+    """A split product of 16384 tiles on a stream of low priority gives its SMs back as it goes: a
+    small split product on a stream of high priority, queued while it runs, is there in less than
+    half of the time the large one takes (one that kept its SMs held the small one up to its end)."""
+    torch = pytest.importorskip("torch")
+    streams = [torch.cuda.Stream(priority=p) for p in (0, -5)]
+    ctxs = [A.Context(0, s.cuda_stream) for s in streams]
+    try:
+        runs = []
+        for ctx, (o, v) in zip(ctxs, [(128, 64), (16, 64)]):
+            ctx.set_spaces(vrt=[v], occ=[o])
+            ctx.set_precision("split_i8", slices=4)
+            ctx.set_split_routing("all")
+            x, y, z = (ctx.tensor(n, *sh, plain=True) for n, sh in
+                       (("x", ((0, 2), (2, 0))), ("y", ((2, 0), (0, 2))), ("z", ((0, 2), (0, 2)))))
+            runs.append(lambda ctx=ctx, x=x, y=y, z=z: ctx.contract(1.0, x, "mnef", y, "efij", 0.0, z, "mnij"))
+        large, small = runs
+        wait = lambda: [ctx.synchronize() for ctx in ctxs]
+        for _ in range(3):
+            large(), small(), wait()
+        t0 = time.perf_counter()
+        large(), wait()
+        whole = time.perf_counter() - t0
+        late = []
+        for _ in range(5):
+            large()
+            time.sleep(0.4 * whole)
+            t0 = time.perf_counter()
+            small(), ctxs[1].synchronize()
+            late.append(time.perf_counter() - t0)
+            wait()
+        assert min(late) < 0.25 * whole, (late, whole)
+        assert sorted(late)[2] < 0.45 * whole, (late, whole)
+    finally:
+        for ctx in ctxs:
+            ctx.close()
