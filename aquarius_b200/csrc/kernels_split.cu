@@ -1,10 +1,11 @@
 // Split (Ozaki-style) contraction path on the sm_100a tensor cores.
 //
 // Each FP64 operand row x (a row of A(m,:) or a column of B(:,n), gathered through
-// the planner's offset tables) is scaled by a power of two from its max-abs and cut
-// into slices, round-to-nearest at each step (so the truncation error is unbiased):
+// the planner's offset tables) is scaled from its max-abs, rounded to nearest and cut into
+// slices:
 //
-// BF16 slices (3 or 4):   x = 2^(e-6) * (s1 + s2 + s3 [+ s4]),  2^e <= max|x| < 2^(e+1),
+// BF16 slices (3 or 4):   x = 2^(e-6) * (s1 + s2 + s3 [+ s4]),  2^e <= max|x| < 2^(e+1), each
+//   the rounded remainder of those before,
 //   s1 an integer in [-128,128], s2 = integer/2^8, s3 = integer/2^16, all exact in BF16.
 //   The tcgen05 GEMM (kind::f16) keeps FP32 accumulators in TMEM:
 //     L2  = sum_k s1a*s1b                         (products <= 2^14: a chunk of 1024 k
@@ -16,9 +17,10 @@
 //
 // INT8 slices (3, 4 or 5):  x = (max/127) * (q1 + q2/254 + q3/254^2 ...),  q_t in [-127,127],
 //   the whole signed 8-bit range: y = x * 127/max lies in [-127,127] and is rounded to a
-//   multiple of 254^-(NS-1), whose digits of base 254 (offset by 127) are the slices, so every
+//   multiple of 254^-(NS-1), whose balanced digits of base 254 are the slices, so every
 //   slice carries log2(254) = 7.99 bits and the first ns slices are an ns-slice slicing (the
-//   rest is within half a unit of the last one).  The tcgen05 GEMM (kind::i8, twice the BF16 rate)
+//   rest is within 0.502 units of the last one, with mean zero over an even and an odd k:
+//   I8Digits).  The tcgen05 GEMM (kind::i8, twice the BF16 rate)
 //   accumulates every level t = i+j of the kept products q_i*q_j (i+j < NS) in its own
 //   INT32 accumulator, which is exact (|q_i q_j| <= 127^2 < 2^14, at most 5 products per
 //   level: a drained chunk of 16384 k stays below 2^31); the epilogue weights level t by
@@ -621,37 +623,42 @@ __device__ __forceinline__ int round_int(double t) {
 // INT8 slices.  127 * 254^3 < 2^31: up to four digits of base 254 are one 32-bit integer, so x
 // is rounded once, to a multiple of 254^-(NS-1), and the digits come from integer divisions by
 // 254 (the running remainder took a double rounding and a conversion per slice, which run at
-// a quarter of the rate of a sum).  Digits are 0..253 (the leading one 0..254) after an
-// offset of 127 each, so every slice lies in [-127, 127].
+// a quarter of the rate of a sum).  Digits are 0..253 (the leading one 0..254) after an offset, and
+// every slice lies in [-127, 127].
 //   five slices: two digits of the rounded value, three of its remainder
+// The leading digit's offset is 127.  The others cover -127..126 (offset 127) for even k and
+// -126..127 (offset 126) for odd k: a contraction that reads a prefix of the slices drops the lower
+// digits, whose mean is -1/2 with one offset for all k.  Over K = 33856 positive elements that mean
+// made the error of three slices of four 1.8 times that of three slices rounded by themselves;
+// with the two offsets in turn it is the same.
 template <int NS>
 struct I8Digits {
     static constexpr int HI = NS == 5 ? 2 : NS, LO = NS - HI;
     // the factor of a row with 127 / max: 254^(HI-1)
     static constexpr double SCALE = HI == 2 ? 254.0 : HI == 3 ? 64516.0 : 16387064.0;
-    static constexpr unsigned OFFSET = HI == 2 ? 127u * 255u : HI == 3 ? 127u * 64771u : 127u * 16451835u;
-    __device__ static __forceinline__ void put(double x, double mul, unsigned (&w)[NS], int at) {
-        const double t = x * mul;
-        const int n = round_int(t);
-        unsigned u = (unsigned)n + OFFSET;
+    // offset of `n` digits, the lower ones' being `low`
+    static constexpr unsigned offset(int n, unsigned low) {
+        return n == 2 ? 127u * 254u + low : n == 3 ? 127u * 64516u + low * 255u : 127u * 16387064u + low * 64771u;
+    }
+    // digits of u, from slice `first + n - 1` up to `first`, as bytes
+    template <int N>
+    __device__ static __forceinline__ void digits(unsigned u, unsigned low, unsigned (&w)[NS], int first, int at) {
 #pragma unroll
-        for (int q = HI - 1; q > 0; q--) {
+        for (int q = N - 1; q > 0; q--) {
             const unsigned r = u / 254u;
-            w[q] |= ((u - r * 254u + 129u) & 255u) << (8 * at);   // - 127 in a byte
+            w[first + q] |= ((u - r * 254u + 256u - low) & 255u) << (8 * at);
             u = r;
         }
-        w[0] |= ((u + 129u) & 255u) << (8 * at);
-        if constexpr (LO > 0) {
-            // the remainder, in [-1/2, 1/2], as three digits
-            unsigned v = (unsigned)round_int((t - (double)n) * 16387064.0) + 127u * 64771u;
-#pragma unroll
-            for (int q = NS - 1; q > HI; q--) {
-                const unsigned r = v / 254u;
-                w[q] |= ((v - r * 254u + 129u) & 255u) << (8 * at);
-                v = r;
-            }
-            w[HI] |= ((v + 129u) & 255u) << (8 * at);
-        }
+        w[first] |= ((u + 129u) & 255u) << (8 * at);
+    }
+    // element `at` of four neighbours from an even k
+    __device__ static __forceinline__ void put(double x, double mul, unsigned (&w)[NS], int at) {
+        const unsigned low = 127u - (at & 1);
+        const double t = x * mul;
+        const int n = round_int(t);
+        digits<HI>((unsigned)n + offset(HI, low), low, w, 0, at);
+        // the remainder, in [-1/2, 1/2]
+        if constexpr (LO > 0) digits<LO>((unsigned)round_int((t - (double)n) * 16387064.0) + offset(LO, low), low, w, HI, at);
     }
 };
 

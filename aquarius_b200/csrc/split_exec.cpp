@@ -183,9 +183,9 @@ void Context::run_split_gemm(GemmStep& g, kern::GemmArgs& a) {
         const bool kc = is_a ? a.a_kcontig : a.b_kcontig;
         const int h = is_a ? g.tA : g.tB;
         bool& cached = is_a ? g.cache_a : g.cache_b;
-        // the first ns slices of a deeper slicing are an ns-slice slicing (the rest is within half
-        // a unit of the last one): a cached operand with more slices serves
-        // a contraction that the autotuner runs with fewer
+        // the first ns slices of a deeper slicing are an ns-slice slicing (the rest is within 0.502
+        // units of the last one, without a bias): a cached operand with more slices serves a
+        // contraction that the autotuner runs with fewer
         if (cached && key >= 0 && split_cache[key].kind == kind && split_cache[key].nslices > ns) {
             kern::SlicedOperand& v = ws_view[is_a ? 0 : 1];
             v = split_cache[key];

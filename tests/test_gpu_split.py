@@ -127,6 +127,39 @@ def test_int8_slices_at_odd_extents(o, v, slices):
         assert np.abs(got - ref).max() <= bound, (sa, np.abs(got - ref).max(), bound)
 
 
+def test_first_slices_of_a_deeper_slicing_are_unbiased():
+    """A constant operand sliced four times serves a contraction with three slices.  Every element here
+    sits half a unit of the third slice beside a multiple of it: rounded all to one side, the K
+    contributions to an element add up to K / 2 units; rounded independently, to sqrt(K) / 2."""
+    o, v = 3, 24
+    rng = np.random.default_rng(4)
+    eps, B, *_ = A.synth_problem(3, o, v)
+    with A.Context(0) as ctx:
+        ctx.set_spaces(vrt=[v], occ=[o])
+        H = ctx.rhf_hamiltonian_from_factor(B, eps)
+        s = ctx.solver(H)                       # the integrals are its constants: their slices are kept
+        V = H["VABCD"]
+        alpha = V.spin_cases()[0]
+        n = 254 * rng.integers(-127 * 254**2 + 1, 127 * 254**2, size=(v, v, v, v)) - 127
+        n[:, :, 0, 0] = 127 * 254**3            # the row maximum, a multiple
+        x = n / (127 * 254.0**3)
+        V.write_block(alpha, x)
+        t = ctx.tensor("t", (2, 0), (0, 2), plain=True)
+        t.fill(1.0)                             # one digit: the other operand is exact
+        z = ctx.tensor("z", (2, 0), (0, 2), plain=True)
+        ctx.set_split_routing("all")
+        err = {}
+        for slices in (4, 3):
+            ctx.set_precision("split_i8", slices=slices)
+            ctx.contract(1.0, V, "abef", t, "efij", 0.0, z, "abij")
+            err[slices] = np.abs(z.to_full() - x.sum((2, 3))[:, :, None, None]).max()
+        ctx.set_precision("fp64")
+        s.close()
+    K, unit = v * v, 1 / 127 / 254.0**2
+    assert err[4] <= 6 * K**0.5 * unit / 254
+    assert 0.01 * unit < err[3] <= 5 * 0.5 * K**0.5 * unit, (err[3] / unit, K)
+
+
 def test_a_small_product_gets_in_beside_a_large_one():
     """A split product of 16384 tiles on a stream of low priority gives its SMs back as it goes: a
     small split product on a stream of high priority, queued while it runs, is there in less than
