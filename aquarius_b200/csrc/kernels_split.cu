@@ -41,7 +41,8 @@
 //               stage, 10 to 25 us of a 90 us tile at K=4416; D2h o=24 v=180, products of a
 //               few hundred rows: 18.7 -> 16.4 ms of four iterations.
 // Every mbarrier wait is bounded (about 2 s); on expiry the kernel records an error
-// code, stops issuing work and returns after releasing its TMEM.
+// code, stops issuing work, waits (bounded again) for its copies and products in flight, which
+// write to its shared memory and TMEM, and returns after releasing its TMEM.
 #include <algorithm>
 #include <atomic>
 #include <cstdint>
@@ -184,6 +185,13 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, volati
     }
 }
 
+// bounded wait after an abort, for work that this thread has in flight
+__device__ __forceinline__ void mbar_drain(uint64_t* bar, uint32_t parity) {
+    const long long t0 = clock64();
+    while (!mbar_try(bar, parity) && clock64() - t0 < WAIT_CYCLES) {
+    }
+}
+
 __device__ __forceinline__ void tma_load_2d(void* dst, const CUtensorMap* map, int x, int y, uint64_t* bar) {
     asm volatile(
         "cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];" ::"r"(
@@ -317,6 +325,8 @@ __global__ void __launch_bounds__(THREADS, 1)
                 }
                 ok = ok && !*abort_flag;
             }
+            if (*abort_flag)
+                for (int i = max(0, it - STAGES); i < it; i++) mbar_drain(&full[i % STAGES], (i / STAGES) & 1);
         }
     } else if (warp == 1) {
         if (lane == 0) {
@@ -376,6 +386,8 @@ __global__ void __launch_bounds__(THREADS, 1)
                 }
                 ok = ok && !*abort_flag;
             }
+            // the last commit to a stage covers every product before it
+            if (*abort_flag && it > 0) mbar_drain(&empty[(it - 1) % STAGES], ((it - 1) / STAGES) & 1);
         }
     } else {
         // ---------------- epilogue ----------------
