@@ -362,12 +362,12 @@ void Context::upload(Plan& p) {
     const bool reserve = split_precision() && !p.split_reserved && (host_only || kern::split_supported());
     if (p.tables_ready && !reserve) return;
     if (p.scratch_elems > 0 && !p.scratch) p.scratch = (double*)dmalloc(p.scratch_elems * sizeof(double));
-    // split-K workspace of the FP64 GEMM, grown before any capture
+    // workspace for the K ranges of skinny and split products, grown before any capture
     int64_t need = 0;
     for (auto& g : p.gemms) {
-        int ks = kern::fp64_ksplit(g.M, g.N, g.K, !fp64_tiled_only);
+        const int ks = fp64_tiled_only ? 1 : kern::skinny_ksplit(g.M, g.N, g.K);
         if (ks > 1) need = std::max<int64_t>(need, (int64_t)ks * g.M * g.N);
-        // split-precision GEMMs share the space (every scheme a refinement may reach)
+        // (split products: every scheme a refinement may reach)
         for (int kind : {kern::SLICE_BF16, kern::SLICE_INT8})
             for (int ns = 3; ns <= 5; ns++) {
                 if (!kern::slice_scheme_ok(kind, ns)) continue;
@@ -525,8 +525,9 @@ kern::GemmArgs Context::gemm_args(Plan& p, const GemmStep& g) {
 // GEMM steps of one statement: they read only the statement's operands and write its
 // output (or the plan scratch), so the only hazard among them is two writes to one
 // output block.  Each step gets a level one above the last level that wrote any of its
-// output blocks; within a level the small FP64 products (fewer than a wave of tiles, no
-// split-K) become one grouped launch per operand contiguity, the rest launch alone.
+// output blocks; within a level the FP64 products of the tiled kernel become one grouped launch
+// per operand contiguity and tile size, the skinny ones without K ranges one per width; large
+// skinny products and split products launch alone.
 // Every output block thus receives its contributions in plan order.  Runs of permuted
 // sums (antisymmetriser images, copies) and of block scalings of one statement are
 // batched the same way, one launch per level.
@@ -599,8 +600,8 @@ void Context::build_run(Plan& p, RunSchedule& rs, int first, int end) {
         if (routes_split(g) || g.M <= 0 || g.N <= 0 || g.K <= 0) return false;
         if (fp64_tiled_only || kern::skinny_groups(g.M, g.N) == 0) return true;
         // a skinny product (one extent <= 32) with a long operand of 4M elements or more is
-        // bandwidth work for the skinny kernel: on a 128 x 64 tile it would use 1/64 to 1/2
-        // of every tile (F(ae) += <am||ef> t(fm) at o=16 v=128: 2.3 ms grouped)
+        // bandwidth work for the skinny kernel: on tiles it would use a part of each (F(ae) +=
+        // <am||ef> t(fm) at o=16 v=128: 2.3 ms on tiles of 128 x 64)
         if ((int64_t)std::max(g.M, g.N) * g.K >= (int64_t)1 << 22) return false;
         // and so is a skinny product with a long side of a tile or more: the grouped skinny
         // launch streams it (the tiles would stay 1/8 to 1/2 empty and walk it at a fraction
@@ -617,7 +618,7 @@ void Context::build_run(Plan& p, RunSchedule& rs, int first, int end) {
     // skinny products without a K split share one launch per level and shape
     auto skinny_groupable = [&](const GemmStep& g) {
         return !fp64_tiled_only && !routes_split(g) && !groupable(g) && kern::skinny_groups(g.M, g.N) > 0 &&
-               kern::fp64_ksplit(g.M, g.N, g.K, true) == 1;
+               kern::skinny_ksplit(g.M, g.N, g.K) == 1;
     };
     // tiled products by operand contiguity (bits 0, 1) and tile size (bit 2: 32 x 32)
     auto tile_class = [](const GemmStep& g) {
@@ -719,7 +720,7 @@ void Context::build_run(Plan& p, RunSchedule& rs, int first, int end) {
                 continue;
             // (small outputs only: one CTA folds a group, so a large partial stays with the
             // product's own launch and its parallel fold)
-            const int ks = kern::fp64_ksplit(g.M, g.N, g.K, true);
+            const int ks = kern::skinny_ksplit(g.M, g.N, g.K);
             const int64_t mn = (int64_t)g.M * g.N;
             if (ks < 2 || mn > 16384 || ks * mn > 262144 || skpart + ks * mn > (64ll << 20)) continue;
             in_fold[i - first] = 3;
@@ -1039,7 +1040,6 @@ GemmLaunch Context::group_tiles(const std::vector<kern::GemmArgs>& probs, int ro
     const kern::TileWork w = kern::plan_tile_work(shapes, rows, true);
     l.nctas = (int)w.seg_start.size() - 1;
     l.nfolds = (int)w.folds.size();
-    l.slots = w.slots;
     if (w.slots > 0) grow_ws(tile_ws, tile_ws_elems, kern::tile_ws_elems(w.slots, rows));
     l.d_probs = (kern::GemmArgs*)dmalloc(probs.size() * sizeof(kern::GemmArgs));
     stage_h2d(l.d_probs, probs.data(), probs.size() * sizeof(kern::GemmArgs));

@@ -194,7 +194,7 @@ struct GemmLaunch {
     int nprob = 0, tiles = 0;
     kern::GemmArgs* d_probs = nullptr; // grouped GEMM: problems and, in d_desc, their TileSeg[], the
     int rows = 64, nctas = 0;          // CTAs' first segments and the TileFold[] of shared tiles
-    int nfolds = 0, slots = 0;
+    int nfolds = 0;
     size_t at_start = 0, at_folds = 0; // byte offsets of the two in d_desc
     int* d_tile_start = nullptr;
     double* d_part = nullptr;          // shared-output group: partial products (part_elems doubles)
@@ -338,7 +338,7 @@ public:
     void batch_merged_slicing(GemmRun& run, size_t launch0);
     int64_t merged_cache_bytes = 0;                        // reserved by merged products' cached slices
     void free_merged(MergedProduct& m);
-    double* splitk_ws = nullptr;                           // FP64 split-K partials
+    double* splitk_ws = nullptr;                           // K ranges of skinny and split products
     int64_t splitk_elems = 0;
     kern::SlicedOperand alloc_sliced(int rows, int K, int nslices, int kind);
     // slices per operand of the split path (3 unless set) and their kind

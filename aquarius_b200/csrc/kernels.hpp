@@ -22,7 +22,7 @@ struct GemmArgs {
     double vsign[4] = {1, 1, 1, 1};
     bool a_kcontig = false;   // consecutive k -> consecutive A addresses
     bool b_kcontig = false;   // consecutive k -> consecutive B addresses
-    // split-K: partial products of ksplit K-ranges go to ws[z][m][n] (M*N*ksplit doubles)
+    // K ranges of skinny and split products: their partial products go to ws (M*N doubles each)
     // and are folded in a fixed order before the scatter into C
     double* ws = nullptr;
     int64_t ws_elems = 0;
@@ -35,7 +35,7 @@ struct GemmArgs {
     // grouped launches with shared outputs: write the raw product to ws[m][n] (no alpha,
     // no scatter); a fold applies it to C
     bool partial_out = false;
-    // split path: write the scaled product to ws[z][m][n] (dense, no alpha, no fold) for a
+    // split path: write the scaled product to ws[z][n][m] (dense, no alpha, no fold) for a
     // scatter by the caller (merged symmetry-blocked products)
     bool dense_out = false;
 };
@@ -120,8 +120,9 @@ int short_ctas(int K, int* kper);
 void short_grouped(const ShortDesc* d, const int* cta_start, int nprob, int total_ctas, int mt, int nt,
                    cudaStream_t s);
 
-// K-ranges the FP64 GEMM splits a contraction into (1 = none); ws needs ksplit*M*N doubles
-int fp64_ksplit(int M, int N, int K, bool skinny_ok = true);
+// K ranges of a skinny product in a launch of its own (1: none, or not a skinny product); ws needs
+// that many times M*N doubles
+int skinny_ksplit(int M, int N, int K);
 
 // out[P][q][p] = in[P][p][q] for naux n x n matrices
 void transpose_factor(const double* in, double* out, int naux, int n, cudaStream_t s);
@@ -143,7 +144,7 @@ struct TileFold {
     int prob = 0, m0 = 0, n0 = 0, slot0 = 0, parts = 0;
 };
 struct TileWork {
-    int rows = 64, slots = 0;
+    int slots = 0;
     std::vector<TileSeg> segs;
     std::vector<int> seg_start;        // CTAs + 1 entries
     std::vector<TileFold> folds;

@@ -332,22 +332,19 @@ __device__ __forceinline__ void tile_write_row(const GemmArgs& g, int m0, int n0
         }
 }
 
-// One problem, one CTA per output tile and K range (blockIdx.y of gridDim.y; more than one
-// range, or partial_out, writes raw products to g.ws[z][m][n]).  The shorter side of the
-// tile grid runs fastest, so that the CTAs in flight share the panels of the longer operand.
+// One problem, one CTA per output tile (the integral build's products; a statement's share
+// grouped launches).  The shorter side of the tile grid runs fastest, so that the CTAs in flight
+// share the panels of the longer operand.
 template <class T, bool AK, bool BKc>
 __global__ void __launch_bounds__(TILE_THREADS, T::PER_SM) gemm_fp64_kernel(GemmArgs g) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     const int tm = (g.M + T::BM - 1) / T::BM, tn = (g.N + T::BN - 1) / T::BN;
     const int t = blockIdx.x;
     const int m0 = (tm <= tn ? t % tm : t / tn) * T::BM, n0 = (tm <= tn ? t / tm : t % tn) * T::BN;
-    const int chunks = (g.K + BK - 1) / BK, per = (chunks + gridDim.y - 1) / gridDim.y;
-    const int kt0 = blockIdx.y * per;
     TileAcc<T> acc;
-    tile_product<T, AK, BKc>(g, m0, n0, kt0, max(0, min(chunks, kt0 + per) - kt0), acc, smem_raw);
-    double* dense = gridDim.y > 1 || g.partial_out ? g.ws + (int64_t)blockIdx.y * g.M * g.N : nullptr;
+    tile_product<T, AK, BKc>(g, m0, n0, 0, (g.K + BK - 1) / BK, acc, smem_raw);
 #pragma unroll
-    for (int i = 0; i < T::MT; i++) tile_write_row<T, AK, BKc>(g, m0, n0, i, acc.v[i], dense);
+    for (int i = 0; i < T::MT; i++) tile_write_row<T, AK, BKc>(g, m0, n0, i, acc.v[i], nullptr);
 }
 
 // Many problems with pairwise disjoint outputs: each CTA walks its segments (a tile and a
@@ -427,19 +424,6 @@ __global__ void __launch_bounds__(256) fold_groups_kernel(const FoldItem* __rest
                 for (int b = 0; b < f.nvn; b++) f.C[f.Cm[a][m] + f.Cn[b][n]] += f.vsign[a * f.nvn + b] * v;
         }
         if (q + 1 < it.n1) __syncthreads();   // the next node may write the same elements
-    }
-}
-
-// fold split-K partials in a fixed order and scatter alpha * sum into every variant
-__global__ void splitk_fold_kernel(GemmArgs g, int ks) {
-    const int64_t mn = (int64_t)g.M * g.N;
-    for (int64_t l = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; l < mn; l += (int64_t)gridDim.x * blockDim.x) {
-        double s = 0.0;
-        for (int z = 0; z < ks; z++) s += g.ws[z * mn + l];
-        const int m = (int)(l / g.N), n = (int)(l % g.N);
-        const double v = g.alpha * s;
-        for (int a = 0; a < g.nvm; a++)
-            for (int b = 0; b < g.nvn; b++) g.C[g.Cm[a][m] + g.Cn[b][n]] += g.vsign[a * g.nvn + b] * v;
     }
 }
 
@@ -866,34 +850,17 @@ void launch_fp64(const GemmArgs& g, cudaStream_t s) {
     using T = Tile<64>;
     constexpr size_t bytes = TileSmem<T, AK, BKc>::bytes;
     set_smem_once((const void*)gemm_fp64_kernel<T, AK, BKc>, (int)bytes);
-    int ks = fp64_ksplit(g.M, g.N, g.K, false);
-    if (!g.ws || (int64_t)ks * g.M * g.N > g.ws_elems) ks = 1;
     const int64_t tiles = (int64_t)((g.M + T::BM - 1) / T::BM) * ((g.N + T::BN - 1) / T::BN);
     if (tiles > INT32_MAX) throw std::runtime_error("FP64 GEMM: too many output tiles for the grid");
-    gemm_fp64_kernel<T, AK, BKc><<<dim3((unsigned)tiles, ks), TILE_THREADS, bytes, s>>>(g);
+    gemm_fp64_kernel<T, AK, BKc><<<(unsigned)tiles, TILE_THREADS, bytes, s>>>(g);
     COUNT_LAUNCH();
-    if (ks > 1) {
-        const int64_t mn = (int64_t)g.M * g.N;
-        int nb = (int)std::min<int64_t>((mn + 255) / 256, 148 * 16);
-        splitk_fold_kernel<<<nb, 256, 0, s>>>(g, ks);
-        COUNT_LAUNCH();
-    }
 }
 
 }  // namespace
 
-// One product in a launch of its own, few output tiles and a long K: split K so that about
-// two waves of CTAs stream the operands; every split keeps at least 512 k.
-int fp64_ksplit(int M, int N, int K, bool skinny_ok) {
-    if (const int nt = skinny_ok ? skinny_groups(M, N) : 0) return skinny_split(std::max(M, N), K, nt).nz;
-    const int64_t tiles = (int64_t)((M + 63) / 64) * ((N + 63) / 64);
-    const int chunks = (K + BK - 1) / BK;
-    const int64_t slots = 148 * Tile<64>::PER_SM;
-    if (tiles >= slots) return 1;
-    int64_t ks = (2 * slots + tiles - 1) / tiles;
-    ks = std::min<int64_t>(ks, chunks / 32);
-    ks = std::min<int64_t>(ks, 256);
-    return (int)std::max<int64_t>(ks, 1);
+int skinny_ksplit(int M, int N, int K) {
+    const int nt = skinny_groups(M, N);
+    return nt ? skinny_split(std::max(M, N), K, nt).nz : 1;
 }
 
 void gemm_fp64(const GemmArgs& g, cudaStream_t s) {
@@ -928,7 +895,6 @@ int fp64_tile_rows(int M, int N) {
 TileWork plan_tile_work(const std::vector<TileProblem>& probs, int rows, bool split) {
     constexpr int TILE_MIN_CHUNKS = 16;
     TileWork w;
-    w.rows = rows;
     const int64_t slots = 148 * (rows == 64 ? Tile<64>::PER_SM : Tile<32>::PER_SM);
     auto tiles_of = [&](const TileProblem& p) { return (int64_t)((p.M + rows - 1) / rows) * ((p.N + rows - 1) / rows); };
     auto chunks_of = [&](const TileProblem& p) { return (int64_t)(p.K + BK - 1) / BK; };
@@ -1272,8 +1238,7 @@ __global__ void kv_read_kernel(const double* X, const int64_t* keys, double* val
         vals[i] = X[keys[i]];
 }
 
-// batched dot: partial[b * ny + j] = sum over the block's range of x * ys[j]
-// out[j] = sum of partial[b][j] over b, one CTA per j
+// out[j] = sum of partial[b * ny + j] over b, one CTA per j
 __global__ void fold_batch_kernel(const double* partial, int nb, int ny, double* out) {
     const int j = blockIdx.x;
     double s = 0;

@@ -28,8 +28,8 @@
 //   (3.7e-8, 1.5e-10, 5.7e-13 for 3, 4, 5 slices).
 //
 // Kernel structure (one CTA per SM walks several 128 x TBN output tiles, 320 threads):
-//   warp 0      TMA producer: NS A-slice + NS B-slice tiles of 128-byte k-blocks per
-//               stage (128-byte swizzle), 2 stages, mbarrier full/empty ring;
+//   warp 0      TMA producer: NS A-slice + NS B-slice tiles of 128- or 64-byte k-blocks per
+//               stage (128- or 64-byte swizzle), 2 or 3 stages, mbarrier full/empty ring;
 //   warp 1      TMEM allocation and the single-thread MMA issuer: one MMA per kept slice
 //               product per k-step, commit to release smem stages and to publish a
 //               finished chunk;
@@ -518,7 +518,7 @@ __global__ void __launch_bounds__(THREADS, 1)
 // tables of the next tile load while the current tile's elements are in flight.
 // ---------------------------------------------------------------------------
 constexpr int SR = 32, SK = 64, STHREADS = 256, SPER = (SR * SK) / STHREADS;
-constexpr int SLICE_CTAS = 148 * 6;   // resident at 6 CTAs per SM (40 registers, 18 KB)
+constexpr int SLICE_CTAS = SMS * 6;   // resident at 6 CTAs per SM (40 registers, 21 KB)
 
 // offset tables of tile t into buffer b (-1 past the operand)
 __device__ __forceinline__ void slice_tables(const int64_t* __restrict__ R, const int64_t* __restrict__ Kt, int nrows,
@@ -995,9 +995,9 @@ int split_ksplit(int M, int N, int K, int nslices, int kind) {
     using namespace split;
     const SchemeInfo si = scheme(kind, nslices);
     const int64_t tiles = (int64_t)((M + BM - 1) / BM) * ((N + si.tbn - 1) / si.tbn);
-    if (tiles >= 148) return 1;
+    if (tiles >= SMS) return 1;
     const int64_t grains = (split_k_pad(K, kind) / si.bke + si.grain - 1) / si.grain;
-    int64_t ks = (2 * 148 + tiles - 1) / tiles;
+    int64_t ks = (2 * SMS + tiles - 1) / tiles;
     ks = std::min<int64_t>(ks, grains);
     ks = std::min<int64_t>(ks, 256);
     return (int)std::max<int64_t>(ks, 1);
