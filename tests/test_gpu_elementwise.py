@@ -57,3 +57,33 @@ def test_sums_dots_weights(o, v, split):
         ctx.weight(z, dv, do)
         den = dv[:, None, None, None] + dv[None, :, None, None] + do[None, None, :, None] + do[None, None, None, :]
         assert np.abs(z.to_full() - fy / den).max() <= 1e-15 * np.abs(fy).max()
+
+
+@pytest.mark.parametrize("group", ["1", "0"], ids=["batched", "one-by-one"])
+@pytest.mark.parametrize("split", [1, 2], ids=["c1", "two-irreps"])
+def test_assignments_over_stale_and_shared_storage(split, group, monkeypatch):
+    """C = alpha A is one pass that does not read C: what was in C, NaN included, is gone.  Sources that
+    are views (<ab||ij> of <ij||ab>) are read through their strides, and a view of C itself as the source
+    is not folded: C is zeroed first, as it is statement by statement."""
+    monkeypatch.setenv("CCSD_GROUP_GEMMS", group)
+    o, v = 5, 9
+    eps, B, occ, vrt, aux = A.synth_problem(11, o, v, nirrep=split)
+    with A.Context(0) as ctx:
+        ctx.set_spaces(vrt=vrt, occ=occ)
+        H = ctx.hamiltonian_from_factor(B, eps, aux_per_irrep=aux if split > 1 else None)
+        ref = H["VABIJ"].to_full()
+        assert np.array_equal(ref, H["VMNEF"].to_full().transpose(2, 3, 0, 1)) and ref.any()
+        z, w = ctx.tensor("z", (2, 0), (0, 2)), ctx.tensor("w", (0, 2), (2, 0))
+        for t in (z, w):
+            t.fill(float("nan"))
+        z["abij"] = H["VABIJ"]["abij"]
+        assert np.array_equal(z.to_full(), ref)
+        w["ijab"] = -2.0 * H["VABIJ"]["abij"]
+        assert np.array_equal(w.to_full(), -2.0 * ref.transpose(2, 3, 0, 1))
+        z.fill(float("nan"))
+        ctx.sum(0.5, H["VMNEF"], "ijab", 0.0, z, "abij")
+        assert np.array_equal(z.to_full(), 0.5 * ref)
+        ctx.sum(0.5, H["VMNEF"], "ijab", 2.0, z, "abij")          # a scaling that is not to zero
+        assert np.array_equal(z.to_full(), 1.5 * ref)
+        H["VMNEF"]["mnef"] = 3.0 * H["VABIJ"]["efmn"]
+        assert not H["VMNEF"].to_full().any()

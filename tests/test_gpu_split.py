@@ -2,7 +2,7 @@
 
 Tolerances: a single contraction agrees with FP64 to 2e-6 of max|C| with three BF16 slices
 per operand (8 bits each, the leading product exact, errors unbiased), 1e-8 with four;
-INT8 slices carry 7 bits each (3e-5, 3e-7, 3e-9 for three, four, five).  A full CCSD solve
+INT8 slices carry 7.99 bits each (3e-5, 3e-7, 3e-9 for three, four, five).  A full CCSD solve
 agrees with the FP64 oracle to |dE| <= 1e-8 Eh and max|dT| <= 1e-7 at every iteration with
 three BF16 or four INT8 slices.
 """
@@ -53,7 +53,7 @@ def _contract(precision, o, v, ia, sa, ib, sb, ic, sc, seed, packed_a=False, sli
 ], ids=["bf16x3", "bf16x4", "i8x3", "i8x4", "i8x5"])
 def test_split_contraction_matches_fp64(case, precision, slices, tol):
     """BF16: three slices 2e-6 of max|C| (FP32-like inputs), four 1e-8 (2^-8 finer);
-    INT8: 7 bits per slice."""
+    INT8: 7.99 bits per slice."""
     sa, ia, sb, ib, sc, ic, packed = case
     o, v = 6, 40
     ref = _contract("fp64", o, v, ia, sa, ib, sb, ic, sc, 11, packed)
@@ -114,17 +114,65 @@ SHAPES.update(amef=((1, 1), (2, 0)), amij=((1, 1), (0, 2)))
 @pytest.mark.parametrize("slices", [3, 4, 5])
 @pytest.mark.parametrize("o,v", [(3, 11), (5, 27), (7, 34)], ids=lambda x: str(x))
 def test_int8_slices_at_odd_extents(o, v, slices):
-    """Rows and k that end inside a packed group of four, both orientations of the gather.  An
-    operand is off by at most half a unit of its last slice (max / 127 / 254^(n-1) / 2), and the
-    products left out (levels of n slices and more, n - 1 of them at the first) by at most
-    127^2 254^-n each in units of (max / 127)^2."""
-    K = max(o * v, v * v) * 4
-    for sa, ia, sb, ib, sc, ic in (("amei", "amei", "abij", "ebjm", "abij", "abij"),
-                                   ("amef", "amef", "abij", "efij", "amij", "amij")):
-        ref = _contract("fp64", o, v, ia, sa, ib, sb, ic, sc, 5, False)
-        got = _contract("split_i8", o, v, ia, sa, ib, sb, ic, sc, 5, False, slices=slices)
-        bound = K * 0.05 * 6 * 0.01 * 6 * (254.0 ** (1 - slices) / 127 + 2 * slices * 254.0 ** -slices)
-        assert np.abs(got - ref).max() <= bound, (sa, np.abs(got - ref).max(), bound)
+    """Rows and k that end inside a packed group of four, both orientations of the gather, and a bound
+    that a lost slice does not meet.  An operand of standard deviation s and row maxima up to m is
+    rounded to multiples of u = m / 127 / 254^(n-1), so that it is off by u / sqrt(12), independently;
+    the products left out (n - 1 of them at level n) are of two digits of 127 / sqrt(3) each, weight
+    254^-n (m / 127)^2.  K terms add as sqrt(K), four images at most add to an element, and the largest
+    of some 10^5 elements stays within six deviations."""
+    sa, sb, m = 0.05, 0.01, 5.0                       # m: row maximum in standard deviations
+
+    def bound(n, K):
+        rounding = 2 * m / 127 / 254.0 ** (n - 1) / 12**0.5
+        left_out = (n - 1) ** 0.5 * (127 / 3**0.5) ** 2 * 254.0**-n * (m / 127) ** 2
+        return 6 * 0.5 * (4 * K) ** 0.5 * sa * sb * (rounding + left_out)
+
+    for xa, ia, xb, ib, xc, ic, K in (("amei", "amei", "abij", "ebjm", "abij", "abij", 2 * o * v),
+                                      ("amef", "amef", "abij", "efij", "amij", "amij", 4 * v * v)):
+        ref = _contract("fp64", o, v, ia, xa, ib, xb, ic, xc, 5, False)
+        err = lambda n: np.abs(_contract("split_i8", o, v, ia, xa, ib, xb, ic, xc, 5, False, slices=n) - ref).max()
+        assert err(slices) <= bound(slices, K), xa
+        if slices > 3:
+            assert err(slices - 1) > bound(slices, K), xa     # one slice less is seen
+
+
+@pytest.mark.parametrize("precision,slices", [("split", 3), ("split", 4), ("split_i8", 3), ("split_i8", 4), ("split_i8", 5)],
+                         ids=["bf16x3", "bf16x4", "i8x3", "i8x4", "i8x5"])
+def test_tiles_of_one_cta_follow_one_another(precision, slices):
+    """2401 x 2401 x 16641: 361 tiles of 128 x 128 (722 of 128 x 64), two and more per CTA, the last of
+    each row and column ragged, and 2 (INT8) to 33 (BF16) drained chunks of k per tile, so that stages,
+    accumulator buffers and their phases go on from one tile to the next.  Rounding and products left
+    out as in the test of the odd extents, BF16 slices with units of 2^(2 - 8 n) of the row maximum."""
+    torch = pytest.importorskip("torch")
+    o, v = 49, 129
+    with A.Context(0) as ctx:
+        ctx.set_spaces(vrt=[v], occ=[o])
+        x, y, z = (ctx.tensor(n, *sh, plain=True) for n, sh in
+                   (("x", ((0, 2), (2, 0))), ("y", ((2, 0), (0, 2))), ("z", ((0, 2), (0, 2)))))
+        g = torch.Generator(device="cuda").manual_seed(slices)
+        for t in (x, y):
+            alpha = t.spin_cases()[0]
+            t.write_block(alpha, torch.rand(t.block_shape(alpha), generator=g, device="cuda", dtype=torch.float64)
+                          .sub_(0.5).cpu().numpy())
+        out = {}
+        for p, n in (("fp64", 0), (precision, slices)):
+            ctx.set_precision(p, slices=n)
+            ctx.set_split_routing("all")
+            ctx.contract(1.0, x, "mnef", y, "efij", 0.0, z, "mnij")
+            out[p] = z.read_block(z.spin_cases()[0])
+        ctx.set_precision("fp64")
+    K, sd = v * v, 12**-0.5
+    if precision == "split_i8":
+        unit = 0.5 / 127 / 254.0 ** (slices - 1)
+        left = (slices - 1) ** 0.5 * (127 / 3**0.5) ** 2 * 254.0**-slices * (0.5 / 127) ** 2
+    else:
+        # 2^(e-6) 2^(-8 (n-1)) with 2^e <= max; FP32 sums of the lower products: 2^-24 of sums below
+        # 2^-8 K max^2, once per product of a chunk
+        unit = 0.25 * 2.0 ** (-6 - 8 * (slices - 1)) * 2
+        left = (slices - 1) ** 0.5 * (2.0**8 / 12**0.5) ** 2 * 2.0 ** (-8 * slices) * 2.0**-14 * 4 + 2.0**-31
+    bound = 7 * K**0.5 * (2 * unit * sd / 12**0.5 + left)
+    err = np.abs(out[precision] - out["fp64"]).max()
+    assert 0 < err <= bound, (err, bound)
 
 
 def test_first_slices_of_a_deeper_slicing_are_unbiased():
