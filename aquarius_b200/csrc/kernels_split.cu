@@ -76,7 +76,7 @@ constexpr int SMS = 148;
 // How long a CTA keeps its SM: as many tiles as make 40960 k, 16 at most (0.3 to 1 ms), so that work of
 // another stream, one of higher priority above all, gets SMs before the product ends.  D2h o=24 v=180
 // beside o=31 v=255 on a stream of lower priority (ms per iteration of the small one, 95th percentile):
-// 77 and 111; 85 and 123 with CTAs that walk the whole product, 70 and 97 with a CTA per tile.  Alone,
+// 78 and 111; 88 and 126 with CTAs that walk the whole product, 70 and 97 with a CTA per tile.  Alone,
 // four iterations of o=24 v=184 take 215.3 ms; 214.0 and 223.8 with those.
 constexpr int HOLD_K = 40960, HOLD_TILES = 16;
 

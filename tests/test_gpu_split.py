@@ -209,15 +209,16 @@ def test_first_slices_of_a_deeper_slicing_are_unbiased():
 
 
 def test_a_small_product_gets_in_beside_a_large_one():
-    """A split product of 16384 tiles on a stream of low priority gives its SMs back as it goes: a
-    small split product on a stream of high priority, queued while it runs, is there in less than
-    half of the time the large one takes (one that kept its SMs held the small one up to its end)."""
+    """A split product of 40000 tiles on a stream of low priority gives its SMs back as it goes: a CTA
+    takes 10 of an SM's 270 tiles.  A small split product on a stream of high priority (five kernels, each
+    of which may wait for such a CTA), queued when 0.4 of the large one's time has gone, is there
+    within 0.3 of it; one that kept its SMs held the small one up to its end, 0.6 later."""
     torch = pytest.importorskip("torch")
     streams = [torch.cuda.Stream(priority=p) for p in (0, -5)]
     ctxs = [A.Context(0, s.cuda_stream) for s in streams]
     try:
         runs = []
-        for ctx, (o, v) in zip(ctxs, [(128, 64), (16, 64)]):
+        for ctx, (o, v) in zip(ctxs, [(160, 64), (16, 64)]):
             ctx.set_spaces(vrt=[v], occ=[o])
             ctx.set_precision("split_i8", slices=4)
             ctx.set_split_routing("all")
@@ -239,8 +240,7 @@ def test_a_small_product_gets_in_beside_a_large_one():
             small(), ctxs[1].synchronize()
             late.append(time.perf_counter() - t0)
             wait()
-        assert min(late) < 0.25 * whole, (late, whole)
-        assert sorted(late)[2] < 0.45 * whole, (late, whole)
+        assert sorted(late)[2] < 0.3 * whole, (late, whole)
     finally:
         for ctx in ctxs:
             ctx.close()
