@@ -48,10 +48,10 @@ constexpr int TILE_THREADS = 128;       // 2 x 2 warps, each a quarter of the ti
 // Tile shapes.  The FP64 tensor pipe (36.8 TFLOP/s measured for m8n8k4) bounds large
 // products.  64 x 64 (32 x 32 per warp, 64 accumulator registers) leaves room for four CTAs
 // of four warps per SM, whose barriers and copy latencies hide behind one another's
-// products: 28.6 TFLOP/s at M=25600 N=400 K=4096 and 29.9 at 2048^3 (pipe 83% busy),
+// products: 28.6 TFLOP/s at M=25600 N=400 K=4096, 29.9 at 2048^3, 31.2 at 2304 x 2304 x 16384 (pipe 84% busy),
 // against 25.4 for 128 x 64 tiles with two CTAs per SM and 18.5-22.7 for 128 x 128 with one;
 // the 128 x 64 kernel with one CTA per SM before it ran the ladder of o=20 v=160 at 13.5.
-// With extents that leave every other pair misaligned (8-byte copies) it keeps 22.3.
+// With extents that leave every other pair misaligned (8-byte copies) it keeps 22.3, 28.5 at 2401 x 2401 x 16641.
 // 32 x 32 (16 x 16 per warp) takes the products that would leave a 64 x 64 tile mostly empty.
 template <int ROWS>
 struct Tile {
